@@ -295,6 +295,17 @@ int lmoe_combine_rows_add(const void* rows_in, const int32_t* index, const float
 int lmoe_gemm_swiglu_bf16(int M, int H, int K, const void* A, int64_t lda, const void* W, int64_t ldw, void* h1,
                           int64_t ld_h1, void* hidden, int64_t ld_hidden, int32_t* status, void* stream);
 
+/* Backward of the non-latent layer's dense parts (autograd of models/moe.py:351-358); s->L is not used.
+ * lmoe_moe_shared_bwd: d_h1_s = swiglu'(h1_s, dy * Wd_s) -> dgrad_cat[T, 2Fs+E][:, :2Fs] (the adjoint runs in the GEMM's
+ * epilogue), d_w_down_s[D, Fs] = dy^T * hidden_s.  lmoe_moe_xside_bwd: dx_dense = [d_h1_s | d_logits] * [Wgu_s ; Wg] and the two
+ * weight gradients that contract with x.  grad_type LMOE_F32 / LMOE_BF16. */
+size_t lmoe_moe_wgrad_workspace_bytes(const lmoe_shape* s);
+int lmoe_moe_shared_bwd(const lmoe_shape* s, const void* dy, const void* w_down_s, const void* h1_s, const void* hidden_s,
+                        void* dgrad_cat, void* d_w_down_s, int grad_type, void* workspace, size_t workspace_bytes,
+                        int32_t* status, void* stream);
+int lmoe_moe_xside_bwd(const lmoe_shape* s, const void* dgrad_cat, const void* w_gate_up_s, const void* w_gate, const void* x,
+                       void* dx_dense, void* d_w_gate_up_s, void* d_w_gate, int grad_type, void* workspace,
+                       size_t workspace_bytes, int32_t* status, void* stream);
 /* Adjoint of lmoe_combine_rows over `rows` rows: flat = row_to_flat[r] (t = flat / K);
  * d_y_rows[r] = weights[flat] * d_routed[t], d_weights[flat] = <d_routed[t], y_rows[r]>; zeros where flat < 0. */
 int lmoe_combine_bwd_rows(const void* d_routed, const void* y_rows, const float* weights, const int32_t* row_to_flat,
@@ -431,9 +442,16 @@ int lmoe_rmsnorm_bwd(const void* x, const float* weight, const float* rstd, cons
  * (expert parallelism) whatever their token counts; s->T is not used.  Replaces models/moe.py:254-275. */
 int lmoe_router_bias_update(const lmoe_shape* s, const int32_t* counts, float gamma, float* expert_bias,
                             float* load_history, void* stream);
+/* The same for callers that also keep an update counter on the device (models/moe.py:275): update_count[0] += 1 in the
+ * same launch. */
+int lmoe_router_bias_update_counted(int E, const int32_t* counts, float gamma, float* expert_bias, float* load_history,
+                                    int64_t* update_count, void* stream);
 
 /* ---- small utilities ---- */
 int lmoe_cast_f32_to_bf16(const float* src, void* dst, int64_t n, void* stream);
+/* Up to LMOE_CAST_MANY_MAX tensors converted by one launch (the fp32 operands of a layer call); n[i] > 0 elements each. */
+#define LMOE_CAST_MANY_MAX 8
+int lmoe_cast_many_f32_to_bf16(int count, const float* const* src, void* const* dst, const int64_t* n, void* stream);
 int lmoe_cast_bf16_to_f32(const void* src, float* dst, int64_t n, void* stream);
 
 #ifdef __cplusplus

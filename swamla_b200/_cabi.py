@@ -103,6 +103,11 @@ SIGNATURES = {
     "lmoe_rmsnorm_fwd": (c_int, [P, P, c_float, c_int64, c_int, P, P, P]),
     "lmoe_add_bf16": (c_int, [P, P, P, c_int64, P]),
     "lmoe_rmsnorm_bwd": (c_int, [P, P, P, P, P, c_int64, c_int, P, P, P, c_size_t, P]),
+    "lmoe_moe_wgrad_workspace_bytes": (c_size_t, [SP]),
+    "lmoe_moe_shared_bwd": (c_int, [SP, P, P, P, P, P, P, c_int, P, c_size_t, P, P]),
+    "lmoe_moe_xside_bwd": (c_int, [SP, P, P, P, P, P, P, P, c_int, P, c_size_t, P, P]),
+    "lmoe_router_bias_update_counted": (c_int, [c_int, P, c_float, P, P, P, P]),
+    "lmoe_cast_many_f32_to_bf16": (c_int, [c_int, P, P, P, P]),
     "lmoe_router_bias_update": (c_int, [SP, P, c_float, P, P, P]),
     "lmoe_cast_f32_to_bf16": (c_int, [P, P, c_int64, P]),
     "lmoe_cast_bf16_to_f32": (c_int, [P, P, c_int64, P]),

@@ -1,4 +1,5 @@
-"""Builds ``liblmoe.so`` (the C-ABI CUDA library) in-tree with nvcc for sm_100a.
+"""Builds ``liblmoe.so`` (the C-ABI CUDA library, nvcc for sm_100a) and ``_host.so`` (the layers' native host path on
+PyTorch's allocator and autograd, g++) in-tree.
 
     python -m swamla_b200.build [--force] [--verbose]
 
@@ -16,6 +17,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 OBJ = os.path.join(CSRC, "_obj")
 LIB = os.path.join(HERE, "liblmoe.so")
+HOST = os.path.join(HERE, "_host.so")
 INCLUDE = os.path.join(os.path.dirname(HERE), "include")
 
 NVCC_FLAGS = [
@@ -42,13 +44,33 @@ def _deps_mtime() -> float:
             if dirpath.startswith(OBJ):
                 continue
             for f in files:
-                if f.endswith((".cu", ".cuh", ".h")):
+                if f.endswith((".cu", ".cuh", ".h", ".cpp")):
                     latest = max(latest, os.path.getmtime(os.path.join(dirpath, f)))
     return latest
 
 
+def _build_host() -> None:
+    """``csrc/torch_host.cpp`` -> ``_host.so``: a Python module against the installed PyTorch's headers and libraries,
+    linked to ``liblmoe.so`` beside it."""
+    import sysconfig
+    import torch
+    root = os.path.dirname(torch.__file__)
+    inc = [os.path.join(root, "include"), os.path.join(root, "include", "torch", "csrc", "api", "include"),
+           sysconfig.get_paths()["include"], os.path.join(os.path.dirname(os.path.dirname(_nvcc())), "include"), INCLUDE]
+    libdir = os.path.join(root, "lib")
+    cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-DTORCH_EXTENSION_NAME=_host",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", *[f"-isystem{i}" for i in inc],
+           os.path.join(CSRC, "torch_host.cpp"), "-o", HOST, f"-L{HERE}", f"-L{libdir}", "-l:liblmoe.so", "-ltorch_python",
+           "-ltorch", "-ltorch_cuda", "-ltorch_cpu", "-lc10_cuda", "-lc10",
+           f"-L{os.path.join(os.path.dirname(os.path.dirname(_nvcc())), 'lib64')}", "-lcudart", "-Wl,-rpath,$ORIGIN"]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode != 0:
+        raise RuntimeError(f"g++ failed for torch_host.cpp:\n{r.stdout}\n{r.stderr}")
+
+
 def build(force: bool = False, verbose: bool = False) -> str:
-    if not force and os.path.exists(LIB) and os.path.getmtime(LIB) >= _deps_mtime():
+    newest = _deps_mtime()
+    if not force and all(os.path.exists(p) and os.path.getmtime(p) >= newest for p in (LIB, HOST)):
         return LIB
     os.makedirs(OBJ, exist_ok=True)
     nvcc = _nvcc()
@@ -73,6 +95,7 @@ def build(force: bool = False, verbose: bool = False) -> str:
     r = subprocess.run(cmd, capture_output=True, text=True)
     if r.returncode != 0:
         raise RuntimeError(f"link failed:\n{r.stdout}\n{r.stderr}")
+    _build_host()
     return LIB
 
 

@@ -564,3 +564,59 @@ extern "C" int lmoe_xside_bwd(const lmoe_shape* s, const void* dgrad_cat, const 
   const long long lds[3] = {s->D, s->D, s->D};
   return splitk_reduce_multi(ws, split, plane, s->D, 3, row0, col0, rows, cols, outs, lds, f32, st);
 }
+
+// ------------------------------------------------------------------ non-latent layer: dense backward
+extern "C" size_t lmoe_moe_wgrad_workspace_bytes(const lmoe_shape* s) {
+  if (!s || s->T <= 0 || s->D <= 0 || s->E <= 0 || s->Fs <= 0) return 0;
+  const int Mx = 2 * s->Fs + s->E;
+  const size_t a = static_cast<size_t>(wgrad_split(Mx, s->D, s->T)) * Mx * s->D;
+  const size_t b = static_cast<size_t>(wgrad_split(s->D, s->Fs, s->T)) * s->D * s->Fs;
+  return (a > b ? a : b) * sizeof(float);
+}
+
+extern "C" int lmoe_moe_shared_bwd(const lmoe_shape* s, const void* dy, const void* w_down_s, const void* h1_s,
+                                   const void* hidden_s, void* dgrad_cat, void* d_w_down_s, int grad_type, void* workspace,
+                                   size_t workspace_bytes, int32_t* status, void* stream) {
+  if (!s || !dy || !w_down_s || !h1_s || !hidden_s || !dgrad_cat || !d_w_down_s || !workspace) return LMOE_ERR_ARG;
+  if (grad_type != LMOE_F32 && grad_type != LMOE_BF16) return LMOE_ERR_ARG;
+  if (s->T <= 0 || s->D <= 0 || (s->D % 8) != 0 || (s->Fs % 32) != 0 || (s->E % 8) != 0) return LMOE_ERR_SHAPE;
+  if (workspace_bytes < lmoe_moe_wgrad_workspace_bytes(s)) return LMOE_ERR_WORKSPACE;
+  GemmCall b = dense(dy, s->D, 0, w_down_s, s->Fs, 1, s->T, s->Fs, s->D, dgrad_cat, 2ll * s->Fs + s->E, EPI_SWIGLU_BWD, status,
+                     stream);
+  b.aux = h1_s;
+  b.ld_aux = 2ll * s->Fs;
+  if (int rc = launch_gemm(b)) return rc;
+  const int split = wgrad_split(s->D, s->Fs, s->T);
+  float* ws = static_cast<float*>(workspace);
+  if (int rc = wgrad_gemm(dy, s->D, s->D, hidden_s, s->Fs, s->Fs, s->T, ws, split, status, stream)) return rc;
+  return splitk_reduce(ws, split, static_cast<long long>(s->D) * s->Fs, s->Fs, 0, 0, s->D, s->Fs, d_w_down_s, s->Fs,
+                       grad_type == LMOE_F32, static_cast<cudaStream_t>(stream));
+}
+
+extern "C" int lmoe_moe_xside_bwd(const lmoe_shape* s, const void* dgrad_cat, const void* w_gate_up_s, const void* w_gate,
+                                  const void* x, void* dx_dense, void* d_w_gate_up_s, void* d_w_gate, int grad_type,
+                                  void* workspace, size_t workspace_bytes, int32_t* status, void* stream) {
+  if (!s || !dgrad_cat || !w_gate_up_s || !w_gate || !x || !dx_dense || !d_w_gate_up_s || !d_w_gate || !workspace)
+    return LMOE_ERR_ARG;
+  if (grad_type != LMOE_F32 && grad_type != LMOE_BF16) return LMOE_ERR_ARG;
+  if (s->T <= 0 || s->D <= 0 || (s->D % 8) != 0 || (s->Fs % 32) != 0 || (s->E % 8) != 0) return LMOE_ERR_SHAPE;
+  if (workspace_bytes < lmoe_moe_wgrad_workspace_bytes(s)) return LMOE_ERR_WORKSPACE;
+  const int Fs2 = 2 * s->Fs, M = Fs2 + s->E;
+  const bf16* d_h1_s = static_cast<const bf16*>(dgrad_cat);
+  GemmCall c = dense(d_h1_s, M, 0, w_gate_up_s, s->D, 1, s->T, s->D, Fs2, dx_dense, s->D, EPI_BF16, status, stream);
+  c.nseg = 2;
+  c.A[1] = d_h1_s + Fs2;
+  c.lda[1] = M;
+  c.B[1] = w_gate;
+  c.ldb[1] = s->D;
+  c.Kseg[1] = s->E;
+  if (int rc = launch_gemm(c)) return rc;
+  const int split = wgrad_split(M, s->D, s->T);
+  float* ws = static_cast<float*>(workspace);
+  if (int rc = wgrad_gemm(dgrad_cat, M, M, x, s->D, s->D, s->T, ws, split, status, stream)) return rc;
+  const int row0[2] = {0, Fs2}, col0[2] = {0, 0}, rows[2] = {Fs2, s->E}, cols[2] = {s->D, s->D};
+  void* const outs[2] = {d_w_gate_up_s, d_w_gate};
+  const long long lds[2] = {s->D, s->D};
+  return splitk_reduce_multi(ws, split, static_cast<long long>(M) * s->D, s->D, 2, row0, col0, rows, cols, outs, lds,
+                             grad_type == LMOE_F32, static_cast<cudaStream_t>(stream));
+}

@@ -363,11 +363,14 @@ route_scatter_kernel(const int* __restrict__ sel, int n, int E, const int* __res
 // whatever the ranks' own token counts were.  One block; E <= LMOE_MAX_EXPERTS threads carry one expert each.
 __global__ void __launch_bounds__(LMOE_MAX_EXPERTS)
 bias_update_kernel(const int* __restrict__ counts, int E, float gamma, float* __restrict__ bias,
-                   float* __restrict__ history) {
+                   float* __restrict__ history, long long* __restrict__ update_count) {
   __shared__ long long total_s;
   const int e = threadIdx.x;
   const int c = (e < E) ? counts[e] : 0;
-  if (e == 0) total_s = 0;
+  if (e == 0) {
+    total_s = 0;
+    if (update_count) update_count[0] += 1;
+  }
   __syncthreads();
   long long part = c;
 #pragma unroll
@@ -533,13 +536,25 @@ extern "C" int lmoe_route_permute_static(const lmoe_shape* s, const int32_t* sel
   return e == cudaSuccess ? 0 : static_cast<int>(e);
 }
 
+static int launch_bias_update(int E, const int32_t* counts, float gamma, float* expert_bias, float* load_history,
+                              int64_t* update_count, void* stream) {
+  if (!counts || !expert_bias || !load_history) return LMOE_ERR_ARG;
+  if (E <= 0 || E > LMOE_MAX_EXPERTS) return LMOE_ERR_SHAPE;
+  count_launch();
+  bias_update_kernel<<<1, LMOE_MAX_EXPERTS, 0, static_cast<cudaStream_t>(stream)>>>(
+      counts, E, gamma, expert_bias, load_history, reinterpret_cast<long long*>(update_count));
+  cudaError_t e = cudaGetLastError();
+  return e == cudaSuccess ? 0 : static_cast<int>(e);
+}
+
 extern "C" int lmoe_router_bias_update(const lmoe_shape* s, const int32_t* counts, float gamma, float* expert_bias,
                                        float* load_history, void* stream) {
   if (int rc = check_shape(s)) return rc;
-  if (!counts || !expert_bias || !load_history) return LMOE_ERR_ARG;
-  count_launch();
-  bias_update_kernel<<<1, LMOE_MAX_EXPERTS, 0, static_cast<cudaStream_t>(stream)>>>(counts, s->E, gamma, expert_bias,
-                                                                                    load_history);
-  cudaError_t e = cudaGetLastError();
-  return e == cudaSuccess ? 0 : static_cast<int>(e);
+  return launch_bias_update(s->E, counts, gamma, expert_bias, load_history, nullptr, stream);
+}
+
+extern "C" int lmoe_router_bias_update_counted(int E, const int32_t* counts, float gamma, float* expert_bias,
+                                               float* load_history, int64_t* update_count, void* stream) {
+  if (!update_count) return LMOE_ERR_ARG;
+  return launch_bias_update(E, counts, gamma, expert_bias, load_history, update_count, stream);
 }

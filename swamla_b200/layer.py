@@ -10,8 +10,8 @@ from __future__ import annotations
 import torch
 import torch.nn as nn
 
-from . import _cabi, status as status_monitor
-from .functional import latent_moe, make_shape, _stream
+from . import _cabi, functional_moe, status as status_monitor
+from .functional import latent_moe, latent_moe_opaque, make_shape, _host, _stream
 from .compiled_ops import latent_moe_compiled
 
 
@@ -107,6 +107,11 @@ class AuxLossFreeRouter(nn.Module):
             return
         status_monitor.poll()            # a step whose kernels reported a failure raises here (or at the next forward)
         counts, T = self._last_counts, self._last_num_tokens
+        if counts.is_cuda and self.expert_bias.dtype == self.load_history.dtype == torch.float32 \
+                and self.update_count.dtype == torch.int64 and self.update_count.is_cuda:
+            _host().bias_update(counts, self.gamma, self.expert_bias, self.load_history, self.update_count)
+            self._last_selected_experts = self._last_counts = self._last_num_tokens = None
+            return
         # the kernel takes the expected load T*K/E from the histogram itself (sum of counts / E), so a histogram
         # summed over expert-parallel ranks with different token counts gives the same update on every rank
         shape = make_shape(T, 8, 64, self.n_experts, self.top_k, 64, 8)
@@ -231,17 +236,42 @@ class LatentMoELayer(nn.Module):
         if n_experts > 256 or n_activated > 32:
             raise ValueError("kernel constraints: at most 256 routed experts and top-32")
 
+    def _arguments(self):
+        """The layer's tensors in the order of ``functional.latent_moe``.  Read through the modules' own tables: attribute
+        access on a module costs several times a dictionary lookup, 14 of them are a fifth of a small call's host time.
+        Anything unusual (several shared experts, parametrised weights) goes through the attributes."""
+        try:
+            m = self._modules
+            router, experts, shared = m["router"], m["experts"]._parameters, m["shared_experts"]._modules
+            if len(shared) == 1:
+                s = shared["0"]._modules
+                return (router._modules["gate"]._parameters["weight"], m["down_proj"]._parameters["weight"],
+                        m["up_proj"]._parameters["weight"], s["gate_up_proj"]._parameters["weight"],
+                        s["down_proj"]._parameters["weight"], experts["gate_up_weight"], experts["down_weight"],
+                        router._buffers["expert_bias"])
+        except KeyError:
+            pass
+        w_gate_up_s, w_down_s = _merged_shared_weights(self.shared_experts)
+        return (self.router.gate.weight, self.down_proj.weight, self.up_proj.weight, w_gate_up_s, w_down_s,
+                self.experts.gate_up_weight, self.experts.down_weight, self.router.expert_bias)
+
     def forward(self, x: torch.Tensor) -> torch.Tensor:
         compiling = torch.compiler.is_compiling()
         if not compiling:
             status_monitor.poll()        # raises if an earlier step's kernels reported a failure (no synchronisation)
         batch_size, seq_len, d_model = x.shape
+        router = self._modules["router"]
+        if self.ep_size == 1 and not compiling and x.is_cuda:
+            y, z_loss, sel, counts = latent_moe(x, *self._arguments(), self.n_activated, router.z_loss_coef, self.fp8_experts)
+            self.aux_loss = z_loss
+            if self.training:
+                router._last_selected_experts, router._last_counts = sel, counts
+                router._last_num_tokens = batch_size * seq_len
+                if self.dropout.p > 0.0:
+                    y = self.dropout(y)
+            return y
         x_flat = x.reshape(-1, d_model)
-        w_gate_up_s, w_down_s = _merged_shared_weights(self.shared_experts)
-        args = (x_flat, self.router.gate.weight, self.down_proj.weight, self.up_proj.weight,
-                w_gate_up_s, w_down_s,
-                self.experts.gate_up_weight, self.experts.down_weight,
-                self.router.expert_bias, self.n_activated, self.router.z_loss_coef)
+        args = (x_flat, *self._arguments(), self.n_activated, router.z_loss_coef)
         if self.ep_size > 1 and self.ep_mode == "p2p_dedup":
             from .ep import DedupBuffers, latent_moe_ep_dedup
             T = x_flat.shape[0]
@@ -266,7 +296,7 @@ class LatentMoELayer(nn.Module):
             # keep one graph across the layer; they run the same kernels as the eager call below
             y, z_loss, sel, counts = latent_moe_compiled(*args)
         else:
-            y, z_loss, sel, counts = latent_moe(*args, fp8=self.fp8_experts)
+            y, z_loss, sel, counts = (latent_moe_opaque if compiling else latent_moe)(*args, fp8=self.fp8_experts)
         self.aux_loss = z_loss                                            # moe.py:719
         if self.training:                                                 # moe.py:237-240
             self.router._last_selected_experts = sel
@@ -342,21 +372,20 @@ class MoELayer(nn.Module):
         status_monitor.poll(block=True)
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
-        from .functional_moe import moe
+        moe = functional_moe.moe_opaque if torch.compiler.is_compiling() else functional_moe.moe
         status_monitor.poll()
-        batch_size, seq_len, d_model = x.shape
-        x_flat = x.reshape(-1, d_model)
         w_gate_up_s, w_down_s = _merged_shared_weights(self.shared_experts)
-        y, z_loss, sel, counts = moe(x_flat, self.router.gate.weight, w_gate_up_s,
+        y, z_loss, sel, counts = moe(x, self.router.gate.weight, w_gate_up_s,
                                      w_down_s, self.experts.gate_up_weight, self.experts.down_weight,
                                      self.router.expert_bias, self.n_activated, self.router.z_loss_coef)
         self.aux_loss = z_loss                                            # moe.py:358
         if self.training:                                                 # moe.py:237-240
             self.router._last_selected_experts = sel
             self.router._last_counts = counts
-            self.router._last_num_tokens = x_flat.shape[0]
-        y = self.dropout(y)                                               # moe.py:367
-        return y.view(batch_size, seq_len, d_model)
+            self.router._last_num_tokens = x.shape[0] * x.shape[1]
+            if self.dropout.p > 0.0:
+                y = self.dropout(y)                                       # moe.py:367
+        return y
 
     def get_aux_loss(self) -> torch.Tensor:
         return self.aux_loss

@@ -1,12 +1,14 @@
-"""Host-side reading of the device status word without stalling the launch queue.
+"""Host-side reading of the device status words without stalling the launch queue.
 
-Every forward/backward of the path owns one int32 status word on the device.  Kernels write a non-zero code into it
-when a bounded wait gives up (101-103) or when an expert-parallel shard receives more rows than its buffers hold
-(201: the excess rows are dropped, the results of that step are wrong).  Reading the word with ``.item()`` would
-synchronise the stream on every step, so the word is copied to pinned host memory behind the step's kernels and looked
-at later: ``poll()`` inspects the copies that have already completed and raises for the first non-zero code;
-``poll(block=True)`` waits for all of them first.  The layers call ``poll()`` at the start of every forward and in
-``update_bias_from_last_forward()`` (once per training step), and expose the blocking form as ``check_status()``.
+Kernels write a non-zero code into the status word of their call when a bounded wait gives up (101-103) or when an
+expert-parallel shard receives more rows than its buffers hold (201: the excess rows are dropped, the results of that step
+are wrong).  Single-GPU layers pass words in mapped host memory (``csrc/torch_host.cpp``), which the native path looks at
+on every call: nothing is queued for them.  An expert-parallel step owns one int32 on the device; reading it with
+``.item()`` would synchronise the stream on every step, so it is copied to pinned host memory behind the step's kernels
+(``post``) and looked at later: ``poll()`` inspects the copies that have already completed and raises for the first
+non-zero code; ``poll(block=True)`` waits for everything queued, the words in host memory included.  The layers poll at
+the start of every forward and in ``update_bias_from_last_forward()`` (once per training step), and expose the blocking
+form as ``check_status()``.
 """
 from __future__ import annotations
 
@@ -34,6 +36,10 @@ def post(status: torch.Tensor, label: str) -> None:
 def poll(block: bool = False) -> None:
     """Raises ``LmoeError`` if a completed step reported a non-zero device status."""
     global _pending
+    if block:
+        from . import functional
+        torch.cuda.synchronize()
+        functional._host().poll_status()
     if not _pending or torch.cuda.is_current_stream_capturing():
         return
     keep, bad = [], None
