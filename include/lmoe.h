@@ -126,7 +126,8 @@ int lmoe_gemm_bf16(int M, int N, int K, const void* A, int64_t lda, int a_mn, co
 
 /* Gate logits (fp32) and latent down-projection (bf16).
  * x[T,D] bf16, w_gate[E,D] bf16, w_down[L,D] bf16 -> logits[T,E] f32, x_latent[T,L] bf16.
- * Replaces models/moe.py:217 (router.gate) and models/moe.py:722 (down_proj). */
+ * Replaces models/moe.py:217 (router.gate) and models/moe.py:722 (down_proj).  Either output may be NULL: the other one is
+ * computed alone (so that the two GEMMs can go to two streams). */
 int lmoe_xproj_fwd(const lmoe_shape* s, const void* x, const void* w_gate, const void* w_down, float* logits,
                    void* x_latent, int32_t* status, void* stream);
 
@@ -142,6 +143,18 @@ int lmoe_gate_topk_fwd(const lmoe_shape* s, const float* logits, const float* ex
  * layout tables.  Deterministic (no global atomics).  Replaces models/moe_triton.py:12-78. */
 int lmoe_route_permute(const lmoe_shape* s, const int32_t* sel, const lmoe_route* r, void* workspace,
                        size_t workspace_bytes, void* stream);
+
+/* Router and permutation of one layer call in two or three launches instead of six: lmoe_topk_hist_fwd is lmoe_gate_topk_fwd
+ * (without the z-loss) that also counts the selections per block of tokens into `workspace`
+ * (lmoe_route_fwd_workspace_bytes); lmoe_route_gather_fwd writes the tables of lmoe_route_permute and z_loss from it and, when
+ * src is given, dst[pos[t*K+k]] = src[t] (rows of row_bytes, a multiple of 16) with the pad rows zeroed.  `sel` is the one
+ * lmoe_topk_hist_fwd wrote: no expert twice in a row.  Same tables and rows as the separate entry points
+ * (models/moe.py:217-233, 749-757; models/moe_triton.py:36-78). */
+size_t lmoe_route_fwd_workspace_bytes(const lmoe_shape* s);
+int lmoe_topk_hist_fwd(const lmoe_shape* s, const float* logits, const float* expert_bias, int32_t* sel, float* weights,
+                       float* lse, void* workspace, size_t workspace_bytes, void* stream);
+int lmoe_route_gather_fwd(const lmoe_shape* s, const int32_t* sel, void* workspace, size_t workspace_bytes, float z_coef,
+                          float* z_loss, const lmoe_route* r, const void* src, int row_bytes, void* dst, void* stream);
 
 /* Same result as lmoe_route_permute, for hosts that have no device memory to give as workspace.
  * (No counterpart in the reference: this entry point exists only on this boundary.)
@@ -174,7 +187,8 @@ int lmoe_experts_fwd(const lmoe_shape* s, const void* x_latent, const void* w_ga
                      void* stream);
 
 /* Shared expert, first half: h1_s = x * w_gate_up_s^T, hidden_s = silu(gate) * up.
- * x[T,D], w_gate_up_s[2Fs,D] -> h1_s[T,2Fs] bf16, hidden_s = act_cat[:, L:].
+ * x[T,D], w_gate_up_s[2Fs,D] -> h1_s[T,2Fs] bf16, hidden_s = act_cat[:, L:].  Here and in every SwiGLU forward below,
+ * h1 (the saved gate / up) may be NULL: a forward that no backward follows writes `hidden` only, a third of the output.
  * Replaces models/moe.py:63-67 (SwiGLUExpert.forward). */
 int lmoe_shared_gateup_fwd(const lmoe_shape* s, const void* x, const void* w_gate_up_s, void* h1_s, void* act_cat,
                            int32_t* status, void* stream);

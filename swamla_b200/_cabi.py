@@ -53,6 +53,9 @@ SIGNATURES = {
     "lmoe_xproj_fwd": (c_int, [SP, P, P, P, P, P, P, P]),
     "lmoe_gate_topk_fwd": (c_int, [SP, P, P, c_float, P, P, P, P, P, P]),
     "lmoe_route_permute": (c_int, [SP, P, RP, P, c_size_t, P]),
+    "lmoe_route_fwd_workspace_bytes": (c_size_t, [SP]),
+    "lmoe_topk_hist_fwd": (c_int, [SP, P, P, P, P, P, P, c_size_t, P]),
+    "lmoe_route_gather_fwd": (c_int, [SP, P, P, c_size_t, c_float, P, RP, P, c_int, P, P]),
     "lmoe_route_permute_static": (c_int, [SP, P, RP, P]),
     "lmoe_experts_fwd": (c_int, [SP, P, P, P, RP, P, P, P, P, P, P]),
     "lmoe_shared_gateup_fwd": (c_int, [SP, P, P, P, P, P, P]),

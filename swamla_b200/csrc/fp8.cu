@@ -130,7 +130,7 @@ extern "C" int lmoe_gemm_fp8(int M, int N, int K, const void* A, int64_t lda, in
 extern "C" int lmoe_grouped_gateup_fp8(int64_t P, int E, int L, int F, const void* xq, const void* wq, const float* deq_x,
                                        const float* deq_w, const int32_t* tile_expert, const int32_t* n_tiles, void* h1,
                                        void* hidden, int32_t* status, void* stream) {
-  if (!xq || !wq || !deq_x || !deq_w || !tile_expert || !n_tiles || !h1 || !hidden) return LMOE_ERR_ARG;
+  if (!xq || !wq || !deq_x || !deq_w || !tile_expert || !n_tiles || !hidden) return LMOE_ERR_ARG;
   if (P <= 0 || (P % LMOE_ROW_PAD) != 0 || E <= 0 || (L % 128) != 0 || (F % 128) != 0) return LMOE_ERR_SHAPE;
   GemmCall a;
   a.esz = 1;

@@ -268,7 +268,7 @@ static int launch_gemm_pair(const GemmCall& c) {
       plane_elems = c.c_group_stride;
       if (plane_elems < static_cast<long long>(c.M) * c.ldc) return LMOE_ERR_ARG;
     }
-    int rc = encode_out(&p.tmC, c.C, f32, cols, c.M, planes, c.ldc, plane_elems);
+    int rc = c.C ? encode_out(&p.tmC, c.C, f32, cols, c.M, planes, c.ldc, plane_elems) : 0;
     if (rc) return rc;
     if (swiglu) {
       rc = encode_out(&p.tmC2, c.C2, false, c.N, c.M, 1, c.ldc2, 0);
@@ -282,6 +282,7 @@ static int launch_gemm_pair(const GemmCall& c) {
   p.n_tiles = n_tiles;
   p.split_k = split;
   p.half = c.N;
+  p.hidden_only = c.C ? 0 : 1;
   p.status = c.status;
   const long long total = static_cast<long long>(m_tiles) * n_tiles * split;
   const int key = c.a_mn | (c.b_mn << 1) | (c.epi << 2);
@@ -337,7 +338,7 @@ static int launch_gemm_pair_grouped(const GemmCall& c) {
   rc = !c.b_mn ? encode_2d(&p.tmB[0], c.B[0], K, b_outer, c.ldb[0], 128, 2)       // this CTA's 128 rows of B[e]
                : encode_2d(&p.tmB[0], c.B[0], n_b_total, b_outer, c.ldb[0], 64, 2);
   if (rc) return rc;
-  rc = encode_out(&p.tmC, c.C, false, swiglu ? 2ll * c.N : c.N, c.padded_rows, 1, c.ldc, 0);
+  rc = c.C ? encode_out(&p.tmC, c.C, false, swiglu ? 2ll * c.N : c.N, c.padded_rows, 1, c.ldc, 0) : 0;
   if (rc) return rc;
   if (swiglu) {
     rc = encode_out(&p.tmC2, c.C2, false, c.N, c.padded_rows, 1, c.ldc2, 0);
@@ -351,6 +352,7 @@ static int launch_gemm_pair_grouped(const GemmCall& c) {
   p.groups = c.groups;
   p.split_k = 1;
   p.half = c.N;
+  p.hidden_only = c.C ? 0 : 1;
   p.b_group_rows = c.b_group_rows;
   p.pad_offsets = c.pad_offsets;
   p.status = c.status;
@@ -362,7 +364,8 @@ static int launch_gemm_pair_grouped(const GemmCall& c) {
 }
 
 int launch_gemm(const GemmCall& c) {
-  if (c.nseg < 1 || c.nseg > 3 || !c.C || c.M <= 0 || c.N <= 0) return LMOE_ERR_ARG;
+  // only a SwiGLU GEMM may leave out its main output (gate / up; see GemmParams::hidden_only)
+  if (c.nseg < 1 || c.nseg > 3 || (!c.C && c.epi != EPI_SWIGLU) || c.M <= 0 || c.N <= 0) return LMOE_ERR_ARG;
   if (c.split_k > 1 && (c.epi != EPI_F32 || c.nseg != 1 || c.grp != GRP_NONE)) return LMOE_ERR_ARG;
   const bool swiglu = (c.epi == EPI_SWIGLU);
   if (c.esz != 1 && c.esz != 2) return LMOE_ERR_ARG;
@@ -471,7 +474,7 @@ int launch_gemm(const GemmCall& c) {
       plane_elems = c.c_group_stride;
       if (plane_elems < static_cast<long long>(c.M) * c.ldc) return LMOE_ERR_ARG;
     }
-    int rc = encode_out(&p.tmC, c.C, f32, cols, rows_total, planes, c.ldc, plane_elems);
+    int rc = c.C ? encode_out(&p.tmC, c.C, f32, cols, rows_total, planes, c.ldc, plane_elems) : 0;
     if (rc) return rc;
     if (swiglu) {
       rc = encode_out(&p.tmC2, c.C2, false, c.N, rows_total, 1, c.ldc2, 0);
@@ -491,6 +494,7 @@ int launch_gemm(const GemmCall& c) {
   p.groups = c.groups;
   p.split_k = split;
   p.half = c.N;
+  p.hidden_only = c.C ? 0 : 1;
   p.tile_expert = c.tile_expert;
   p.n_m_tiles = c.n_m_tiles;
   p.b_group_rows = c.b_group_rows;

@@ -62,6 +62,7 @@ struct alignas(64) GemmParams {
   int groups;            // GRP_K: number of experts
   int split_k;           // GRP_NONE: number of k-slices (each writes its own output plane)
   int half;              // SwiGLU: width of the gate half (F or Fs)
+  int hidden_only;       // SwiGLU: gate / up are not written (a forward that no backward follows); tmC is not set
   const int* tile_expert;  // GRP_M
   const int* n_m_tiles;    // GRP_M: device scalar, number of 128-row tiles in use
   int b_group_rows;        // GRP_M: rows of the stacked B tensor per expert
@@ -215,7 +216,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_kernel(const __grid_cons
       tma_prefetch_desc(&p.tmA[i]);
       tma_prefetch_desc(&p.tmB[i]);
     }
-    tma_prefetch_desc(&p.tmC);
+    if (!kSwiglu || !p.hidden_only) tma_prefetch_desc(&p.tmC);
     if (kSwiglu) tma_prefetch_desc(&p.tmC2);
   }
   if (warp == 1) {
@@ -592,6 +593,21 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_kernel(const __grid_cons
             const float u0 = __uint_as_float(pu[j] << 16), u1 = __uint_as_float(pu[j] & 0xffff0000u);
             ph[j] = pack_bf16x2(silu_f(g0) * u0, silu_f(g1) * u1);
           }
+        }
+        if (kSwiglu && p.hidden_only) {
+          // one store per slab instead of three: the gate and up slabs' buffers take the hidden slabs in turn
+          uint8_t* hbuf = sbuf0 + buf * S::kSlabBytes;
+          if (issuer) tma_store_wait_read_1();
+          epi_bar_sync(bar_id);
+          stage_row_bf16(hbuf, r, ph);
+          fence_proxy_async_smem();
+          epi_bar_sync(bar_id);
+          if (issuer) {
+            tma_store_3d(&p.tmC2, hbuf, n0 + c * kSlabCols, t.m0, 0);
+            tma_store_commit();
+          }
+          buf ^= 1;
+          continue;
         }
         // the staging buffer about to be written was last read by the store issued kBufsPerGroup slabs ago
         uint8_t* sbuf = sbuf0 + buf * (S::kStreams * S::kSlabBytes);

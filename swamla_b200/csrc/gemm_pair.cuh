@@ -114,7 +114,7 @@ gemm_pair_kernel(const __grid_constant__ GemmParams p) {
       tma_prefetch_desc(&p.tmA[i]);
       tma_prefetch_desc(&p.tmB[i]);
     }
-    tma_prefetch_desc(&p.tmC);
+    if (!kSwiglu || !p.hidden_only) tma_prefetch_desc(&p.tmC);
     if (kSwiglu) tma_prefetch_desc(&p.tmC2);
   }
   if (warp == 1) {
@@ -344,6 +344,18 @@ gemm_pair_kernel(const __grid_constant__ GemmParams p) {
             const float u0 = __uint_as_float(pu[j] << 16), u1 = __uint_as_float(pu[j] & 0xffff0000u);
             ph[j] = pack_bf16x2(silu_f(g0) * u0, silu_f(g1) * u1);
           }
+        }
+        if (kSwiglu && p.hidden_only) {  // as in gemm.cuh: one store per slab, two staging buffers in turn
+          uint8_t* hbuf = sbuf0 + buf * S::kSlabBytes;
+          if (issuer) tma_store_wait_read_1();
+          epi_bar_sync(bar_id);
+          stage_row_bf16(hbuf, r, ph);
+          fence_proxy_async_smem();
+          epi_bar_sync(bar_id);
+          if (issuer && t.live && (GRP == GRP_M || t.m0 < p.M)) tma_store_3d(&p.tmC2, hbuf, n0 + c * kSlabCols, t.m0, 0);
+          if (issuer) tma_store_commit();
+          buf ^= 1;
+          continue;
         }
         uint8_t* sbuf = sbuf0 + buf * (S::kStreams * S::kSlabBytes);
         if (issuer) {

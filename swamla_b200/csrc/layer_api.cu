@@ -119,9 +119,11 @@ extern "C" size_t lmoe_wgrad_workspace_bytes(const lmoe_shape* s) {
 extern "C" int lmoe_xproj_fwd(const lmoe_shape* s, const void* x, const void* w_gate, const void* w_down, float* logits,
                               void* x_latent, int32_t* status, void* stream) {
   if (int rc = check_dims(s)) return rc;
-  if (!x || !w_gate || !w_down || !logits || !x_latent) return LMOE_ERR_ARG;
+  if (!x || (!logits && !x_latent) || (logits && !w_gate) || (x_latent && !w_down)) return LMOE_ERR_ARG;
   GemmCall g = dense(x, s->D, 0, w_gate, s->D, 0, s->T, s->E, s->D, logits, s->E, EPI_F32, status, stream);
-  if (int rc = launch_gemm(g)) return rc;
+  if (logits)
+    if (int rc = launch_gemm(g)) return rc;
+  if (!x_latent) return 0;
   GemmCall d = dense(x, s->D, 0, w_down, s->D, 0, s->T, s->L, s->D, x_latent, s->L, EPI_BF16, status, stream);
   return launch_gemm(d);
 }
@@ -129,7 +131,7 @@ extern "C" int lmoe_xproj_fwd(const lmoe_shape* s, const void* x, const void* w_
 extern "C" int lmoe_shared_gateup_fwd(const lmoe_shape* s, const void* x, const void* w_gate_up_s, void* h1_s,
                                       void* act_cat, int32_t* status, void* stream) {
   if (int rc = check_dims(s)) return rc;
-  if (!x || !w_gate_up_s || !h1_s || !act_cat) return LMOE_ERR_ARG;
+  if (!x || !w_gate_up_s || !act_cat) return LMOE_ERR_ARG;  // h1_s NULL: forward only
   GemmCall c = dense(x, s->D, 0, w_gate_up_s, s->D, 0, s->T, s->Fs, s->D, h1_s, 2ll * s->Fs, EPI_SWIGLU, status, stream);
   c.C2 = static_cast<bf16*>(act_cat) + s->L;  // hidden_s = act_cat[:, L:]
   c.ldc2 = s->L + s->Fs;
@@ -139,7 +141,7 @@ extern "C" int lmoe_shared_gateup_fwd(const lmoe_shape* s, const void* x, const 
 extern "C" int lmoe_gemm_swiglu_bf16(int M, int H, int K, const void* A, int64_t lda, const void* W, int64_t ldw,
                                      void* h1, int64_t ld_h1, void* hidden, int64_t ld_hidden, int32_t* status,
                                      void* stream) {
-  if (!A || !W || !h1 || !hidden || M <= 0 || H <= 0 || K <= 0) return LMOE_ERR_ARG;
+  if (!A || !W || !hidden || M <= 0 || H <= 0 || K <= 0) return LMOE_ERR_ARG;
   if ((H % 32) != 0 || ld_h1 < 2ll * H || ld_hidden < H) return LMOE_ERR_SHAPE;
   GemmCall c = dense(A, lda, 0, W, ldw, 0, M, H, K, h1, ld_h1, EPI_SWIGLU, status, stream);
   c.C2 = hidden;
@@ -172,10 +174,10 @@ static int grouped_fwd_impl(int64_t P, int E, int L, int F, const void* x_sorted
                             const void* w_down, const int32_t* tile_expert, const int32_t* n_tiles,
                             const int32_t* pad_offsets, void* h1,
                             void* hidden, void* y_sorted, int32_t* status, void* stream) {
-  if (!x_sorted || !w_gate_up || !w_down || !tile_expert || !n_tiles || !h1 || !hidden || !y_sorted) return LMOE_ERR_ARG;
+  if (!x_sorted || !w_gate_up || !w_down || !tile_expert || !n_tiles || !hidden || !y_sorted) return LMOE_ERR_ARG;
   if (P <= 0 || (P % LMOE_ROW_PAD) != 0 || E <= 0 || (L % 64) != 0 || (F % 64) != 0) return LMOE_ERR_SHAPE;
   // one kernel for gate_up -> SwiGLU -> down per 128-row tile when the latent width fits the second accumulator
-  if (!g && chain_applies(L, F))
+  if (!g && h1 && chain_applies(L, F))
     return launch_chain(CHAIN_FWD, P, E, L, F, x_sorted, w_gate_up, w_down, tile_expert, n_tiles, pad_offsets, h1, hidden,
                         y_sorted, status, static_cast<cudaStream_t>(stream));
   // h1 = x_sorted * Wgu[e]  (Wgu stacked [E*L, 2F], N contiguous), hidden = silu(gate) * up

@@ -17,17 +17,30 @@ constexpr int kMaxPerLane = LMOE_MAX_EXPERTS / 32;  // 8 scores per lane at E = 
 
 __device__ __forceinline__ float sigmoid_f(float x) { return 1.0f / (1.0f + expf(-x)); }
 
+// The top-k kernels can also count their block's selections: chunk_hist[blockIdx.x][E], the first pass of the routing
+// tables (the counts are whole numbers, so the order of the shared-memory additions does not matter).
+__device__ __forceinline__ void topk_hist_clear(int* s_hist, int E) {
+  for (int e = threadIdx.x; e < E; e += blockDim.x) s_hist[e] = 0;
+  __syncthreads();
+}
+__device__ __forceinline__ void topk_hist_store(const int* s_hist, int E, int* __restrict__ chunk_hist) {
+  // the caller's last __syncthreads() lies after every addition
+  for (int e = threadIdx.x; e < E; e += blockDim.x) chunk_hist[static_cast<long long>(blockIdx.x) * E + e] = s_hist[e];
+}
 
-// One warp per token row.  Lane l holds experts l, l+32, ...
+// One warp per token row, `per_warp` consecutive rows each.  Lane l holds experts l, l+32, ...
 __global__ void __launch_bounds__(kTopkWarpsPerBlock * 32)
 gate_topk_kernel(const float* __restrict__ logits, const float* __restrict__ bias, int T, int E, int K,
                  int* __restrict__ sel, float* __restrict__ weights, float* __restrict__ lse_out,
-                 float* __restrict__ z_partial) {
+                 float* __restrict__ z_partial, int per_warp, int* __restrict__ chunk_hist) {
   __shared__ float s_lse2[kTopkWarpsPerBlock];
+  __shared__ int s_hist[LMOE_MAX_EXPERTS];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int t = blockIdx.x * kTopkWarpsPerBlock + warp;
+  if (chunk_hist) topk_hist_clear(s_hist, E);
   float lse2 = 0.f;
-  if (t < T) {
+  for (int r = 0; r < per_warp; ++r) {
+    const int t = (blockIdx.x * kTopkWarpsPerBlock + warp) * per_warp + r;
+    if (t >= T) break;
     float aff[kMaxPerLane], score[kMaxPerLane];
     const float* row = logits + static_cast<long long>(t) * E;
     float mx = -CUDART_INF_F;
@@ -56,7 +69,7 @@ gate_topk_kernel(const float* __restrict__ logits, const float* __restrict__ bia
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) se += __shfl_xor_sync(0xffffffffu, se, o);
     const float lse = mx + logf(se);
-    lse2 = lse * lse;
+    lse2 += lse * lse;
     if (lane == 0) lse_out[t] = lse;
 
     // Order-preserving 32-bit keys: key(a) > key(b) <=> a > b (with -0 folded onto +0), so that the
@@ -104,6 +117,7 @@ gate_topk_kernel(const float* __restrict__ logits, const float* __restrict__ bia
     if (lane < K) {
       sel[static_cast<long long>(t) * K + lane] = my_idx;
       weights[static_cast<long long>(t) * K + lane] = my_aff / (aff_sum + 1e-9f);
+      if (chunk_hist) atomicAdd(&s_hist[my_idx], 1);
     }
   }
   if (lane == 0) s_lse2[warp] = lse2;
@@ -113,6 +127,7 @@ gate_topk_kernel(const float* __restrict__ logits, const float* __restrict__ bia
     for (int i = 0; i < kTopkWarpsPerBlock; ++i) s += s_lse2[i];
     z_partial[blockIdx.x] = s;
   }
+  if (chunk_hist) topk_hist_store(s_hist, E, chunk_hist);
 }
 
 // Same result for E = 32 * PER: lane l holds the PER CONSECUTIVE experts l*PER .. l*PER+PER-1, so "lower expert index
@@ -122,13 +137,16 @@ template <int PER>
 __global__ void __launch_bounds__(kTopkWarpsPerBlock * 32)
 gate_topk_blocked_kernel(const float* __restrict__ logits, const float* __restrict__ bias, int T, int K,
                          int* __restrict__ sel, float* __restrict__ weights, float* __restrict__ lse_out,
-                         float* __restrict__ z_partial) {
+                         float* __restrict__ z_partial, int per_warp, int* __restrict__ chunk_hist) {
   constexpr int E = 32 * PER;
   __shared__ float s_lse2[kTopkWarpsPerBlock];
+  __shared__ int s_hist[E];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int t = blockIdx.x * kTopkWarpsPerBlock + warp;
+  if (chunk_hist) topk_hist_clear(s_hist, E);
   float lse2 = 0.f;
-  if (t < T) {
+  for (int r = 0; r < per_warp; ++r) {
+    const int t = (blockIdx.x * kTopkWarpsPerBlock + warp) * per_warp + r;
+    if (t >= T) break;
     float x[PER], aff[PER];
     unsigned key[PER];
     const float* row = logits + static_cast<long long>(t) * E + lane * PER;
@@ -149,7 +167,7 @@ gate_topk_blocked_kernel(const float* __restrict__ logits, const float* __restri
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) se += __shfl_xor_sync(0xffffffffu, se, o);
     const float lse = mx + logf(se);
-    lse2 = lse * lse;
+    lse2 += lse * lse;
     if (lane == 0) lse_out[t] = lse;
 
     float my_aff = 0.f;
@@ -188,6 +206,7 @@ gate_topk_blocked_kernel(const float* __restrict__ logits, const float* __restri
     if (lane < K) {
       sel[static_cast<long long>(t) * K + lane] = my_idx;
       weights[static_cast<long long>(t) * K + lane] = my_aff / (aff_sum + 1e-9f);
+      if (chunk_hist) atomicAdd(&s_hist[my_idx], 1);
     }
   }
   if (lane == 0) s_lse2[warp] = lse2;
@@ -197,6 +216,7 @@ gate_topk_blocked_kernel(const float* __restrict__ logits, const float* __restri
     for (int i = 0; i < kTopkWarpsPerBlock; ++i) s += s_lse2[i];
     z_partial[blockIdx.x] = s;
   }
+  if (chunk_hist) topk_hist_store(s_hist, E, chunk_hist);
 }
 
 // Deterministic final reduction of the z-loss partials (fixed order, one block).
@@ -358,6 +378,149 @@ route_scatter_kernel(const int* __restrict__ sel, int n, int E, const int* __res
   }
 }
 
+// The same tables from the chunk histograms of the top-k kernel, and the gather in the same launch.  A chunk is the
+// `tokens` (at most 128) consecutive tokens of one top-k block, a token selects an expert at most once; so the rank of an
+// entry among its expert's entries of the chunk is a population count over a bit mask of the tokens before it, and no warp
+// walks its entries in order.  Every latent row is read ONCE and written to its K places (a gather by destination row reads
+// it K times).  Blocks beyond the last chunk, and every block besides its chunk, publish the tables and zero the pad rows of
+// experts b, b + gridDim.x, ...; block 0 also adds up the z-loss.
+constexpr int kDirectChunks = 128;
+constexpr int kMaxPerWarp = 16;
+constexpr int kMaskWords = kTopkWarpsPerBlock * kMaxPerWarp / 32;
+
+__global__ void __launch_bounds__(256)
+route_gather_kernel(const int* __restrict__ sel, int T, int E, int K, int tokens, int chunks, int direct,
+                    const int* __restrict__ hist, const float* __restrict__ z_partial, float z_scale, float* __restrict__ z_loss,
+                    const lmoe_route r, const uint4* __restrict__ src, int vec_per_row, uint4* __restrict__ dst) {
+  __shared__ int s_cnt[LMOE_MAX_EXPERTS], s_base[LMOE_MAX_EXPERTS];
+  __shared__ int s_off[LMOE_MAX_EXPERTS + 1], s_poff[LMOE_MAX_EXPERTS + 1];
+  __shared__ unsigned s_mask[LMOE_MAX_EXPERTS][kMaskWords];
+  __shared__ int s_wsum[2][8];
+  __shared__ double s_z[256];
+  extern __shared__ int s_row[];  // [tokens * K] padded row of every entry of the chunk
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int chunk = blockIdx.x;
+  const int mask_words = (tokens + 31) / 32;
+
+  for (int i = tid; i < E * mask_words; i += 256) s_mask[i / mask_words][i % mask_words] = 0u;
+  if (direct) {
+    // thread t sums a share of the chunks for expert t % E': per = threads per expert (E <= 128 leaves room for more)
+    const int per = E <= 64 ? 4 : (E <= 128 ? 2 : 1);
+    if (tid < E) s_cnt[tid] = s_base[tid] = 0;
+    __syncthreads();
+    const int e = tid / per, part = tid - e * per;
+    if (e < E) {
+      int before = 0, all = 0;
+#pragma unroll 8
+      for (int c = part; c < chunks; c += per) {
+        const int v = hist[static_cast<long long>(c) * E + e];
+        all += v;
+        if (c < chunk) before += v;
+      }
+      atomicAdd(&s_cnt[e], all);
+      atomicAdd(&s_base[e], before);
+    }
+  } else if (tid < E) {
+    s_cnt[tid] = r.counts[tid];
+    if (chunk < chunks) s_base[tid] = hist[static_cast<long long>(chunk) * E + tid];
+  }
+  __syncthreads();
+  {  // canonical and padded offsets of every expert (blockDim.x == LMOE_MAX_EXPERTS == 256)
+    const int c = (tid < E) ? s_cnt[tid] : 0;
+    const int pc = (c + LMOE_ROW_PAD - 1) / LMOE_ROW_PAD * LMOE_ROW_PAD;
+    int ic = c, ip = pc;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int a = __shfl_up_sync(0xffffffffu, ic, o), b = __shfl_up_sync(0xffffffffu, ip, o);
+      if (lane >= o) {
+        ic += a;
+        ip += b;
+      }
+    }
+    if (lane == 31) {
+      s_wsum[0][warp] = ic;
+      s_wsum[1][warp] = ip;
+    }
+    __syncthreads();
+    int wc = 0, wp = 0;
+    for (int w = 0; w < warp; ++w) {
+      wc += s_wsum[0][w];
+      wp += s_wsum[1][w];
+    }
+    if (tid < E) {
+      s_off[tid] = wc + ic - c;
+      s_poff[tid] = wp + ip - pc;
+      if (tid == E - 1) {
+        s_off[E] = wc + ic;
+        s_poff[E] = wp + ip;
+      }
+    }
+    __syncthreads();
+  }
+  // ---- tables and pad rows of this block's experts
+  for (int e = blockIdx.x; e < E; e += gridDim.x) {
+    if (tid == 0) {
+      if (direct) r.counts[e] = s_cnt[e];
+      r.offsets[e] = s_off[e];
+      r.pad_offsets[e] = s_poff[e];
+    }
+    for (int t = s_poff[e] / LMOE_ROW_PAD + tid; t < s_poff[e + 1] / LMOE_ROW_PAD; t += 256) r.tile_expert[t] = e;
+    const int first = s_poff[e] + s_cnt[e];
+    for (int q = first + tid; q < s_poff[e + 1]; q += 256) r.row_src[q] = -1;
+    if (dst)
+      for (long long i = static_cast<long long>(first) * vec_per_row + tid; i < static_cast<long long>(s_poff[e + 1]) * vec_per_row;
+           i += 256)
+        dst[i] = make_uint4(0, 0, 0, 0);
+  }
+  if (blockIdx.x == 0) {
+    if (tid == 0) {
+      r.offsets[E] = s_off[E];
+      r.pad_offsets[E] = s_poff[E];
+      r.n_tiles[0] = s_poff[E] / LMOE_ROW_PAD;
+    }
+    double acc = 0.0;
+    for (int i = tid; i < chunks; i += 256) acc += static_cast<double>(z_partial[i]);
+    s_z[tid] = acc;
+    __syncthreads();
+    for (int o = 128; o > 0; o >>= 1) {
+      if (tid < o) s_z[tid] += s_z[tid + o];
+      __syncthreads();
+    }
+    if (tid == 0) z_loss[0] = static_cast<float>(s_z[0] * static_cast<double>(z_scale));
+  }
+  if (chunk >= chunks) return;
+
+  // ---- this chunk's entries
+  const int t0 = chunk * tokens;
+  const int n_tok = min(tokens, T - t0), n = n_tok * K;
+  const int* my = sel + static_cast<long long>(t0) * K;
+  for (int i = tid; i < n; i += 256) {
+    const int tok = i / K;
+    atomicOr(&s_mask[my[i]][tok >> 5], 1u << (tok & 31));
+  }
+  __syncthreads();
+  for (int i = tid; i < n; i += 256) {
+    const int tok = i / K, e = my[i];
+    int rank = s_base[e];
+    for (int w = 0; w < (tok >> 5); ++w) rank += __popc(s_mask[e][w]);
+    rank += __popc(s_mask[e][tok >> 5] & ((1u << (tok & 31)) - 1u));
+    const int row = s_poff[e] + rank, flat = t0 * K + i;
+    r.perm[s_off[e] + rank] = flat;
+    r.pos[flat] = row;
+    r.row_src[row] = flat;
+    s_row[i] = row;
+  }
+  if (!dst) return;
+  __syncthreads();
+  for (int tok = warp; tok < n_tok; tok += 8) {
+    const uint4* from = src + static_cast<long long>(t0 + tok) * vec_per_row;
+    for (int v = lane; v < vec_per_row; v += 32) {
+      const uint4 x = from[v];
+      for (int k = 0; k < K; ++k) dst[static_cast<long long>(s_row[tok * K + k]) * vec_per_row + v] = x;
+    }
+  }
+}
+
 // Router bias update from the routing histogram.  The expected load per expert is taken from the histogram itself
 // (sum of the counts / E = tokens * K / E): a histogram summed over several ranks then gives the global figure
 // whatever the ranks' own token counts were.  One block; E <= LMOE_MAX_EXPERTS threads carry one expert each.
@@ -405,6 +568,7 @@ static void configure_route_kernels() {
   prefer_max_carveout(route_hist_kernel);
   prefer_max_carveout(route_scan_chunks_kernel);
   prefer_max_carveout(route_scatter_kernel);
+  prefer_max_carveout(route_gather_kernel);
   return 0;
   });
 }
@@ -421,25 +585,96 @@ static inline int check_shape(const lmoe_shape* s) {
 
 using namespace lmoe;
 
+static void launch_topk(const lmoe_shape* s, const float* logits, const float* bias, int32_t* sel, float* weights, float* lse,
+                        float* z_partial, int per_warp, int* chunk_hist, cudaStream_t st) {
+  configure_route_kernels();
+  const int per_block = kTopkWarpsPerBlock * per_warp;
+  const int blocks = (s->T + per_block - 1) / per_block;
+  const int thr = kTopkWarpsPerBlock * 32;
+  switch (s->E) {  // blocked layout when the expert count is a multiple of the warp size
+    case 32: gate_topk_blocked_kernel<1><<<blocks, thr, 0, st>>>(logits, bias, s->T, s->K, sel, weights, lse, z_partial, per_warp, chunk_hist); break;
+    case 64: gate_topk_blocked_kernel<2><<<blocks, thr, 0, st>>>(logits, bias, s->T, s->K, sel, weights, lse, z_partial, per_warp, chunk_hist); break;
+    case 128: gate_topk_blocked_kernel<4><<<blocks, thr, 0, st>>>(logits, bias, s->T, s->K, sel, weights, lse, z_partial, per_warp, chunk_hist); break;
+    case 256: gate_topk_blocked_kernel<8><<<blocks, thr, 0, st>>>(logits, bias, s->T, s->K, sel, weights, lse, z_partial, per_warp, chunk_hist); break;
+    default:
+      gate_topk_kernel<<<blocks, thr, 0, st>>>(logits, bias, s->T, s->E, s->K, sel, weights, lse, z_partial, per_warp, chunk_hist);
+  }
+  count_launch();
+}
+
 extern "C" int lmoe_gate_topk_fwd(const lmoe_shape* s, const float* logits, const float* expert_bias, float z_coef,
                                   int32_t* sel, float* weights, float* lse, float* z_partial, float* z_loss,
                                   void* stream) {
   if (int rc = check_shape(s)) return rc;
   if (!logits || !expert_bias || !sel || !weights || !lse || !z_partial || !z_loss) return LMOE_ERR_ARG;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  configure_route_kernels();
+  launch_topk(s, logits, expert_bias, sel, weights, lse, z_partial, 1, nullptr, st);
   const int blocks = (s->T + kTopkWarpsPerBlock - 1) / kTopkWarpsPerBlock;
-  const int thr = kTopkWarpsPerBlock * 32;
-  switch (s->E) {  // blocked layout when the expert count is a multiple of the warp size
-    case 32: gate_topk_blocked_kernel<1><<<blocks, thr, 0, st>>>(logits, expert_bias, s->T, s->K, sel, weights, lse, z_partial); break;
-    case 64: gate_topk_blocked_kernel<2><<<blocks, thr, 0, st>>>(logits, expert_bias, s->T, s->K, sel, weights, lse, z_partial); break;
-    case 128: gate_topk_blocked_kernel<4><<<blocks, thr, 0, st>>>(logits, expert_bias, s->T, s->K, sel, weights, lse, z_partial); break;
-    case 256: gate_topk_blocked_kernel<8><<<blocks, thr, 0, st>>>(logits, expert_bias, s->T, s->K, sel, weights, lse, z_partial); break;
-    default:
-      gate_topk_kernel<<<blocks, thr, 0, st>>>(logits, expert_bias, s->T, s->E, s->K, sel, weights, lse, z_partial);
-  }
-  count_launch(2);
+  count_launch();
   zloss_finalize_kernel<<<1, 256, 0, st>>>(z_partial, blocks, z_coef / static_cast<float>(s->T), z_loss);
+  cudaError_t e = cudaGetLastError();
+  return e == cudaSuccess ? 0 : static_cast<int>(e);
+}
+
+// ----------------------------------------------------------------------------- routing in two or three launches
+// lmoe_topk_hist_fwd + lmoe_route_gather_fwd do what lmoe_gate_topk_fwd, lmoe_route_permute and lmoe_gather_rows do in six
+// launches.  Tokens are cut into chunks of one top-k block each.  Up to kDirectChunks of them, every block of the scatter
+// adds up the chunk histograms itself (they are a few KB per block, from L2); beyond, a scan kernel does it once.
+static int tokens_per_warp(int T) {
+  const int direct = (T + kTopkWarpsPerBlock * kDirectChunks - 1) / (kTopkWarpsPerBlock * kDirectChunks);
+  if (direct <= 4) return direct;                                       // up to 4,096 tokens
+  const int r = (T + kTopkWarpsPerBlock * 1024 - 1) / (kTopkWarpsPerBlock * 1024);  // about 1,024 chunks
+  return r < 4 ? 4 : (r > kMaxPerWarp ? kMaxPerWarp : r);
+}
+static int route_chunks(const lmoe_shape* s) {
+  const int per_block = kTopkWarpsPerBlock * tokens_per_warp(s->T);
+  return (s->T + per_block - 1) / per_block;
+}
+
+extern "C" size_t lmoe_route_fwd_workspace_bytes(const lmoe_shape* s) {
+  if (check_shape(s)) return 0;
+  const size_t chunks = static_cast<size_t>(route_chunks(s));
+  return (chunks * s->E + (chunks + 3) / 4 * 4) * sizeof(int);
+}
+
+extern "C" int lmoe_topk_hist_fwd(const lmoe_shape* s, const float* logits, const float* expert_bias, int32_t* sel,
+                                  float* weights, float* lse, void* workspace, size_t workspace_bytes, void* stream) {
+  if (int rc = check_shape(s)) return rc;
+  if (!logits || !expert_bias || !sel || !weights || !lse || !workspace) return LMOE_ERR_ARG;
+  if (workspace_bytes < lmoe_route_fwd_workspace_bytes(s)) return LMOE_ERR_WORKSPACE;
+  int* hist = static_cast<int*>(workspace);
+  float* z_partial = reinterpret_cast<float*>(hist + static_cast<size_t>(route_chunks(s)) * s->E);
+  launch_topk(s, logits, expert_bias, sel, weights, lse, z_partial, tokens_per_warp(s->T), hist, static_cast<cudaStream_t>(stream));
+  cudaError_t e = cudaGetLastError();
+  return e == cudaSuccess ? 0 : static_cast<int>(e);
+}
+
+extern "C" int lmoe_route_gather_fwd(const lmoe_shape* s, const int32_t* sel, void* workspace, size_t workspace_bytes,
+                                     float z_coef, float* z_loss, const lmoe_route* r, const void* src, int row_bytes, void* dst,
+                                     void* stream) {
+  if (int rc = check_shape(s)) return rc;
+  if (!sel || !workspace || !z_loss || !r || !r->counts || !r->offsets || !r->perm || !r->pad_offsets || !r->pos ||
+      !r->row_src || !r->tile_expert || !r->n_tiles || (src == nullptr) != (dst == nullptr))
+    return LMOE_ERR_ARG;
+  if (src && (row_bytes <= 0 || (row_bytes & 15) != 0)) return LMOE_ERR_SHAPE;
+  if (workspace_bytes < lmoe_route_fwd_workspace_bytes(s)) return LMOE_ERR_WORKSPACE;
+  configure_route_kernels();
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  const int chunks = route_chunks(s), tokens = kTopkWarpsPerBlock * tokens_per_warp(s->T);
+  int* hist = static_cast<int*>(workspace);
+  const float* z_partial = reinterpret_cast<float*>(hist + static_cast<size_t>(chunks) * s->E);
+  const bool direct = chunks <= kDirectChunks;
+  if (!direct) {
+    count_launch();
+    route_scan_chunks_kernel<<<s->E, 256, 0, st>>>(hist, chunks, s->E, r->counts);
+  }
+  // at least one block per expert: the pad rows of an expert (up to 127 rows to zero) are a block's extra duty
+  const int blocks = chunks > s->E ? chunks : s->E;
+  const size_t smem = static_cast<size_t>(tokens) * s->K * sizeof(int);
+  count_launch();
+  route_gather_kernel<<<blocks, 256, smem, st>>>(sel, s->T, s->E, s->K, tokens, chunks, direct ? 1 : 0, hist, z_partial,
+                                                 z_coef / static_cast<float>(s->T), z_loss, *r, static_cast<const uint4*>(src),
+                                                 row_bytes / 16, static_cast<uint4*>(dst));
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : static_cast<int>(e);
 }

@@ -218,7 +218,8 @@ struct LatentLayout {
   size_t x_rows = 0, hidden = 0;                                      // bf16 experts (x_rows: x_sorted, or the latent rows)
   size_t xq = 0, hq = 0, wguq = 0, wdq = 0, scal = 0;                 // e4m3 experts
   size_t bytes = 0;
-  LatentLayout(const Sizes& d, bool fp8, bool gather) {
+  LatentLayout(const Sizes& d, bool fp8, bool gather, bool keep = true) {  // !keep: no backward follows, no gate / up
+
     Carver c;
     const int64_t T = d.T, P = d.P;
     logits = c.take(T * d.E * 4);
@@ -226,9 +227,9 @@ struct LatentLayout {
     lse = c.take(T * 4);
     route = c.take(d.route_ints() * 4);
     act_cat = c.take(T * (d.L + d.Fs) * 2);
-    h1_s = c.take(T * 2 * d.Fs * 2);
+    h1_s = c.take(keep ? T * 2 * d.Fs * 2 : 0);
     y_sorted = c.take(P * d.L * 2);
-    h1 = c.take(P * 2 * d.F * 2);
+    h1 = c.take(keep ? P * 2 * d.F * 2 : 0);
     if (fp8) {
       xq = c.take(P * d.L);
       hq = c.take(P * d.F);
@@ -268,13 +269,16 @@ Sizes latent_sizes(const Tensor& x2d, const Tensor& wgu, const Tensor& wds, int6
   return Sizes(x2d.size(0), x2d.size(1), wgu.size(1), wgu.size(0), top_k, wgu.size(2) / 2, wds.size(1));
 }
 
-LatentOut latent_forward(const Sizes& d, const LatentOps& o, const Tensor& bias, float z_coef, bool fp8,
+// Up to this many tokens the dense GEMMs leave SMs free: the router chain and the shared expert then run side by side.
+constexpr int kForkForwardTokens = 2048;
+
+LatentOut latent_forward(const Sizes& d, const LatentOps& o, const Tensor& bias, float z_coef, bool fp8, bool keep,
                          const c10::optional<Tensor>& forced_sel, Views* views) {
   const auto stream = at::cuda::getCurrentCUDAStream();
   void* st = stream.stream();
   int32_t* status = status_word(kLatentFwd);
   const bool gather = tma_gather_enabled() && !fp8 && d.L % 128 == 0;  // whole 128-column tiles of the weight gradient
-  const LatentLayout at_(d, fp8, gather);
+  const LatentLayout at_(d, fp8, gather, keep);
   const int64_t T = d.T, P = d.P;
 
   LatentOut r;
@@ -289,8 +293,8 @@ LatentOut latent_forward(const Sizes& d, const LatentOps& o, const Tensor& bias,
 
   // scratch that nothing keeps
   Carver c;
-  const size_t ws_bytes = std::max<size_t>(16, lmoe_route_workspace_bytes(&d.s));
-  const size_t t_ws = c.take(ws_bytes), t_zp = c.take((T + 7) / 8 * 4);
+  const size_t ws_bytes = std::max<size_t>({16, lmoe_route_workspace_bytes(&d.s), lmoe_route_fwd_workspace_bytes(&d.s)});
+  const size_t t_ws = c.take(ws_bytes), t_zp = forced_sel ? c.take((T + 7) / 8 * 4) : 0;
   const size_t t_lat = gather ? 0 : c.take(T * d.L * 2);
   const size_t t_xs = (fp8 || (gather && views)) ? c.take(P * d.L * 2) : 0;
   const size_t t_hid = fp8 ? c.take(P * d.F * 2) : 0;
@@ -302,9 +306,9 @@ LatentOut latent_forward(const Sizes& d, const LatentOps& o, const Tensor& bias,
   float* lse = reinterpret_cast<float*>(sv + at_.lse);
   const lmoe_route route = d.route(sv + at_.route, r.counts.data_ptr<int32_t>());
   void* act_cat = sv + at_.act_cat;
-  void* h1_s = sv + at_.h1_s;
+  void* h1_s = keep ? sv + at_.h1_s : nullptr;
   void* y_sorted = sv + at_.y_sorted;
-  void* h1 = sv + at_.h1;
+  void* h1 = keep ? sv + at_.h1 : nullptr;
   void* x_latent = gather ? sv + at_.x_rows : tv + t_lat;
   void* x_sorted = fp8 ? tv + t_xs : (gather ? (views ? tv + t_xs : nullptr) : sv + at_.x_rows);
   void* hidden = fp8 ? tv + t_hid : sv + at_.hidden;
@@ -312,18 +316,32 @@ LatentOut latent_forward(const Sizes& d, const LatentOps& o, const Tensor& bias,
 
   if (gather)  // the pad rows of the routed layout read a row of zeros behind the T latent rows
     C10_CUDA_CHECK(cudaMemsetAsync(static_cast<char*>(x_latent) + T * d.L * 2, 0, d.L * 2, stream.stream()));
-  LMOE(lmoe_xproj_fwd, &d.s, o.x.data_ptr(), o.wg.data_ptr(), o.wdn.data_ptr(), logits, x_latent, status, st);
-  // One stream: the routing kernels' static shared memory does not fit on an SM beside a GEMM CTA.
-  LMOE(lmoe_gate_topk_fwd, &d.s, logits, bias.data_ptr<float>(), z_coef, sel, weights, lse,
-       reinterpret_cast<float*>(tv + t_zp), r.z_loss.data_ptr<float>(), st);
+  const bool forked = d.T <= kForkForwardTokens && !forced_sel;
+  c10::optional<Fork> fork;
+  if (forked) fork.emplace(stream);
   if (forced_sel) {  // parity tests: another selection, the gating weights recomputed from this pass's own logits
+    LMOE(lmoe_xproj_fwd, &d.s, o.x.data_ptr(), o.wg.data_ptr(), o.wdn.data_ptr(), logits, x_latent, status, st);
+    LMOE(lmoe_gate_topk_fwd, &d.s, logits, bias.data_ptr<float>(), z_coef, sel, weights, lse,
+         reinterpret_cast<float*>(tv + t_zp), r.z_loss.data_ptr<float>(), st);
     r.sel.copy_(*forced_sel);
     Tensor aff = at::sigmoid(view_of(r.saved, at_.logits, {T, d.E}, at::kFloat)).gather(1, r.sel.to(at::kLong));
     view_of(r.saved, at_.weights, {T, d.K}, at::kFloat).copy_(aff / (aff.sum(-1, true) + 1e-9));
+    LMOE(lmoe_route_permute, &d.s, sel, &route, tv + t_ws, ws_bytes, st);
+    if (x_sorted) LMOE(lmoe_gather_rows, x_latent, route.row_src, d.K, P, d.L, route.n_tiles, x_sorted, st);
+    LMOE(lmoe_shared_gateup_fwd, &d.s, o.x.data_ptr(), o.wgus.data_ptr(), h1_s, act_cat, status, st);
+  } else {
+    // Small batches: [x_latent, shared gate_up] on the side stream beside [logits, top-k].  At larger ones every GEMM
+    // fills the SMs and the routing kernels' static shared memory does not fit beside a GEMM CTA: one stream.
+    void* side = forked ? fork->side() : st;
+    if (forked) fork->to_side();
+    LMOE(lmoe_xproj_fwd, &d.s, o.x.data_ptr(), o.wg.data_ptr(), nullptr, logits, nullptr, status, st);
+    LMOE(lmoe_xproj_fwd, &d.s, o.x.data_ptr(), nullptr, o.wdn.data_ptr(), nullptr, x_latent, status, side);
+    LMOE(lmoe_topk_hist_fwd, &d.s, logits, bias.data_ptr<float>(), sel, weights, lse, tv + t_ws, ws_bytes, st);
+    if (forked) fork->to_main();
+    LMOE(lmoe_route_gather_fwd, &d.s, sel, tv + t_ws, ws_bytes, z_coef, r.z_loss.data_ptr<float>(), &route,
+         x_sorted ? x_latent : nullptr, 2 * d.L, x_sorted, st);
+    LMOE(lmoe_shared_gateup_fwd, &d.s, o.x.data_ptr(), o.wgus.data_ptr(), h1_s, act_cat, status, side);
   }
-  LMOE(lmoe_route_permute, &d.s, sel, &route, tv + t_ws, ws_bytes, st);
-  if (x_sorted) LMOE(lmoe_gather_rows, x_latent, route.row_src, d.K, P, d.L, route.n_tiles, x_sorted, st);
-  LMOE(lmoe_shared_gateup_fwd, &d.s, o.x.data_ptr(), o.wgus.data_ptr(), h1_s, act_cat, status, st);
 
   // routed experts in the padded layout
   if (fp8) {
@@ -346,6 +364,7 @@ LatentOut latent_forward(const Sizes& d, const LatentOps& o, const Tensor& bias,
          route.pad_offsets, h1, hidden, y_sorted, status, st);
   }
   // weighted combine, up-projection, shared down-projection, add
+  if (forked) fork->to_main();
   LMOE(lmoe_combine_out_fwd, &d.s, y_sorted, &route, weights, act_cat, o.wds.data_ptr(), o.wup.data_ptr(), r.y.data_ptr(),
        status, st);
 
@@ -492,9 +511,9 @@ const float* scalar_grad(const Tensor& d_z, Tensor& keep) {
 // ---------------------------------------------------------------- non-latent MoE layer
 // The same kernels at the model width (L = D): x itself is gathered into the padded layout and the weighted sum of the
 // expert outputs is added to the shared expert's output (models/moe.py:344-372).
-struct MoeLayout {
+struct MoeLayout {  // !keep: no backward follows, no gate / up
   size_t logits, weights, lse, route, x_sorted, h1, hidden, y_sorted, h1_s, hidden_s, bytes;
-  explicit MoeLayout(const Sizes& d) {
+  explicit MoeLayout(const Sizes& d, bool keep = true) {
     Carver c;
     const int64_t T = d.T, P = d.P;
     logits = c.take(T * d.E * 4);
@@ -502,10 +521,10 @@ struct MoeLayout {
     lse = c.take(T * 4);
     route = c.take(d.route_ints() * 4);
     x_sorted = c.take(P * d.D * 2);
-    h1 = c.take(P * 2 * d.F * 2);
+    h1 = c.take(keep ? P * 2 * d.F * 2 : 0);
     hidden = c.take(P * d.F * 2);
     y_sorted = c.take(P * d.D * 2);
-    h1_s = c.take(T * 2 * d.Fs * 2);
+    h1_s = c.take(keep ? T * 2 * d.Fs * 2 : 0);
     hidden_s = c.take(T * d.Fs * 2);
     bytes = c.bytes;
   }
@@ -520,12 +539,12 @@ Sizes moe_sizes(const Tensor& x2d, const Tensor& wgu, const Tensor& wds, int64_t
   return Sizes(x2d.size(0), x2d.size(1), x2d.size(1), wgu.size(0), top_k, wgu.size(2) / 2, wds.size(1));
 }
 
-LatentOut moe_forward(const Sizes& d, const MoeOps& o, const Tensor& bias, float z_coef,
+LatentOut moe_forward(const Sizes& d, const MoeOps& o, const Tensor& bias, float z_coef, bool keep,
                       const c10::optional<Tensor>& forced_sel) {
   const auto stream = at::cuda::getCurrentCUDAStream();
   void* st = stream.stream();
   int32_t* status = status_word(kMoeFwd);
-  const MoeLayout at_(d);
+  const MoeLayout at_(d, keep);
   const int64_t T = d.T, P = d.P, D = d.D;
   LatentOut r;
   const auto f32 = o.x.options().dtype(at::kFloat).requires_grad(false);
@@ -536,8 +555,8 @@ LatentOut moe_forward(const Sizes& d, const MoeOps& o, const Tensor& bias, float
   r.saved = new_bytes(at_.bytes, o.x);
   char* sv = base_of(r.saved);
   Carver c;
-  const size_t ws_bytes = std::max<size_t>(16, lmoe_route_workspace_bytes(&d.s));
-  const size_t t_ws = c.take(ws_bytes), t_zp = c.take((T + 7) / 8 * 4), t_ysh = c.take(T * D * 2);
+  const size_t ws_bytes = std::max<size_t>({16, lmoe_route_workspace_bytes(&d.s), lmoe_route_fwd_workspace_bytes(&d.s)});
+  const size_t t_ws = c.take(ws_bytes), t_zp = forced_sel ? c.take((T + 7) / 8 * 4) : 0, t_ysh = c.take(T * D * 2);
   Tensor tmp = new_bytes(c.bytes, o.x);
   char* tv = base_of(tmp);
   float* logits = reinterpret_cast<float*>(sv + at_.logits);
@@ -549,20 +568,26 @@ LatentOut moe_forward(const Sizes& d, const MoeOps& o, const Tensor& bias, float
 
   // router: fp32 logits, top-k, z-loss; routing tables                         (moe.py:357-358)
   LMOE(lmoe_gemm_bf16, d.T, d.E, d.D, x, D, 0, o.wg.data_ptr(), D, 0, logits, d.E, LMOE_F32, 1, nullptr, 0, status, st);
-  LMOE(lmoe_gate_topk_fwd, &d.s, logits, bias.data_ptr<float>(), z_coef, sel, weights, lse,
-       reinterpret_cast<float*>(tv + t_zp), r.z_loss.data_ptr<float>(), st);
   if (forced_sel) {  // parity tests only
+    LMOE(lmoe_gate_topk_fwd, &d.s, logits, bias.data_ptr<float>(), z_coef, sel, weights, lse,
+         reinterpret_cast<float*>(tv + t_zp), r.z_loss.data_ptr<float>(), st);
     r.sel.copy_(*forced_sel);
     Tensor aff = at::sigmoid(view_of(r.saved, at_.logits, {T, d.E}, at::kFloat)).gather(1, r.sel.to(at::kLong));
     view_of(r.saved, at_.weights, {T, d.K}, at::kFloat).copy_(aff / (aff.sum(-1, true) + 1e-9));
+    LMOE(lmoe_route_permute, &d.s, sel, &route, tv + t_ws, ws_bytes, st);
+    LMOE(lmoe_gather_rows, x, route.row_src, d.K, P, d.D, route.n_tiles, sv + at_.x_sorted, st);
+  } else {
+    LMOE(lmoe_topk_hist_fwd, &d.s, logits, bias.data_ptr<float>(), sel, weights, lse, tv + t_ws, ws_bytes, st);
+    LMOE(lmoe_route_gather_fwd, &d.s, sel, tv + t_ws, ws_bytes, z_coef, r.z_loss.data_ptr<float>(), &route, x, 2 * d.D,
+         sv + at_.x_sorted, st);
   }
-  LMOE(lmoe_route_permute, &d.s, sel, &route, tv + t_ws, ws_bytes, st);
   // routed experts on x itself                                                 (moe.py:462-470, 509-532)
-  LMOE(lmoe_gather_rows, x, route.row_src, d.K, P, d.D, route.n_tiles, sv + at_.x_sorted, st);
+  void* h1 = keep ? sv + at_.h1 : nullptr;
+  void* h1_s = keep ? sv + at_.h1_s : nullptr;
   LMOE(lmoe_grouped_fwd, P, d.E, d.D, d.F, sv + at_.x_sorted, o.wgu.data_ptr(), o.wde.data_ptr(), route.tile_expert,
-       route.n_tiles, route.pad_offsets, sv + at_.h1, sv + at_.hidden, sv + at_.y_sorted, status, st);
+       route.n_tiles, route.pad_offsets, h1, sv + at_.hidden, sv + at_.y_sorted, status, st);
   // shared expert                                                              (moe.py:351-354, 63-69)
-  LMOE(lmoe_gemm_swiglu_bf16, d.T, d.Fs, d.D, x, D, o.wgus.data_ptr(), D, sv + at_.h1_s, 2 * int64_t(d.Fs), sv + at_.hidden_s,
+  LMOE(lmoe_gemm_swiglu_bf16, d.T, d.Fs, d.D, x, D, o.wgus.data_ptr(), D, h1_s, 2 * int64_t(d.Fs), sv + at_.hidden_s,
        d.Fs, status, st);
   LMOE(lmoe_gemm_bf16, d.T, d.D, d.Fs, sv + at_.hidden_s, d.Fs, 0, o.wds.data_ptr(), d.Fs, 0, tv + t_ysh, D, LMOE_BF16, 1,
        nullptr, 0, status, st);
@@ -671,7 +696,7 @@ class LatentFn : public torch::autograd::Function<LatentFn> {
                                int64_t top_k, double z_coef, bool fp8) {
     const LatentOps o = latent_ops(x, wg, wdn, wup, wgus, wds, wgu, wde);
     const Sizes d = latent_sizes(o.x, o.wgu, o.wds, top_k);
-    LatentOut r = latent_forward(d, o, f32_bias(bias), static_cast<float>(z_coef), fp8, c10::nullopt, nullptr);
+    LatentOut r = latent_forward(d, o, f32_bias(bias), static_cast<float>(z_coef), fp8, true, c10::nullopt, nullptr);
     ctx->set_materialize_grads(false);
     // e4m3: the quantised copies in `saved` replace the bf16 expert weights
     const Tensor none = fp8 ? Tensor() : o.wgu;
@@ -718,7 +743,7 @@ class MoeFn : public torch::autograd::Function<MoeFn> {
     const MoeOps o{cast(x).view({-1, x.size(-1)}), cast(wg), cast(wgus), cast(wds), cast(wgu), cast(wde)};
     cast.run(at::cuda::getCurrentCUDAStream().stream());
     const Sizes d = moe_sizes(o.x, o.wgu, o.wds, top_k);
-    LatentOut r = moe_forward(d, o, f32_bias(bias), static_cast<float>(z_coef), forced);
+    LatentOut r = moe_forward(d, o, f32_bias(bias), static_cast<float>(z_coef), true, forced);
     ctx->set_materialize_grads(false);
     ctx->save_for_backward({o.x, o.wg, o.wgus, o.wds, o.wgu, o.wde, r.sel, r.saved});
     ctx->saved_data["i"] = std::vector<int64_t>{d.E, d.K, d.F, d.Fs};
@@ -770,7 +795,7 @@ std::vector<Tensor> latent_moe(const Tensor& x, const Tensor& wg, const Tensor& 
     return LatentFn::apply(x, wg, wdn, wup, wgus, wds, wgu, wde, bias, top_k, z_coef, fp8);
   const LatentOps o = latent_ops(x, wg, wdn, wup, wgus, wds, wgu, wde);
   LatentOut r = latent_forward(latent_sizes(o.x, o.wgu, o.wds, top_k), o, f32_bias(bias), static_cast<float>(z_coef), fp8,
-                               c10::nullopt, nullptr);
+                               false, c10::nullopt, nullptr);
   return {as_param(r.y.view(x.sizes()), x.scalar_type()), r.z_loss, r.sel, r.counts};
 }
 
@@ -784,7 +809,7 @@ std::vector<Tensor> moe(const Tensor& x, const Tensor& wg, const Tensor& wgus, c
   Caster cast;
   const MoeOps o{cast(x).view({-1, x.size(-1)}), cast(wg), cast(wgus), cast(wds), cast(wgu), cast(wde)};
   cast.run(at::cuda::getCurrentCUDAStream().stream());
-  LatentOut r = moe_forward(moe_sizes(o.x, o.wgu, o.wds, top_k), o, f32_bias(bias), static_cast<float>(z_coef), forced_sel);
+  LatentOut r = moe_forward(moe_sizes(o.x, o.wgu, o.wds, top_k), o, f32_bias(bias), static_cast<float>(z_coef), false, forced_sel);
   return {as_param(r.y.view(x.sizes()), x.scalar_type()), r.z_loss, r.sel, r.counts};
 }
 
@@ -804,7 +829,7 @@ py::tuple latent_fwd_raw(const Tensor& x, const Tensor& wg, const Tensor& wdn, c
   const LatentOps o = latent_ops(x, wg, wdn, wup, wgus, wds, wgu, wde);
   Views views;
   LatentOut r = latent_forward(latent_sizes(o.x, o.wgu, o.wds, top_k), o, f32_bias(bias), static_cast<float>(z_coef), fp8,
-                               forced_sel, capture ? &views : nullptr);
+                               true, forced_sel, capture ? &views : nullptr);
   return py::make_tuple(as_param(r.y.view(x.sizes()), x.scalar_type()), r.z_loss, r.sel, r.counts, r.saved, dict_of(views));
 }
 
