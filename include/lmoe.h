@@ -419,6 +419,24 @@ int lmoe_ep_flag_barrier(void* const* peer_flags, int32_t* epoch_counter, int ra
  * 128 * n_tiles_dev[0] rows are read and written (padded routed layout). */
 int lmoe_fp8_quantize(const void* x_bf16, int64_t rows, int row_len, const int32_t* n_tiles_dev, void* q_e4m3,
                       float* amax, float* deq, void* stream);
+/* The two passes of lmoe_fp8_quantize for up to LMOE_FP8_MAX_TENSORS tensors per launch.  lmoe_fp8_amax: amax[0] =
+ * max(amax[0], max |x|) (the caller zeroes it); lmoe_fp8_cast: q = e4m3(x * 448 / amax[0]), deq[0] = amax[0] / 448. */
+#define LMOE_FP8_MAX_TENSORS 3
+typedef struct lmoe_fp8_tensor {
+  const void* x;
+  void* q;
+  int64_t rows;
+  int32_t row_len;
+  const int32_t* n_tiles;   /* NULL, or device scalar: only the first 128 * n_tiles[0] rows */
+  float* amax;
+  float* deq;
+} lmoe_fp8_tensor;
+int lmoe_fp8_amax(int count, const lmoe_fp8_tensor* t, void* stream);
+int lmoe_fp8_cast(int count, const lmoe_fp8_tensor* t, void* stream);
+/* lmoe_combine_bwd with d_y_sorted leaving as e4m3 (d_y_q[P, L] bytes): the per-tensor maximum comes from d_routed and the
+ * weights (amax[0] zeroed by the caller), so the bf16 rows are neither written nor read again. */
+int lmoe_fp8_combine_bwd(const lmoe_shape* s, const void* d_routed, const void* y_sorted, const float* weights,
+                         const lmoe_route* r, float* amax, float* deq, void* d_y_q, float* d_weights, void* stream);
 /* C[M,N] bf16 = deq_a * deq_b * A_q[M,K] * B_q[N,K]^T; operand major-ness as in lmoe_gemm_bf16. */
 int lmoe_gemm_fp8(int M, int N, int K, const void* A, int64_t lda, int a_mn, const void* B, int64_t ldb, int b_mn,
                   const float* deq_a, const float* deq_b, void* C, int64_t ldc, int32_t* status, void* stream);
@@ -426,6 +444,15 @@ int lmoe_gemm_fp8(int M, int N, int K, const void* A, int64_t lda, int a_mn, con
 int lmoe_grouped_gateup_fp8(int64_t P, int E, int L, int F, const void* xq, const void* wq, const float* deq_x,
                             const float* deq_w, const int32_t* tile_expert, const int32_t* n_tiles, void* h1,
                             void* hidden, int32_t* status, void* stream);
+/* The same, amax_hidden[0] = max(amax_hidden[0], max |hidden|) on the way (may be NULL). */
+int lmoe_grouped_gateup_fp8_amax(int64_t P, int E, int L, int F, const void* xq, const void* wq, const float* deq_x,
+                                 const float* deq_w, const int32_t* tile_expert, const int32_t* n_tiles, void* h1, void* hidden,
+                                 float* amax_hidden, int32_t* status, void* stream);
+/* Routed d_hidden with the SwiGLU adjoint in the epilogue: dyq[P,L], wdq[E,F,L] e4m3, h1[P,2F] -> d_h1[P,2F] bf16, and
+ * amax_d_h1[0] = max(amax_d_h1[0], max |d_h1|) (may be NULL). */
+int lmoe_grouped_swiglu_bwd_fp8(int64_t P, int E, int L, int F, const void* dyq, const void* wdq, const float* deq_dy,
+                                const float* deq_wd, const int32_t* tile_expert, const int32_t* n_tiles, const void* h1,
+                                void* d_h1, float* amax_d_h1, int32_t* status, void* stream);
 /* out[P,N] bf16 = aq[P,K] * Bq[e]: Bq stacked [E,K,N] (b_mn = 1: forward down GEMM, models/moe.py:828) or
  * [E,N,K] (b_mn = 0: the same weights as dgrad operand). */
 int lmoe_grouped_rows_fp8(int64_t P, int E, int K, int N, const void* aq, const void* bq, int b_mn, const float* deq_a,

@@ -98,6 +98,11 @@ SIGNATURES = {
     "lmoe_epd_sum": (c_int, [P, P, c_int64, c_int, c_int, c_int, c_int, c_int64, P, c_int64, P]),
     "lmoe_ep_flag_barrier": (c_int, [P, P, c_int, c_int, P, P]),
     "lmoe_fp8_quantize": (c_int, [P, c_int64, c_int, P, P, P, P, P]),
+    "lmoe_fp8_amax": (c_int, [c_int, P, P]),
+    "lmoe_fp8_cast": (c_int, [c_int, P, P]),
+    "lmoe_fp8_combine_bwd": (c_int, [SP, P, P, P, RP, P, P, P, P, P]),
+    "lmoe_grouped_gateup_fp8_amax": (c_int, [c_int64, c_int, c_int, c_int, P, P, P, P, P, P, P, P, P, P, P]),
+    "lmoe_grouped_swiglu_bwd_fp8": (c_int, [c_int64, c_int, c_int, c_int, P, P, P, P, P, P, P, P, P, P, P]),
     "lmoe_gemm_fp8": (c_int, [c_int, c_int, c_int, P, c_int64, c_int, P, c_int64, c_int, P, P, P, c_int64, P, P]),
     "lmoe_grouped_gateup_fp8": (c_int, [c_int64, c_int, c_int, c_int, P, P, P, P, P, P, P, P, P, P]),
     "lmoe_grouped_rows_fp8": (c_int, [c_int64, c_int, c_int, c_int, P, P, c_int, P, P, P, P, P, P, P]),

@@ -164,6 +164,7 @@ static int dispatch(const GemmCall& c, int bn, const GemmParams& p, int grid, cu
     // ---- e4m3 ----
     LMOE_CASE_MAJORS(EPI_BF16, GRP_NONE, 1)
     LMOE_CASE(0, 1, 256, EPI_SWIGLU, GRP_M, 1)
+    LMOE_CASE(0, 0, 128, EPI_SWIGLU_BWD, GRP_M, 1)
     LMOE_CASE_BN(0, 1, EPI_BF16, GRP_M, 1)
     LMOE_CASE_BN(0, 0, EPI_BF16, GRP_M, 1)
     LMOE_CASE_BN(1, 1, EPI_BF16, GRP_K, 1)
@@ -501,6 +502,7 @@ int launch_gemm(const GemmCall& c) {
   p.pad_offsets = c.pad_offsets;
   p.deq_a = c.deq_a;
   p.deq_b = c.deq_b;
+  p.amax = c.amax;
   p.aux = c.aux;
   p.ld_aux = c.ld_aux;
   p.a_rows = c.a_rows;

@@ -69,6 +69,7 @@ struct alignas(64) GemmParams {
   const int* pad_offsets;  // GRP_K
   const float* deq_a;      // e4m3: per-tensor de-scale factors (amax / 448) of A and B, device scalars
   const float* deq_b;
+  float* amax;             // e4m3 operands, SwiGLU epilogues: max |hidden| / max |d_h1| (bf16-rounded), device scalar or NULL
   const void* aux;         // EPI_SWIGLU_BWD: h1 [rows, 2*N] bf16 (gate | up), row stride ld_aux elements
   long long ld_aux;
   CUtensorMap tmAux;       // EPI_SWIGLU_BWD: the same tensor as 128-row boxes of 64 columns (128-byte swizzle), staged by TMA
@@ -451,6 +452,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_kernel(const __grid_cons
     int acc = 0;
     uint32_t acc_phase = 0;
     bool ok = true;
+    constexpr bool kAmax = (ESZ == 1 && (EPI == EPI_SWIGLU || EPI == EPI_SWIGLU_BWD));
+    __nv_bfloat162 vmax = __float2bfloat162_rn(0.f);
     // EPI_SWIGLU_BWD (BN = 128): group g owns the tile's columns [64 g, 64 g + 64), i.e. slabs 2g and 2g + 1, and the
     // saved gate / up of those columns arrive as TWO 128-row boxes of 64 columns (128-byte rows, 128-byte swizzle: a
     // TMA load costs the SM one request slot per box row whatever the row's width, so 64-column boxes halve what the
@@ -594,6 +597,16 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_kernel(const __grid_cons
             ph[j] = pack_bf16x2(silu_f(g0) * u0, silu_f(g1) * u1);
           }
         }
+        if (kAmax) {  // the values as they will be stored
+#pragma unroll
+          for (int j = 0; j < 16; ++j) {
+            if (kSwiglu) vmax = __hmax2(vmax, __habs2(*reinterpret_cast<const __nv_bfloat162*>(&ph[j])));
+            if (EPI == EPI_SWIGLU_BWD) {
+              vmax = __hmax2(vmax, __habs2(*reinterpret_cast<const __nv_bfloat162*>(&pk[j])));
+              vmax = __hmax2(vmax, __habs2(*reinterpret_cast<const __nv_bfloat162*>(&pu[j])));
+            }
+          }
+        }
         if (kSwiglu && p.hidden_only) {
           // one store per slab instead of three: the gate and up slabs' buffers take the hidden slabs in turn
           uint8_t* hbuf = sbuf0 + buf * S::kSlabBytes;
@@ -669,6 +682,12 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_kernel(const __grid_cons
         acc ^= 1;
         if (acc == 0) acc_phase ^= 1;
       }
+    }
+    if (kAmax && p.amax) {
+      float m = fmaxf(__low2float(vmax), __high2float(vmax));
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+      if (lane == 0) atomicMax(reinterpret_cast<int*>(p.amax), __float_as_int(m));  // non-negative: ordered like integers
     }
     if (issuer) tma_store_wait0();  // staging memory must outlive the last reads
   }

@@ -8,6 +8,7 @@
 #include "../../include/lmoe.h"
 #include "counters.h"
 #include "device_once.h"
+#include "fp8_device.cuh"
 #include "rowops.h"
 
 namespace lmoe {
@@ -149,6 +150,85 @@ combine_bwd_kernel(const uint4* __restrict__ d_routed, const uint4* __restrict__
       for (int o = 16; o > 0; o >>= 1) dot[u] += __shfl_xor_sync(0xffffffffu, dot[u], o);
       if (lane == 0 && flat[u] >= 0) d_w[flat[u]] = dot[u];
     }
+  }
+}
+
+// The same adjoint token by token: one warp takes a token's row of d_routed once and walks its K expert rows (pos), four at
+// a time, so four independent y rows are in flight per lane and no index has to arrive before a row can be asked for by
+// the next one.  Pad rows (any d_y that is not some token's) are zeroed by the blocks that own the experts b, b + gridDim.x..
+// 1.57 M rows of 512 bytes beside the weight gradient GEMM: see the numbers at lmoe_combine_bwd.
+// QUANT: d_y leaves as e4m3 of the bf16-rounded product, scaled by 448 / amax (amax computed by amax_weighted_kernel).
+template <bool QUANT>
+__global__ void __launch_bounds__(kRowWarps * 32)
+combine_bwd_tokens_kernel(const uint4* __restrict__ d_routed, const uint4* __restrict__ y, const float* __restrict__ w,
+                          const int* __restrict__ pos, const int* __restrict__ offsets, const int* __restrict__ pad_offsets,
+                          int T, int E, int K, int vec_per_row, void* __restrict__ d_y, float* __restrict__ d_w,
+                          const float* __restrict__ amax, float* __restrict__ deq) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  float scale = 1.f;
+  if (QUANT) {
+    const float a = amax[0];
+    scale = a > 0.f ? kE4M3Max / a : 1.0f;
+    if (blockIdx.x == 0 && threadIdx.x == 0) deq[0] = a > 0.f ? a / kE4M3Max : 1.0f;
+  }
+  for (int e = blockIdx.x; e < E; e += gridDim.x) {
+    const long long first = pad_offsets[e] + (offsets[e + 1] - offsets[e]), last = pad_offsets[e + 1];
+    for (long long i = first * vec_per_row + threadIdx.x; i < last * vec_per_row; i += blockDim.x) {
+      if (QUANT)
+        static_cast<uint2*>(d_y)[i] = make_uint2(0, 0);
+      else
+        static_cast<uint4*>(d_y)[i] = make_uint4(0, 0, 0, 0);
+    }
+  }
+  for (long long t = static_cast<long long>(blockIdx.x) * kRowWarps + warp; t < T; t += static_cast<long long>(gridDim.x) * kRowWarps) {
+    int my_pos = 0;
+    float my_w = 0.f;
+    if (lane < K) {
+      my_pos = pos[t * K + lane];
+      my_w = w[t * K + lane];
+    }
+    float my_dot = 0.f;
+    for (int k0 = 0; k0 < K; k0 += kGatherUnroll) {
+      long long row[kGatherUnroll];
+      float wk[kGatherUnroll], dot[kGatherUnroll];
+#pragma unroll
+      for (int u = 0; u < kGatherUnroll; ++u) {
+        const int k = min(k0 + u, K - 1);
+        row[u] = static_cast<long long>(__shfl_sync(0xffffffffu, my_pos, k)) * vec_per_row;
+        wk[u] = __shfl_sync(0xffffffffu, my_w, k);
+        dot[u] = 0.f;
+      }
+      for (int v = lane; v < vec_per_row; v += 32) {
+        uint4 y4[kGatherUnroll];
+#pragma unroll
+        for (int u = 0; u < kGatherUnroll; ++u) y4[u] = y[row[u] + v];
+        float g[8];
+        unpack8(d_routed[t * vec_per_row + v], g);
+#pragma unroll
+        for (int u = 0; u < kGatherUnroll; ++u) {
+          if (k0 + u >= K) continue;
+          float yy[8], o[8];
+          unpack8(y4[u], yy);
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            dot[u] = fmaf(g[j], yy[j], dot[u]);
+            o[j] = wk[u] * g[j];
+          }
+          const uint4 packed = pack8(o);
+          if (QUANT)
+            static_cast<uint2*>(d_y)[row[u] + v] = quantize8(packed, scale);
+          else
+            static_cast<uint4*>(d_y)[row[u] + v] = packed;
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < kGatherUnroll; ++u) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) dot[u] += __shfl_xor_sync(0xffffffffu, dot[u], o);
+        if (lane == k0 + u) my_dot = dot[u];
+      }
+    }
+    if (lane < K) d_w[t * K + lane] = my_dot;
   }
 }
 
@@ -305,6 +385,22 @@ int combine_rows(const void* y_sorted, const int* pos, const float* w, int T, in
   return last_error();
 }
 
+int combine_bwd_tokens(const lmoe_shape* s, const void* d_routed, const void* y_sorted, const float* weights,
+                       const lmoe_route* r, void* d_y, float* d_weights, const float* amax, float* deq, cudaStream_t st) {
+  if (!r->pos || !r->offsets || !r->pad_offsets) return LMOE_ERR_ARG;
+  if (s->T <= 0 || s->K <= 0 || s->K > 32 || s->E <= 0) return LMOE_ERR_SHAPE;
+  const int grid = grid_for(s->T, kRowWarps);
+  const int blocks = grid < s->E ? s->E : grid;  // an expert's pad rows are a block's extra duty
+  const uint4 *g = static_cast<const uint4*>(d_routed), *y = static_cast<const uint4*>(y_sorted);
+  if (amax)
+    combine_bwd_tokens_kernel<true><<<blocks, kRowWarps * 32, 0, st>>>(g, y, weights, r->pos, r->offsets, r->pad_offsets, s->T, s->E,
+                                                                      s->K, s->L / 8, d_y, d_weights, amax, deq);
+  else
+    combine_bwd_tokens_kernel<false><<<blocks, kRowWarps * 32, 0, st>>>(g, y, weights, r->pos, r->offsets, r->pad_offsets, s->T, s->E,
+                                                                       s->K, s->L / 8, d_y, d_weights, nullptr, nullptr);
+  return last_error();
+}
+
 }  // namespace lmoe
 
 using namespace lmoe;
@@ -313,11 +409,8 @@ extern "C" int lmoe_combine_bwd(const lmoe_shape* s, const void* d_routed, const
                                 const lmoe_route* r, void* d_y_sorted, float* d_weights, void* stream) {
   if (!s || !d_routed || !y_sorted || !weights || !r || !d_y_sorted || !d_weights) return LMOE_ERR_ARG;
   if ((s->L & 7) != 0) return LMOE_ERR_SHAPE;
-  const long long P = lmoe_padded_rows(s);
-  combine_bwd_kernel<<<grid_for(P, kRowWarps), kRowWarps * 32, 0, static_cast<cudaStream_t>(stream)>>>(
-      static_cast<const uint4*>(d_routed), static_cast<const uint4*>(y_sorted), weights, r->row_src, r->n_tiles, s->K,
-      s->L / 8, static_cast<uint4*>(d_y_sorted), d_weights, P);
-  return last_error();
+  return combine_bwd_tokens(s, d_routed, y_sorted, weights, r, d_y_sorted, d_weights, nullptr, nullptr,
+                            static_cast<cudaStream_t>(stream));
 }
 
 extern "C" int lmoe_swiglu_bwd(int64_t rows, int H, const void* h1, const void* d_hidden, void* d_h1, int64_t ld_d_h1,

@@ -296,7 +296,8 @@ LatentOut latent_forward(const Sizes& d, const LatentOps& o, const Tensor& bias,
   const size_t ws_bytes = std::max<size_t>({16, lmoe_route_workspace_bytes(&d.s), lmoe_route_fwd_workspace_bytes(&d.s)});
   const size_t t_ws = c.take(ws_bytes), t_zp = forced_sel ? c.take((T + 7) / 8 * 4) : 0;
   const size_t t_lat = gather ? 0 : c.take(T * d.L * 2);
-  const size_t t_xs = (fp8 || (gather && views)) ? c.take(P * d.L * 2) : 0;
+  const size_t t_xs = (gather && views) ? c.take(P * d.L * 2) : 0;
+  const size_t t_latq = fp8 ? c.take(T * d.L) : 0;
   const size_t t_hid = fp8 ? c.take(P * d.F * 2) : 0;
   Tensor tmp = new_bytes(c.bytes, o.x);
   char* tv = base_of(tmp);
@@ -310,7 +311,19 @@ LatentOut latent_forward(const Sizes& d, const LatentOps& o, const Tensor& bias,
   void* y_sorted = sv + at_.y_sorted;
   void* h1 = keep ? sv + at_.h1 : nullptr;
   void* x_latent = gather ? sv + at_.x_rows : tv + t_lat;
-  void* x_sorted = fp8 ? tv + t_xs : (gather ? (views ? tv + t_xs : nullptr) : sv + at_.x_rows);
+  // what the routed GEMMs read: e4m3 rows (the latents are quantised before they are gathered: the maximum over the
+  // gathered rows is theirs, every token being routed), bf16 rows, or nothing (gather in the GEMM's producer)
+  void* x_sorted = fp8 ? sv + at_.xq : (gather ? (views ? tv + t_xs : nullptr) : sv + at_.x_rows);
+  const void* gather_src = fp8 ? tv + t_latq : x_latent;
+  const int gather_bytes = fp8 ? d.L : 2 * d.L;
+  float* scal = fp8 ? reinterpret_cast<float*>(sv + at_.scal) : nullptr;
+  lmoe_fp8_tensor q[3];
+  if (fp8) {
+    C10_CUDA_CHECK(cudaMemsetAsync(scal, 0, 32 * sizeof(float), stream.stream()));
+    q[0] = {x_latent, tv + t_latq, T, d.L, nullptr, amax_of(scal, kSx), deq_of(scal, kSx)};
+    q[1] = {o.wgu.data_ptr(), sv + at_.wguq, int64_t(d.E) * d.L, 2 * d.F, nullptr, amax_of(scal, kSwgu), deq_of(scal, kSwgu)};
+    q[2] = {o.wde.data_ptr(), sv + at_.wdq, int64_t(d.E) * d.F, d.L, nullptr, amax_of(scal, kSwd), deq_of(scal, kSwd)};
+  }
   void* hidden = fp8 ? tv + t_hid : sv + at_.hidden;
   int32_t* sel = r.sel.data_ptr<int32_t>();
 
@@ -327,7 +340,11 @@ LatentOut latent_forward(const Sizes& d, const LatentOps& o, const Tensor& bias,
     Tensor aff = at::sigmoid(view_of(r.saved, at_.logits, {T, d.E}, at::kFloat)).gather(1, r.sel.to(at::kLong));
     view_of(r.saved, at_.weights, {T, d.K}, at::kFloat).copy_(aff / (aff.sum(-1, true) + 1e-9));
     LMOE(lmoe_route_permute, &d.s, sel, &route, tv + t_ws, ws_bytes, st);
-    if (x_sorted) LMOE(lmoe_gather_rows, x_latent, route.row_src, d.K, P, d.L, route.n_tiles, x_sorted, st);
+    if (fp8) {
+      LMOE(lmoe_fp8_amax, 3, q, st);
+      LMOE(lmoe_fp8_cast, 3, q, st);
+    }
+    if (x_sorted) LMOE(lmoe_gather_rows, gather_src, route.row_src, d.K, P, gather_bytes / 2, route.n_tiles, x_sorted, st);
     LMOE(lmoe_shared_gateup_fwd, &d.s, o.x.data_ptr(), o.wgus.data_ptr(), h1_s, act_cat, status, st);
   } else {
     // Small batches: [x_latent, shared gate_up] on the side stream beside [logits, top-k].  At larger ones every GEMM
@@ -338,22 +355,28 @@ LatentOut latent_forward(const Sizes& d, const LatentOps& o, const Tensor& bias,
     LMOE(lmoe_xproj_fwd, &d.s, o.x.data_ptr(), nullptr, o.wdn.data_ptr(), nullptr, x_latent, status, side);
     LMOE(lmoe_topk_hist_fwd, &d.s, logits, bias.data_ptr<float>(), sel, weights, lse, tv + t_ws, ws_bytes, st);
     if (forked) fork->to_main();
+    if (fp8) {  // the weights beside the latents: on the side stream, or in the same launches
+      const int n = forked ? 1 : 3;
+      LMOE(lmoe_fp8_amax, n, q, st);
+      LMOE(lmoe_fp8_cast, n, q, st);
+      if (forked) {
+        LMOE(lmoe_fp8_amax, 2, q + 1, side);
+        LMOE(lmoe_fp8_cast, 2, q + 1, side);
+      }
+    }
     LMOE(lmoe_route_gather_fwd, &d.s, sel, tv + t_ws, ws_bytes, z_coef, r.z_loss.data_ptr<float>(), &route,
-         x_sorted ? x_latent : nullptr, 2 * d.L, x_sorted, st);
+         x_sorted ? gather_src : nullptr, gather_bytes, x_sorted, st);
+    if (fp8 && forked) fork->to_main();
     LMOE(lmoe_shared_gateup_fwd, &d.s, o.x.data_ptr(), o.wgus.data_ptr(), h1_s, act_cat, status, side);
   }
 
   // routed experts in the padded layout
   if (fp8) {
-    float* scal = reinterpret_cast<float*>(sv + at_.scal);
-    void *xq = sv + at_.xq, *hq = sv + at_.hq, *wguq = sv + at_.wguq, *wdq = sv + at_.wdq;
-    LMOE(lmoe_fp8_quantize, x_sorted, P, d.L, route.n_tiles, xq, amax_of(scal, kSx), deq_of(scal, kSx), st);
-    LMOE(lmoe_fp8_quantize, o.wgu.data_ptr(), int64_t(d.E) * d.L, 2 * d.F, nullptr, wguq, amax_of(scal, kSwgu),
-         deq_of(scal, kSwgu), st);
-    LMOE(lmoe_fp8_quantize, o.wde.data_ptr(), int64_t(d.E) * d.F, d.L, nullptr, wdq, amax_of(scal, kSwd), deq_of(scal, kSwd), st);
-    LMOE(lmoe_grouped_gateup_fp8, P, d.E, d.L, d.F, xq, wguq, deq_of(scal, kSx), deq_of(scal, kSwgu), route.tile_expert,
-         route.n_tiles, h1, hidden, status, st);
-    LMOE(lmoe_fp8_quantize, hidden, P, d.F, route.n_tiles, hq, amax_of(scal, kSh), deq_of(scal, kSh), st);
+    void *hq = sv + at_.hq, *wguq = sv + at_.wguq, *wdq = sv + at_.wdq;
+    LMOE(lmoe_grouped_gateup_fp8_amax, P, d.E, d.L, d.F, x_sorted, wguq, deq_of(scal, kSx), deq_of(scal, kSwgu), route.tile_expert,
+         route.n_tiles, h1, hidden, amax_of(scal, kSh), status, st);
+    const lmoe_fp8_tensor h = {hidden, hq, P, d.F, route.n_tiles, amax_of(scal, kSh), deq_of(scal, kSh)};
+    LMOE(lmoe_fp8_cast, 1, &h, st);
     LMOE(lmoe_grouped_rows_fp8, P, d.E, d.F, d.L, hq, wdq, 1, deq_of(scal, kSh), deq_of(scal, kSwd), route.tile_expert,
          route.n_tiles, y_sorted, status, st);
   } else if (gather) {
@@ -375,7 +398,7 @@ LatentOut latent_forward(const Sizes& d, const LatentOps& o, const Tensor& bias,
     views->emplace_back("lse", view_of(r.saved, at_.lse, {T}, at::kFloat));
     views->emplace_back("route_storage", view_of(r.saved, at_.route, {d.route_ints()}, at::kInt));
     views->emplace_back("x_latent", gather ? view_of(r.saved, at_.x_rows, {T, d.L}, bf) : view_of(tmp, t_lat, {T, d.L}, bf));
-    views->emplace_back("x_sorted", (fp8 || gather) ? view_of(tmp, t_xs, {P, d.L}, bf) : view_of(r.saved, at_.x_rows, {P, d.L}, bf));
+    if (!fp8) views->emplace_back("x_sorted", gather ? view_of(tmp, t_xs, {P, d.L}, bf) : view_of(r.saved, at_.x_rows, {P, d.L}, bf));
     views->emplace_back("h1", view_of(r.saved, at_.h1, {P, 2 * d.F}, bf));
     views->emplace_back("hidden", fp8 ? view_of(tmp, t_hid, {P, d.F}, bf) : view_of(r.saved, at_.hidden, {P, d.F}, bf));
     views->emplace_back("y_sorted", view_of(r.saved, at_.y_sorted, {P, d.L}, bf));
@@ -419,9 +442,11 @@ LatentGrads latent_backward(const Sizes& d, const LatentOps& o, const Tensor& dy
   Carver c;
   const size_t ws_bytes = std::max<size_t>(16, lmoe_wgrad_workspace_bytes(&d.s));
   const size_t t_ws = c.take(ws_bytes), t_dr = c.take(T * d.L * 2), t_cat = c.take(T * ld_cat * 2);
-  const size_t t_dw = c.take(T * d.K * 4), t_dys = c.take(P * d.L * 2), t_dh1 = c.take(P * 2 * d.F * 2);
+  const size_t t_dw = c.take(T * d.K * 4), t_dys = c.take(P * d.L * (fp8 ? 1 : 2)), t_dh1 = c.take(P * 2 * d.F * 2);
   const size_t t_dxs = c.take(P * d.L * 2);
-  const size_t t_dhid = fp8 ? c.take(P * d.F * 2) : 0, t_dyq = fp8 ? c.take(P * d.L) : 0, t_dh1q = fp8 ? c.take(P * 2 * d.F) : 0;
+  const size_t t_dh1q = fp8 ? c.take(P * 2 * d.F) : 0;
+  float* scal = fp8 ? reinterpret_cast<float*>(static_cast<char*>(saved.data_ptr()) + at_.scal) : nullptr;
+  if (fp8) C10_CUDA_CHECK(cudaMemsetAsync(amax_of(scal, kSdy), 0, 4 * sizeof(float), stream.stream()));
   Tensor tmp = new_bytes(c.bytes, o.x);
   char *tv = base_of(tmp), *sv = base_of(saved);
 
@@ -441,30 +466,32 @@ LatentGrads latent_backward(const Sizes& d, const LatentOps& o, const Tensor& dy
   LMOE(lmoe_combine_out_bwd_dgrad, &d.s, dy.data_ptr(), o.wup.data_ptr(), o.wds.data_ptr(), h1_s, d_routed, nullptr, cat,
        status, st);
   fork.to_side();
-  LMOE(lmoe_combine_bwd, &d.s, d_routed, y_sorted, weights, &route, d_ys, d_w, side);
+  if (fp8)
+    LMOE(lmoe_fp8_combine_bwd, &d.s, d_routed, y_sorted, weights, &route, amax_of(scal, kSdy), deq_of(scal, kSdy), d_ys, d_w, side);
+  else
+    LMOE(lmoe_combine_bwd, &d.s, d_routed, y_sorted, weights, &route, d_ys, d_w, side);
   LMOE(lmoe_combine_out_bwd_wgrad, &d.s, dy.data_ptr(), act_cat, g.wup.data_ptr(), g.wds.data_ptr(), gtype, ws, ws_bytes,
        status, st);
   fork.to_main();
 
   if (fp8) {
-    float* scal = reinterpret_cast<float*>(sv + at_.scal);
-    void *xq = sv + at_.xq, *hq = sv + at_.hq, *wguq = sv + at_.wguq, *wdq = sv + at_.wdq;
-    void *d_hid = tv + t_dhid, *dyq = tv + t_dyq, *dh1q = tv + t_dh1q;
-    LMOE(lmoe_fp8_quantize, d_ys, P, d.L, route.n_tiles, dyq, amax_of(scal, kSdy), deq_of(scal, kSdy), st);
-    // d_hidden = d_y * Wd[e]^T: the down weights [E, F, L] read as [N = F rows, K = L] (K-major operand)
-    LMOE(lmoe_grouped_rows_fp8, P, d.E, d.L, d.F, dyq, wdq, 0, deq_of(scal, kSdy), deq_of(scal, kSwd), route.tile_expert,
-         route.n_tiles, d_hid, status, st);
-    LMOE(lmoe_swiglu_bwd, P, d.F, h1, d_hid, d_h1, 2 * d.F, route.n_tiles, st);
-    LMOE(lmoe_fp8_quantize, d_h1, P, 2 * d.F, route.n_tiles, dh1q, amax_of(scal, kSdh1), deq_of(scal, kSdh1), st);
+    void *xq = sv + at_.xq, *hq = sv + at_.hq, *wguq = sv + at_.wguq, *wdq = sv + at_.wdq, *dyq = d_ys, *dh1q = tv + t_dh1q;
+    // d_h1 = swiglu'(h1, d_y * Wd[e]^T): the down weights [E, F, L] read as [N = F rows, K = L] (K-major operand)
+    LMOE(lmoe_grouped_swiglu_bwd_fp8, P, d.E, d.L, d.F, dyq, wdq, deq_of(scal, kSdy), deq_of(scal, kSwd), route.tile_expert,
+         route.n_tiles, h1, d_h1, amax_of(scal, kSdh1), status, st);
+    const lmoe_fp8_tensor h = {d_h1, dh1q, P, 2 * d.F, route.n_tiles, amax_of(scal, kSdh1), deq_of(scal, kSdh1)};
+    LMOE(lmoe_fp8_cast, 1, &h, st);
     // d_x_sorted = d_h1 * Wgu[e]^T: the gate_up weights [E, L, 2F] read as [N = L rows, K = 2F]
     LMOE(lmoe_grouped_rows_fp8, P, d.E, 2 * d.F, d.L, dh1q, wguq, 0, deq_of(scal, kSdh1), deq_of(scal, kSwgu),
          route.tile_expert, route.n_tiles, d_xs, status, st);
+    fork.to_side();
+    LMOE(lmoe_unpermute_sum_bwd, &d.s, d_xs, &route, cat, side);
+    LMOE(lmoe_gate_topk_bwd, &d.s, logits, sel, weights, d_w, lse, dz, z_coef, cat, side);
     LMOE(lmoe_grouped_wgrad_fp8, P, d.E, d.L, 2 * d.F, xq, dh1q, deq_of(scal, kSx), deq_of(scal, kSdh1), route.pad_offsets,
          g.wgu.data_ptr(), status, st);
     LMOE(lmoe_grouped_wgrad_fp8, P, d.E, d.F, d.L, hq, dyq, deq_of(scal, kSh), deq_of(scal, kSdy), route.pad_offsets,
          g.wde.data_ptr(), status, st);
-    LMOE(lmoe_unpermute_sum_bwd, &d.s, d_xs, &route, cat, st);
-    LMOE(lmoe_gate_topk_bwd, &d.s, logits, sel, weights, d_w, lse, dz, z_coef, cat, st);
+    fork.to_main();
   } else {
     void *x_rows = sv + at_.x_rows, *hidden = sv + at_.hidden;
     // d_h1 = swiglu'(h1, d_y_sorted * Wd[e]^T), d_x_sorted = d_h1 * Wgu[e]^T; d_hidden never reaches memory
@@ -494,7 +521,7 @@ LatentGrads latent_backward(const Sizes& d, const LatentOps& o, const Tensor& dy
     views->emplace_back("d_x_latent", cv.narrow(1, 2 * d.Fs, d.L));
     views->emplace_back("d_logits", cv.narrow(1, 2 * d.Fs + d.L, d.E));
     views->emplace_back("d_weights", view_of(tmp, t_dw, {T, d.K}, at::kFloat));
-    views->emplace_back("d_y_sorted", view_of(tmp, t_dys, {P, d.L}, b16));
+    if (!fp8) views->emplace_back("d_y_sorted", view_of(tmp, t_dys, {P, d.L}, b16));
     views->emplace_back("d_h1", view_of(tmp, t_dh1, {P, 2 * d.F}, b16));
     views->emplace_back("d_x_sorted", view_of(tmp, t_dxs, {P, d.L}, b16));
   }
@@ -634,8 +661,7 @@ MoeGrads moe_backward(const Sizes& d, const MoeOps& o, const Tensor& dy, const f
   LMOE(lmoe_moe_shared_bwd, &d.s, dy.data_ptr(), o.wds.data_ptr(), sv + at_.h1_s, sv + at_.hidden_s, cat, g.wds.data_ptr(), gtype,
        ws, ws_bytes, status, st);
   // adjoint of the weighted sum: d_y_sorted = w * dy[t], d_w = <dy[t], y_sorted>
-  LMOE(lmoe_combine_bwd_rows, dy.data_ptr(), sv + at_.y_sorted, weights, route.row_src, P, d.K, d.D, route.n_tiles, d_ys, d_w,
-       st);
+  LMOE(lmoe_combine_bwd, &d.s, dy.data_ptr(), sv + at_.y_sorted, weights, &route, d_ys, d_w, st);
   // routed experts
   LMOE(lmoe_grouped_bwd_dgrad, P, d.E, d.D, d.F, d_ys, sv + at_.h1, o.wgu.data_ptr(), o.wde.data_ptr(), route.tile_expert,
        route.n_tiles, route.pad_offsets, nullptr, d_h1, d_xs, status, st);
