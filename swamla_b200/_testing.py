@@ -20,10 +20,6 @@ def capture(**tensors) -> None:
         SINK.update(tensors)
 
 
-def hooked() -> bool:
-    return SINK is not None or FORCE_SEL is not None
-
-
 def capturing() -> bool:
     return SINK is not None
 

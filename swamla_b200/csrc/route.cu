@@ -9,214 +9,52 @@
 #include "../../include/lmoe.h"
 #include "counters.h"
 #include "device_once.h"
+#include "topk.cuh"
 
 namespace lmoe {
 
-constexpr int kTopkWarpsPerBlock = 8;
-constexpr int kMaxPerLane = LMOE_MAX_EXPERTS / 32;  // 8 scores per lane at E = 256
+constexpr int kTopkWarps = 8;       // warps of a top-k block, and the fewest of one that also counts
+constexpr int kMaxTopkWarps = 32;
 
-__device__ __forceinline__ float sigmoid_f(float x) { return 1.0f / (1.0f + expf(-x)); }
-
-// The top-k kernels can also count their block's selections: chunk_hist[blockIdx.x][E], the first pass of the routing
-// tables (the counts are whole numbers, so the order of the shared-memory additions does not matter).
-__device__ __forceinline__ void topk_hist_clear(int* s_hist, int E) {
-  for (int e = threadIdx.x; e < E; e += blockDim.x) s_hist[e] = 0;
-  __syncthreads();
-}
-__device__ __forceinline__ void topk_hist_store(const int* s_hist, int E, int* __restrict__ chunk_hist) {
-  // the caller's last __syncthreads() lies after every addition
-  for (int e = threadIdx.x; e < E; e += blockDim.x) chunk_hist[static_cast<long long>(blockIdx.x) * E + e] = s_hist[e];
-}
-
-// One warp per token row, `per_warp` consecutive rows each.  Lane l holds experts l, l+32, ...
-__global__ void __launch_bounds__(kTopkWarpsPerBlock * 32)
-gate_topk_kernel(const float* __restrict__ logits, const float* __restrict__ bias, int T, int E, int K,
-                 int* __restrict__ sel, float* __restrict__ weights, float* __restrict__ lse_out,
-                 float* __restrict__ z_partial, int per_warp, int* __restrict__ chunk_hist) {
-  __shared__ float s_lse2[kTopkWarpsPerBlock];
-  __shared__ int s_hist[LMOE_MAX_EXPERTS];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (chunk_hist) topk_hist_clear(s_hist, E);
-  float lse2 = 0.f;
-  for (int r = 0; r < per_warp; ++r) {
-    const int t = (blockIdx.x * kTopkWarpsPerBlock + warp) * per_warp + r;
-    if (t >= T) break;
-    float aff[kMaxPerLane], score[kMaxPerLane];
-    const float* row = logits + static_cast<long long>(t) * E;
-    float mx = -CUDART_INF_F;
-#pragma unroll
-    for (int j = 0; j < kMaxPerLane; ++j) {
-      const int e = lane + 32 * j;
-      if (e < E) {
-        const float x = row[e];
-        mx = fmaxf(mx, x);
-        aff[j] = sigmoid_f(x);
-        score[j] = aff[j] + bias[e];
-      } else {
-        aff[j] = 0.f;
-        score[j] = -CUDART_INF_F;
-      }
-    }
-    // logsumexp over the row
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-    float se = 0.f;
-#pragma unroll
-    for (int j = 0; j < kMaxPerLane; ++j) {
-      const int e = lane + 32 * j;
-      if (e < E) se += expf(row[e] - mx);
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) se += __shfl_xor_sync(0xffffffffu, se, o);
-    const float lse = mx + logf(se);
-    lse2 += lse * lse;
-    if (lane == 0) lse_out[t] = lse;
-
-    // Order-preserving 32-bit keys: key(a) > key(b) <=> a > b (with -0 folded onto +0), so that the
-    // warp-wide maximum is one redux instruction.  Ties go to the lower expert index through a
-    // second redux (minimum index among the lanes that hold the maximum).
-    unsigned key[kMaxPerLane];
-#pragma unroll
-    for (int j = 0; j < kMaxPerLane; ++j) {
-      const unsigned u = __float_as_uint(score[j] + 0.0f);
-      key[j] = (lane + 32 * j < E) ? ((u & 0x80000000u) ? ~u : (u | 0x80000000u)) : 0u;
-    }
-    float my_aff = 0.f;  // lane k keeps the affinity of the k-th winner
-    int my_idx = 0;
-    float aff_sum = 0.f;
-    for (int k = 0; k < K; ++k) {
-      unsigned bk = 0u;
-      int bj = 0;
-#pragma unroll
-      for (int j = 0; j < kMaxPerLane; ++j) {
-        if (key[j] > bk) {  // strict: the lowest j (lowest expert index) wins a tie inside the lane
-          bk = key[j];
-          bj = j;
-        }
-      }
-      const unsigned wmax = __reduce_max_sync(0xffffffffu, bk);
-      const unsigned cand = (bk == wmax) ? static_cast<unsigned>(lane + 32 * bj) : 0xffffffffu;
-      const int bi = static_cast<int>(__reduce_min_sync(0xffffffffu, cand));
-      const int wl = bi & 31;
-      float la = 0.f;
-#pragma unroll
-      for (int j = 0; j < kMaxPerLane; ++j)
-        if (j == bj) la = aff[j];
-      const float ba = __shfl_sync(0xffffffffu, la, wl);
-      if (lane == wl) {
-#pragma unroll
-        for (int j = 0; j < kMaxPerLane; ++j)
-          if (j == (bi >> 5)) key[j] = 0u;  // retire the winner (every live key has its top bit pattern > 0)
-      }
-      if (lane == k) {
-        my_aff = ba;
-        my_idx = bi;
-      }
-      aff_sum += ba;  // same order on every lane: slot 0, 1, ...
-    }
-    if (lane < K) {
-      sel[static_cast<long long>(t) * K + lane] = my_idx;
-      weights[static_cast<long long>(t) * K + lane] = my_aff / (aff_sum + 1e-9f);
-      if (chunk_hist) atomicAdd(&s_hist[my_idx], 1);
-    }
-  }
-  if (lane == 0) s_lse2[warp] = lse2;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    float s = 0.f;
-    for (int i = 0; i < kTopkWarpsPerBlock; ++i) s += s_lse2[i];
-    z_partial[blockIdx.x] = s;
-  }
-  if (chunk_hist) topk_hist_store(s_hist, E, chunk_hist);
-}
-
-// Same result for E = 32 * PER: lane l holds the PER CONSECUTIVE experts l*PER .. l*PER+PER-1, so "lower expert index
-// first" is "lower lane first, then lower slot inside the lane": the arg-max of a round is one redux (maximum key), one
-// ballot (which lanes hold it) and a find-first-set, instead of two reductions.
+// One warp per token, `per_warp` consecutive tokens each.  With chunk_hist the block also counts its selections:
+// chunk_hist[blockIdx.x][E] is the first pass of the routing tables (whole numbers: the order of the shared-memory
+// additions does not matter).
 template <int PER>
-__global__ void __launch_bounds__(kTopkWarpsPerBlock * 32)
-gate_topk_blocked_kernel(const float* __restrict__ logits, const float* __restrict__ bias, int T, int K,
-                         int* __restrict__ sel, float* __restrict__ weights, float* __restrict__ lse_out,
-                         float* __restrict__ z_partial, int per_warp, int* __restrict__ chunk_hist) {
-  constexpr int E = 32 * PER;
-  __shared__ float s_lse2[kTopkWarpsPerBlock];
-  __shared__ int s_hist[E];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (chunk_hist) topk_hist_clear(s_hist, E);
+__global__ void __launch_bounds__(kMaxTopkWarps * 32)
+gate_topk_kernel(const float* __restrict__ logits, const float* __restrict__ bias, int T, int E, int K, int* __restrict__ sel,
+                 float* __restrict__ weights, float* __restrict__ lse_out, float* __restrict__ z_partial, int per_warp,
+                 int* __restrict__ chunk_hist) {
+  __shared__ float s_lse2[kMaxTopkWarps];
+  __shared__ int s_hist[32 * PER];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
+  if (chunk_hist) {
+    for (int e = threadIdx.x; e < E; e += blockDim.x) s_hist[e] = 0;
+    __syncthreads();
+  }
   float lse2 = 0.f;
   for (int r = 0; r < per_warp; ++r) {
-    const int t = (blockIdx.x * kTopkWarpsPerBlock + warp) * per_warp + r;
+    const int t = (blockIdx.x * warps + warp) * per_warp + r;
     if (t >= T) break;
-    float x[PER], aff[PER];
-    unsigned key[PER];
-    const float* row = logits + static_cast<long long>(t) * E + lane * PER;
-    float mx = -CUDART_INF_F;
-#pragma unroll
-    for (int j = 0; j < PER; ++j) {
-      x[j] = row[j];
-      mx = fmaxf(mx, x[j]);
-      aff[j] = sigmoid_f(x[j]);
-      const unsigned u = __float_as_uint((aff[j] + bias[lane * PER + j]) + 0.0f);
-      key[j] = (u & 0x80000000u) ? ~u : (u | 0x80000000u);
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-    float se = 0.f;
-#pragma unroll
-    for (int j = 0; j < PER; ++j) se += expf(x[j] - mx);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) se += __shfl_xor_sync(0xffffffffu, se, o);
-    const float lse = mx + logf(se);
+    int idx;
+    float aff, aff_sum, lse;
+    topk_row<PER>(logits + static_cast<long long>(t) * E, bias, E, K, lane, idx, aff, aff_sum, lse);
     lse2 += lse * lse;
     if (lane == 0) lse_out[t] = lse;
-
-    float my_aff = 0.f;
-    int my_idx = 0;
-    float aff_sum = 0.f;
-    for (int k = 0; k < K; ++k) {
-      unsigned bk = 0u;
-      int bj = 0;
-#pragma unroll
-      for (int j = 0; j < PER; ++j) {
-        if (key[j] > bk) {  // strict: the lowest slot wins a tie inside the lane
-          bk = key[j];
-          bj = j;
-        }
-      }
-      const unsigned wmax = __reduce_max_sync(0xffffffffu, bk);
-      const unsigned holders = __ballot_sync(0xffffffffu, bk == wmax);
-      const int wl = __ffs(holders) - 1;  // lowest lane = lowest expert index among the maxima
-      float la = 0.f;
-#pragma unroll
-      for (int j = 0; j < PER; ++j)
-        if (j == bj) la = aff[j];
-      const float ba = __shfl_sync(0xffffffffu, la, wl);
-      const int bi = __shfl_sync(0xffffffffu, lane * PER + bj, wl);
-      if (lane == wl) {
-#pragma unroll
-        for (int j = 0; j < PER; ++j)
-          if (j == bj) key[j] = 0u;
-      }
-      if (lane == k) {
-        my_aff = ba;
-        my_idx = bi;
-      }
-      aff_sum += ba;
-    }
     if (lane < K) {
-      sel[static_cast<long long>(t) * K + lane] = my_idx;
-      weights[static_cast<long long>(t) * K + lane] = my_aff / (aff_sum + 1e-9f);
-      if (chunk_hist) atomicAdd(&s_hist[my_idx], 1);
+      sel[static_cast<long long>(t) * K + lane] = idx;
+      weights[static_cast<long long>(t) * K + lane] = aff / (aff_sum + 1e-9f);
+      if (chunk_hist) atomicAdd(&s_hist[idx], 1);
     }
   }
   if (lane == 0) s_lse2[warp] = lse2;
   __syncthreads();
   if (threadIdx.x == 0) {
     float s = 0.f;
-    for (int i = 0; i < kTopkWarpsPerBlock; ++i) s += s_lse2[i];
+    for (int i = 0; i < warps; ++i) s += s_lse2[i];
     z_partial[blockIdx.x] = s;
   }
-  if (chunk_hist) topk_hist_store(s_hist, E, chunk_hist);
+  if (chunk_hist)
+    for (int e = threadIdx.x; e < E; e += blockDim.x) chunk_hist[static_cast<long long>(blockIdx.x) * E + e] = s_hist[e];
 }
 
 // Deterministic final reduction of the z-loss partials (fixed order, one block).
@@ -385,8 +223,8 @@ route_scatter_kernel(const int* __restrict__ sel, int n, int E, const int* __res
 // it K times).  Blocks beyond the last chunk, and every block besides its chunk, publish the tables and zero the pad rows of
 // experts b, b + gridDim.x, ...; block 0 also adds up the z-loss.
 constexpr int kDirectChunks = 128;
-constexpr int kMaxPerWarp = 16;
-constexpr int kMaskWords = kTopkWarpsPerBlock * kMaxPerWarp / 32;
+constexpr int kMaxChunkTokens = 128;
+constexpr int kMaskWords = kMaxChunkTokens / 32;
 
 __global__ void __launch_bounds__(256)
 route_gather_kernel(const int* __restrict__ sel, int T, int E, int K, int tokens, int chunks, int direct,
@@ -559,11 +397,10 @@ static inline void prefer_max_carveout(F* fn) {
 static void configure_route_kernels() {
   static PerDeviceOnce once;
   once.run([] {
-  prefer_max_carveout(gate_topk_kernel);
-  prefer_max_carveout(gate_topk_blocked_kernel<1>);
-  prefer_max_carveout(gate_topk_blocked_kernel<2>);
-  prefer_max_carveout(gate_topk_blocked_kernel<4>);
-  prefer_max_carveout(gate_topk_blocked_kernel<8>);
+  prefer_max_carveout(gate_topk_kernel<1>);
+  prefer_max_carveout(gate_topk_kernel<2>);
+  prefer_max_carveout(gate_topk_kernel<4>);
+  prefer_max_carveout(gate_topk_kernel<8>);
   prefer_max_carveout(zloss_finalize_kernel);
   prefer_max_carveout(route_hist_kernel);
   prefer_max_carveout(route_scan_chunks_kernel);
@@ -586,19 +423,12 @@ static inline int check_shape(const lmoe_shape* s) {
 using namespace lmoe;
 
 static void launch_topk(const lmoe_shape* s, const float* logits, const float* bias, int32_t* sel, float* weights, float* lse,
-                        float* z_partial, int per_warp, int* chunk_hist, cudaStream_t st) {
+                        float* z_partial, int warps, int per_warp, int* chunk_hist, cudaStream_t st) {
   configure_route_kernels();
-  const int per_block = kTopkWarpsPerBlock * per_warp;
+  const int per_block = warps * per_warp;
   const int blocks = (s->T + per_block - 1) / per_block;
-  const int thr = kTopkWarpsPerBlock * 32;
-  switch (s->E) {  // blocked layout when the expert count is a multiple of the warp size
-    case 32: gate_topk_blocked_kernel<1><<<blocks, thr, 0, st>>>(logits, bias, s->T, s->K, sel, weights, lse, z_partial, per_warp, chunk_hist); break;
-    case 64: gate_topk_blocked_kernel<2><<<blocks, thr, 0, st>>>(logits, bias, s->T, s->K, sel, weights, lse, z_partial, per_warp, chunk_hist); break;
-    case 128: gate_topk_blocked_kernel<4><<<blocks, thr, 0, st>>>(logits, bias, s->T, s->K, sel, weights, lse, z_partial, per_warp, chunk_hist); break;
-    case 256: gate_topk_blocked_kernel<8><<<blocks, thr, 0, st>>>(logits, bias, s->T, s->K, sel, weights, lse, z_partial, per_warp, chunk_hist); break;
-    default:
-      gate_topk_kernel<<<blocks, thr, 0, st>>>(logits, bias, s->T, s->E, s->K, sel, weights, lse, z_partial, per_warp, chunk_hist);
-  }
+  auto kernel = s->E <= 32 ? gate_topk_kernel<1> : s->E <= 64 ? gate_topk_kernel<2> : s->E <= 128 ? gate_topk_kernel<4> : gate_topk_kernel<8>;
+  kernel<<<blocks, warps * 32, 0, st>>>(logits, bias, s->T, s->E, s->K, sel, weights, lse, z_partial, per_warp, chunk_hist);
   count_launch();
 }
 
@@ -608,8 +438,8 @@ extern "C" int lmoe_gate_topk_fwd(const lmoe_shape* s, const float* logits, cons
   if (int rc = check_shape(s)) return rc;
   if (!logits || !expert_bias || !sel || !weights || !lse || !z_partial || !z_loss) return LMOE_ERR_ARG;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  launch_topk(s, logits, expert_bias, sel, weights, lse, z_partial, 1, nullptr, st);
-  const int blocks = (s->T + kTopkWarpsPerBlock - 1) / kTopkWarpsPerBlock;
+  launch_topk(s, logits, expert_bias, sel, weights, lse, z_partial, kTopkWarps, 1, nullptr, st);
+  const int blocks = (s->T + kTopkWarps - 1) / kTopkWarps;
   count_launch();
   zloss_finalize_kernel<<<1, 256, 0, st>>>(z_partial, blocks, z_coef / static_cast<float>(s->T), z_loss);
   cudaError_t e = cudaGetLastError();
@@ -620,20 +450,24 @@ extern "C" int lmoe_gate_topk_fwd(const lmoe_shape* s, const float* logits, cons
 // lmoe_topk_hist_fwd + lmoe_route_gather_fwd do what lmoe_gate_topk_fwd, lmoe_route_permute and lmoe_gather_rows do in six
 // launches.  Tokens are cut into chunks of one top-k block each.  Up to kDirectChunks of them, every block of the scatter
 // adds up the chunk histograms itself (they are a few KB per block, from L2); beyond, a scan kernel does it once.
-static int tokens_per_warp(int T) {
-  const int direct = (T + kTopkWarpsPerBlock * kDirectChunks - 1) / (kTopkWarpsPerBlock * kDirectChunks);
-  if (direct <= 4) return direct;                                       // up to 4,096 tokens
-  const int r = (T + kTopkWarpsPerBlock * 1024 - 1) / (kTopkWarpsPerBlock * 1024);  // about 1,024 chunks
-  return r < 4 ? 4 : (r > kMaxPerWarp ? kMaxPerWarp : r);
-}
-static int route_chunks(const lmoe_shape* s) {
-  const int per_block = kTopkWarpsPerBlock * tokens_per_warp(s->T);
-  return (s->T + per_block - 1) / per_block;
+// A token takes a warp about 2 us, so a batch is spread over as many warps as it has tokens; the blocks get larger (8 to 32
+// warps) to keep at most kDirectChunks of them up to 4,096 tokens, and then each warp takes more tokens, for about 1,024 chunks.
+struct RouteChunks {
+  int warps, per_warp, tokens, n;
+};
+static RouteChunks route_chunks(int T) {
+  RouteChunks c;
+  c.warps = T <= kTopkWarps * kDirectChunks ? kTopkWarps : T <= 2 * kTopkWarps * kDirectChunks ? 2 * kTopkWarps : kMaxTopkWarps;
+  c.per_warp = (T + kMaxTopkWarps * 1024 - 1) / (kMaxTopkWarps * 1024);
+  if (c.per_warp > kMaxChunkTokens / kMaxTopkWarps) c.per_warp = kMaxChunkTokens / kMaxTopkWarps;
+  c.tokens = c.warps * c.per_warp;
+  c.n = (T + c.tokens - 1) / c.tokens;
+  return c;
 }
 
 extern "C" size_t lmoe_route_fwd_workspace_bytes(const lmoe_shape* s) {
   if (check_shape(s)) return 0;
-  const size_t chunks = static_cast<size_t>(route_chunks(s));
+  const size_t chunks = static_cast<size_t>(route_chunks(s->T).n);
   return (chunks * s->E + (chunks + 3) / 4 * 4) * sizeof(int);
 }
 
@@ -643,8 +477,9 @@ extern "C" int lmoe_topk_hist_fwd(const lmoe_shape* s, const float* logits, cons
   if (!logits || !expert_bias || !sel || !weights || !lse || !workspace) return LMOE_ERR_ARG;
   if (workspace_bytes < lmoe_route_fwd_workspace_bytes(s)) return LMOE_ERR_WORKSPACE;
   int* hist = static_cast<int*>(workspace);
-  float* z_partial = reinterpret_cast<float*>(hist + static_cast<size_t>(route_chunks(s)) * s->E);
-  launch_topk(s, logits, expert_bias, sel, weights, lse, z_partial, tokens_per_warp(s->T), hist, static_cast<cudaStream_t>(stream));
+  const RouteChunks c = route_chunks(s->T);
+  float* z_partial = reinterpret_cast<float*>(hist + static_cast<size_t>(c.n) * s->E);
+  launch_topk(s, logits, expert_bias, sel, weights, lse, z_partial, c.warps, c.per_warp, hist, static_cast<cudaStream_t>(stream));
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : static_cast<int>(e);
 }
@@ -660,7 +495,8 @@ extern "C" int lmoe_route_gather_fwd(const lmoe_shape* s, const int32_t* sel, vo
   if (workspace_bytes < lmoe_route_fwd_workspace_bytes(s)) return LMOE_ERR_WORKSPACE;
   configure_route_kernels();
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  const int chunks = route_chunks(s), tokens = kTopkWarpsPerBlock * tokens_per_warp(s->T);
+  const RouteChunks rc = route_chunks(s->T);
+  const int chunks = rc.n, tokens = rc.tokens;
   int* hist = static_cast<int*>(workspace);
   const float* z_partial = reinterpret_cast<float*>(hist + static_cast<size_t>(chunks) * s->E);
   const bool direct = chunks <= kDirectChunks;

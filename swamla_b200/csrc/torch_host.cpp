@@ -210,6 +210,10 @@ bool tma_gather_enabled() {
   return on;
 }
 
+Tensor f32_bias(const Tensor& b) {
+  return b.scalar_type() == at::kFloat && b.is_contiguous() ? b : b.detach().to(at::kFloat).contiguous();
+}
+
 // ---------------------------------------------------------------- LatentMoE: what a forward keeps
 // Byte offsets in the saved allocation.  functional.saved_bytes (shape arithmetic of the compiled operators) computes the
 // same total.
@@ -678,8 +682,24 @@ MoeGrads moe_backward(const Sizes& d, const MoeOps& o, const Tensor& dy, const f
   return g;
 }
 
+// ---------------------------------------------------------------- a few tokens, no backward
+// For a module in evaluation mode only: the sums run in another order than in the training forward, which an activation
+// checkpoint recomputes bit for bit.
+std::vector<Tensor> few_forward(const Sizes& d, const Tensor& x2d, const Tensor& wg, const Tensor* wdn, const Tensor* wup,
+                                const Tensor& wgus, const Tensor& wds, const Tensor& wgu, const Tensor& wde, const Tensor& bias,
+                                float z_coef) {
+  Tensor y = at::empty({d.T, d.D}, x2d.options());
+  Tensor z = at::empty({}, x2d.options().dtype(at::kFloat));
+  const size_t n = lmoe_few_workspace_bytes(&d.s);
+  Tensor ws = new_bytes(n, x2d);
+  LMOE(lmoe_few_forward, &d.s, x2d.data_ptr(), wg.data_ptr(), wdn ? wdn->data_ptr() : nullptr, wup ? wup->data_ptr() : nullptr,
+       wgus.data_ptr(), wds.data_ptr(), wgu.data_ptr(), wde.data_ptr(), bias.data_ptr<float>(), z_coef, y.data_ptr(),
+       z.data_ptr<float>(), ws.data_ptr(), n, at::cuda::getCurrentCUDAStream().stream());
+  return {y, z};
+}
+
 // ---------------------------------------------------------------- autograd
-Tensor f32_bias(const Tensor& b) { return b.detach().to(at::kFloat).contiguous(); }
+
 
 void require_cuda(const Tensor& x, const char* what) {
   if (!x.is_cuda()) throw LmoeFailure(std::string("the ") + what + " path runs on a CUDA device only (no CPU fallback)");
@@ -813,21 +833,26 @@ bool any_grad(std::initializer_list<const Tensor*> ts) {
 // ---------------------------------------------------------------- Python entry points
 std::vector<Tensor> latent_moe(const Tensor& x, const Tensor& wg, const Tensor& wdn, const Tensor& wup, const Tensor& wgus,
                                const Tensor& wds, const Tensor& wgu, const Tensor& wde, const Tensor& bias, int64_t top_k,
-                               double z_coef, bool fp8) {
+                               double z_coef, bool fp8, bool evaluation) {
   require_cuda(x, "LatentMoE");
   poll_status();
   const c10::cuda::CUDAGuard guard(x.device());
   if (any_grad({&x, &wg, &wdn, &wup, &wgus, &wds, &wgu, &wde}))
     return LatentFn::apply(x, wg, wdn, wup, wgus, wds, wgu, wde, bias, top_k, z_coef, fp8);
   const LatentOps o = latent_ops(x, wg, wdn, wup, wgus, wds, wgu, wde);
-  LatentOut r = latent_forward(latent_sizes(o.x, o.wgu, o.wds, top_k), o, f32_bias(bias), static_cast<float>(z_coef), fp8,
+  const Sizes d = latent_sizes(o.x, o.wgu, o.wds, top_k);
+  if (evaluation && d.T <= LMOE_FEW_TOKENS && lmoe_few_applies(&d.s)) {
+    auto yz = few_forward(d, o.x, o.wg, &o.wdn, &o.wup, o.wgus, o.wds, o.wgu, o.wde, f32_bias(bias), static_cast<float>(z_coef));
+    return {as_param(yz[0].view(x.sizes()), x.scalar_type()), yz[1]};
+  }
+  LatentOut r = latent_forward(d, o, f32_bias(bias), static_cast<float>(z_coef), fp8,
                                false, c10::nullopt, nullptr);
   return {as_param(r.y.view(x.sizes()), x.scalar_type()), r.z_loss, r.sel, r.counts};
 }
 
 std::vector<Tensor> moe(const Tensor& x, const Tensor& wg, const Tensor& wgus, const Tensor& wds, const Tensor& wgu,
                         const Tensor& wde, const Tensor& bias, int64_t top_k, double z_coef,
-                        const c10::optional<Tensor>& forced_sel) {
+                        const c10::optional<Tensor>& forced_sel, bool evaluation) {
   require_cuda(x, "MoE");
   poll_status();
   const c10::cuda::CUDAGuard guard(x.device());
@@ -835,7 +860,12 @@ std::vector<Tensor> moe(const Tensor& x, const Tensor& wg, const Tensor& wgus, c
   Caster cast;
   const MoeOps o{cast(x).view({-1, x.size(-1)}), cast(wg), cast(wgus), cast(wds), cast(wgu), cast(wde)};
   cast.run(at::cuda::getCurrentCUDAStream().stream());
-  LatentOut r = moe_forward(moe_sizes(o.x, o.wgu, o.wds, top_k), o, f32_bias(bias), static_cast<float>(z_coef), false, forced_sel);
+  const Sizes d = moe_sizes(o.x, o.wgu, o.wds, top_k);
+  if (evaluation && !forced_sel && d.T <= LMOE_FEW_TOKENS && lmoe_few_applies(&d.s)) {
+    auto yz = few_forward(d, o.x, o.wg, nullptr, nullptr, o.wgus, o.wds, o.wgu, o.wde, f32_bias(bias), static_cast<float>(z_coef));
+    return {as_param(yz[0].view(x.sizes()), x.scalar_type()), yz[1]};
+  }
+  LatentOut r = moe_forward(d, o, f32_bias(bias), static_cast<float>(z_coef), false, forced_sel);
   return {as_param(r.y.view(x.sizes()), x.scalar_type()), r.z_loss, r.sel, r.counts};
 }
 

@@ -262,10 +262,12 @@ class LatentMoELayer(nn.Module):
         batch_size, seq_len, d_model = x.shape
         router = self._modules["router"]
         if self.ep_size == 1 and not compiling and x.is_cuda:
-            y, z_loss, sel, counts = latent_moe(x, *self._arguments(), self.n_activated, router.z_loss_coef, self.fp8_experts)
-            self.aux_loss = z_loss
-            if self.training:
-                router._last_selected_experts, router._last_counts = sel, counts
+            training = self.training
+            out = latent_moe(x, *self._arguments(), self.n_activated, router.z_loss_coef, self.fp8_experts, not training)
+            y = out[0]
+            self.__dict__["aux_loss"] = out[1]      # (plain attribute: skips the module's parameter bookkeeping)
+            if training:
+                router._last_selected_experts, router._last_counts = out[2], out[3]
                 router._last_num_tokens = batch_size * seq_len
                 if self.dropout.p > 0.0:
                     y = self.dropout(y)
@@ -375,13 +377,11 @@ class MoELayer(nn.Module):
         moe = functional_moe.moe_opaque if torch.compiler.is_compiling() else functional_moe.moe
         status_monitor.poll()
         w_gate_up_s, w_down_s = _merged_shared_weights(self.shared_experts)
-        y, z_loss, sel, counts = moe(x, self.router.gate.weight, w_gate_up_s,
-                                     w_down_s, self.experts.gate_up_weight, self.experts.down_weight,
-                                     self.router.expert_bias, self.n_activated, self.router.z_loss_coef)
-        self.aux_loss = z_loss                                            # moe.py:358
+        out = moe(x, self.router.gate.weight, w_gate_up_s, w_down_s, self.experts.gate_up_weight, self.experts.down_weight,
+                  self.router.expert_bias, self.n_activated, self.router.z_loss_coef, not self.training)
+        y, self.aux_loss = out[0], out[1]                                 # moe.py:358
         if self.training:                                                 # moe.py:237-240
-            self.router._last_selected_experts = sel
-            self.router._last_counts = counts
+            self.router._last_selected_experts, self.router._last_counts = out[2], out[3]
             self.router._last_num_tokens = x.shape[0] * x.shape[1]
             if self.dropout.p > 0.0:
                 y = self.dropout(y)                                       # moe.py:367

@@ -1,0 +1,67 @@
+"""The few-token forward (evaluation mode, no gradients) against the padded path of the same layer.
+
+Both are bf16 pipelines with the same rounding points and fp32 sums in another order: they differ by single bf16 ulps of
+intermediates, for which the layer tests allow 2.5e-3 relative Frobenius error and two ulps (2^-6) per element of the output's
+scale.  A token whose K-th and (K+1)-th scores are within the fp32 rounding of the logits may select another expert; tokens
+with such a near-tie (gap below 1e-5) are left out of the comparison.
+"""
+import pytest
+import torch
+
+from oracle import inputs
+
+pytestmark = pytest.mark.gpu
+
+
+# one token, the edges of every token-tile count (8, 16, 32, 64), and the first size beyond the path
+@pytest.mark.parametrize("T", [1, 2, 8, 9, 16, 17, 33, 64, 65])
+# widths of one and several passes, fewer slots than experts and more, 4 to 256 experts, both layer classes
+@pytest.mark.parametrize("name", ["tiny", "cfg1", "cfg5_2k", "cfg3", "tiny_moe", "moe_1b"])
+def test_few_token_forward_matches_padded_path(name, T):
+    from swamla_b200 import _cabi
+    from swamla_b200.layer import create_moe_layer
+    w = inputs.WORKLOADS[name]
+    torch.manual_seed(T)
+    with torch.device("cuda:0"):
+        layer = create_moe_layer(w.config()).to(torch.bfloat16)
+        with torch.no_grad():
+            for p in layer.parameters():
+                p.normal_(0.0, 0.05)
+            layer.router.expert_bias.normal_(0.0, 0.05)
+        x = torch.randn(T, 1, w.D).to(torch.bfloat16)
+    lib = _cabi.load()
+    shape = _cabi.Shape(T=T, D=w.D, L=w.L, E=w.E, K=w.K, F=w.F, Fs=w.Fs, n_shared=1)
+    assert lib.lmoe_few_applies(shape) == (1 if T <= 64 else 0)
+    with torch.no_grad():
+        y_ref = layer.train()(x)
+        z_ref = layer.get_aux_loss().clone()
+        before = lib.lmoe_launch_count()
+        y = layer.eval()(x)
+        assert (lib.lmoe_launch_count() - before == 4) == (T <= 64)
+        y2 = layer(x)
+    layer.check_status()
+    assert torch.equal(y, y2)                                             # deterministic
+    scores = torch.sigmoid(x.reshape(T, -1).float() @ layer.router.gate.weight.float().t()) + layer.router.expert_bias.float()
+    top = scores.topk(w.K + 1, dim=1).values if w.K < w.E else None
+    clear = (top[:, w.K - 1] - top[:, w.K] > 1e-5) if top is not None else torch.ones(T, dtype=torch.bool, device=x.device)
+    assert clear.float().mean().item() > 0.5
+    a, b = y.reshape(T, -1)[clear].float(), y_ref.reshape(T, -1)[clear].float()
+    assert ((a - b).norm() / b.norm()).item() <= 2.5e-3
+    rms = b.square().mean().sqrt()
+    assert ((a - b).abs() / torch.maximum(b.abs(), rms)).max().item() <= 2.0 ** -6
+    assert abs(layer.get_aux_loss().item() - z_ref.item()) <= 1e-5 * abs(z_ref.item())
+
+
+def test_gradients_and_training_mode_keep_the_padded_path():
+    from swamla_b200 import _cabi
+    from swamla_b200.layer import create_moe_layer
+    w = inputs.WORKLOADS["tiny"]
+    with torch.device("cuda:0"):
+        layer = create_moe_layer(w.config()).to(torch.bfloat16).eval()
+        x = torch.randn(2, 3, w.D).to(torch.bfloat16)
+    lib = _cabi.load()
+    before = lib.lmoe_launch_count()
+    y = layer(x.requires_grad_(True))                                    # evaluation mode with gradients: a backward may follow
+    assert lib.lmoe_launch_count() - before > 4
+    y.sum().backward()
+    assert x.grad is not None and layer.down_proj.weight.grad is not None
