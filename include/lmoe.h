@@ -201,7 +201,7 @@ int lmoe_shared_gateup_fwd(const lmoe_shape* s, const void* x, const void* w_gat
 int lmoe_combine_out_fwd(const lmoe_shape* s, const void* y_sorted, const lmoe_route* r, const float* weights,
                          void* act_cat, const void* w_down_s, const void* w_up, void* y, int32_t* status, void* stream);
 
-/* Whole forward of a few tokens (generation) in four launches without the padded layout: T <= LMOE_FEW_TOKENS, every other
+/* Whole forward of a few tokens (generation) in three or four launches without the padded layout: T <= LMOE_FEW_TOKENS, every other
  * dimension as lmoe_few_applies says.  With w_down = w_up = NULL and L = D: the non-latent layer (models/moe.py:344-372).
  * Same stages and rounding points as the entry points above (models/moe.py:702-734), fp32 sums in another order; the
  * expert weights are bf16 whatever the layer's precision for large batches.  Nothing is kept for a backward. */
@@ -211,7 +211,7 @@ size_t lmoe_few_workspace_bytes(const lmoe_shape* s);
 int lmoe_few_forward(const lmoe_shape* s, const void* x, const void* w_gate, const void* w_down, const void* w_up,
                      const void* w_gate_up_s, const void* w_down_s, const void* w_gate_up, const void* w_down_e,
                      const float* expert_bias, float z_coef, void* y, float* z_loss, void* workspace, size_t workspace_bytes,
-                     void* stream);
+                     int32_t* status, void* stream);
 
 /* ---- backward (adjoints of the lines cited above; the reference defines them only through
  *      autograd, and not at all for its grouped GEMM) ----

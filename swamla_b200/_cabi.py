@@ -62,7 +62,7 @@ SIGNATURES = {
     "lmoe_combine_out_fwd": (c_int, [SP, P, RP, P, P, P, P, P, P, P]),
     "lmoe_few_applies": (c_int, [SP]),
     "lmoe_few_workspace_bytes": (c_size_t, [SP]),
-    "lmoe_few_forward": (c_int, [SP, P, P, P, P, P, P, P, P, P, c_float, P, P, P, c_size_t, P]),
+    "lmoe_few_forward": (c_int, [SP, P, P, P, P, P, P, P, P, P, c_float, P, P, P, c_size_t, P, P]),
     "lmoe_combine_out_bwd_dgrad": (c_int, [SP, P, P, P, P, P, P, P, P, P]),
     "lmoe_combine_out_bwd_wgrad": (c_int, [SP, P, P, P, P, c_int, P, c_size_t, P, P]),
     "lmoe_combine_bwd": (c_int, [SP, P, P, P, RP, P, P, P]),

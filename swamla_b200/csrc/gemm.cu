@@ -262,13 +262,16 @@ static int launch_gemm_pair(const GemmCall& c) {
   }
   {
     const bool f32 = (c.epi == EPI_F32);
-    const long long cols = swiglu ? 2ll * c.N : c.N;
+    const bool adjoint = (c.epi == EPI_SWIGLU_BWD);
+    const long long cols = (swiglu || adjoint) ? 2ll * c.N : c.N;
     long long planes = 1, plane_elems = 0;
     if (split > 1) {
       planes = split;
       plane_elems = c.c_group_stride;
       if (plane_elems < static_cast<long long>(c.M) * c.ldc) return LMOE_ERR_ARG;
     }
+    if (adjoint)
+      if (int rc = encode_2d(&p.tmAux, c.aux, 2ll * c.N, c.M, c.ld_aux, kBM, 2)) return rc;
     int rc = c.C ? encode_out(&p.tmC, c.C, f32, cols, c.M, planes, c.ldc, plane_elems) : 0;
     if (rc) return rc;
     if (swiglu) {
@@ -297,28 +300,31 @@ static int launch_gemm_pair(const GemmCall& c) {
     case 2 | (EPI_F32 << 2): return launch_pair_inst<false, true, EPI_F32>(p, total, c.stream);
     case 3 | (EPI_F32 << 2): return launch_pair_inst<true, true, EPI_F32>(p, total, c.stream);
     case 0 | (EPI_SWIGLU << 2): return launch_pair_inst<false, false, EPI_SWIGLU>(p, total, c.stream);
+    case 2 | (EPI_SWIGLU_BWD << 2): return launch_pair_inst<false, true, EPI_SWIGLU_BWD>(p, total, c.stream);
     default: return LMOE_ERR_ARG;
   }
 }
 
 // Grouped-over-rows GEMM on CTA pairs: two tiles of the same expert share the expert's B loads (gemm_pair.cuh, GRP_M).
 // Needs the per-expert padded offsets; K-major A, one K segment, plain bf16 or SwiGLU epilogue.
-// Off unless the environment has LMOE_PAIR_GROUPED=1 (2: only the SwiGLU GEMM, 3: only the plain ones): with the
-// 256-element contractions of the routed experts a tile's main loop is four k-blocks long, an expert with an odd tile
-// count wastes half a pair and the last round of pairs is mostly empty (measured at E = 128, L = F = 256, 1,594 tiles:
-// gate_up + down 140 us on pairs against 134 us with one CTA per tile).
+// Used from kPairGroupedK elements of contraction on: with 256 a tile's main loop is four k-blocks long, an expert with an
+// odd tile count wastes half a pair and the last round of pairs is mostly empty (E = 128, L = F = 256, 1,594 tiles: gate_up +
+// down 140 us on pairs against 134 us with one CTA per tile; 512: even), while the long ones are bound by what an SM can pull
+// in (6,300 tiles: K = 768 311 -> 272 us, K = 1,536 553 -> 490 us; 112 tiles of 32 experts: K = 1,024 64 -> 60 us, K = 2,048
+// 61 -> 54 us).  LMOE_PAIR_GROUPED=1 puts every such GEMM on pairs (2: only the SwiGLU GEMM, 3: only the plain ones), 0 none.
+constexpr int kPairGroupedK = 768;
 static int pair_grouped_mode() {
   static int v = -1;
   if (v < 0) {
     const char* e = getenv("LMOE_PAIR_GROUPED");
-    v = (e && e[0] >= '1' && e[0] <= '3') ? e[0] - '0' : 0;
+    v = (e && e[0] >= '0' && e[0] <= '3') ? e[0] - '0' : 4;  // 4: by the length of the contraction
   }
   return v;
 }
 static bool pair_grouped_applies(const GemmCall& c) {
   const bool swiglu = (c.epi == EPI_SWIGLU);
   const int mode = pair_grouped_mode();
-  if (mode == 0 || (mode == 2 && !swiglu) || (mode == 3 && swiglu)) return false;
+  if (mode == 0 || (mode == 2 && !swiglu) || (mode == 3 && swiglu) || (mode == 4 && c.Kseg[0] < kPairGroupedK)) return false;
   return c.grp == GRP_M && c.pad_offsets && pair_gemm_enabled() && c.esz == 2 && !c.a_rows && !c.a_mn && c.nseg == 1 &&
          c.bn == 0 && (c.epi == EPI_BF16 || (swiglu && c.b_mn)) && c.groups > 0 && c.groups <= LMOE_MAX_EXPERTS &&
          c.padded_rows / kBM < (1 << 23) && (c.N % (swiglu ? 128 : 32)) == 0 && (c.Kseg[0] % 64) == 0;
@@ -383,7 +389,7 @@ int launch_gemm(const GemmCall& c) {
   const bool gather = c.a_rows != nullptr;
   if (pair_grouped_applies(c)) return launch_gemm_pair_grouped(c);
   if (c.grp == GRP_NONE && esz == 2 && !gather && c.bn != 128 && pair_gemm_applies(c.M, swiglu ? 2 * c.N : c.N) &&
-      (c.epi == EPI_BF16 || c.epi == EPI_F32 || (swiglu && !c.a_mn && !c.b_mn)))
+      (c.epi == EPI_BF16 || c.epi == EPI_F32 || (swiglu && !c.a_mn && !c.b_mn) || (swiglu_bwd && !c.a_mn && c.b_mn && c.nseg == 1)))
     return launch_gemm_pair(c);
   if (gather) {
     const bool shape_ok = (c.grp == GRP_M && !c.a_mn) || (c.grp == GRP_K && c.a_mn);

@@ -170,6 +170,29 @@ __device__ __forceinline__ void stage_row_f32(uint8_t* buf, int r, const float (
   }
 }
 
+// SwiGLU adjoint of 32 columns of one row: v = d_hidden (fp32 accumulator), wg / wu = saved gate / up (bf16 pairs) ->
+// pg = d_gate, pu = d_up.  d_hidden is rounded to bf16 first (what a stored d_hidden would hold), then
+//   d_up = dh * g * sig(g),  d_gate = dh * u * sig(g) * (1 + g * (1 - sig(g)))
+__device__ __forceinline__ void swiglu_adjoint_slab(const float (&v)[32], const uint32_t* wg, const uint32_t* wu,
+                                                    uint32_t (&pg)[16], uint32_t (&pu)[16]) {
+#pragma unroll
+  for (int j = 0; j < 16; ++j) {
+    const uint32_t dh2 = pack_bf16x2(v[2 * j], v[2 * j + 1]);
+    float dh[2] = {__uint_as_float(dh2 << 16), __uint_as_float(dh2 & 0xffff0000u)};
+    float g[2] = {__uint_as_float(wg[j] << 16), __uint_as_float(wg[j] & 0xffff0000u)};
+    float uu[2] = {__uint_as_float(wu[j] << 16), __uint_as_float(wu[j] & 0xffff0000u)};
+    float dg[2], du[2];
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      const float sg = sigmoid_fast(g[k]);
+      du[k] = dh[k] * g[k] * sg;
+      dg[k] = dh[k] * uu[k] * sg * (1.0f + g[k] * (1.0f - sg));
+    }
+    pg[j] = pack_bf16x2(dg[0], dg[1]);
+    pu[j] = pack_bf16x2(du[0], du[1]);
+  }
+}
+
 // ESZ = operand element size in bytes: 2 (bf16) or 1 (e4m3).
 template <bool A_MN, bool B_MN, int BN, int EPI, int GRP, int ESZ = 2>
 __global__ void __launch_bounds__(kGemmThreads, 1) gemm_kernel(const __grid_constant__ GemmParams p) {
@@ -565,26 +588,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_kernel(const __grid_cons
 #pragma unroll
           for (int j = 0; j < 16; ++j) pk[j] = pack_bf16x2(v[2 * j], v[2 * j + 1]);
         } else if (EPI == EPI_SWIGLU_BWD) {
-          const uint32_t* wg = reinterpret_cast<const uint32_t*>(hg);
-          const uint32_t* wu = reinterpret_cast<const uint32_t*>(hu);
-#pragma unroll
-          for (int j = 0; j < 16; ++j) {
-            // d_hidden is rounded to bf16 first (what a stored d_hidden would hold), then
-            //   d_up = dh * g * sig(g),  d_gate = dh * u * sig(g) * (1 + g * (1 - sig(g)))
-            const uint32_t dh2 = pack_bf16x2(v[2 * j], v[2 * j + 1]);
-            float dh[2] = {__uint_as_float(dh2 << 16), __uint_as_float(dh2 & 0xffff0000u)};
-            float g[2] = {__uint_as_float(wg[j] << 16), __uint_as_float(wg[j] & 0xffff0000u)};
-            float uu[2] = {__uint_as_float(wu[j] << 16), __uint_as_float(wu[j] & 0xffff0000u)};
-            float dg[2], du[2];
-#pragma unroll
-            for (int k = 0; k < 2; ++k) {
-              const float sg = sigmoid_fast(g[k]);
-              du[k] = dh[k] * g[k] * sg;
-              dg[k] = dh[k] * uu[k] * sg * (1.0f + g[k] * (1.0f - sg));
-            }
-            pk[j] = pack_bf16x2(dg[0], dg[1]);
-            pu[j] = pack_bf16x2(du[0], du[1]);
-          }
+          swiglu_adjoint_slab(v, reinterpret_cast<const uint32_t*>(hg), reinterpret_cast<const uint32_t*>(hu), pk, pu);
         } else if (EPI == EPI_SWIGLU) {
 #pragma unroll
           for (int j = 0; j < 16; ++j) {

@@ -12,7 +12,7 @@
 //   * only rank 0 issues MMAs; its tcgen05.commit arrives at the "empty" / "accumulator full" barriers of both CTAs;
 //   * the epilogue warps of both CTAs release an accumulator on rank 0's "accumulator empty" barrier (16 arrivals);
 //   * the CTAs meet at a cluster barrier after set-up and before tear-down.
-// Dense GEMMs only (no expert grouping), bf16 operands, BN = 256, epilogues bf16 / fp32 (split-K planes) / SwiGLU.
+// bf16 operands, BN = 256, epilogues bf16 / fp32 (split-K planes) / SwiGLU / SwiGLU adjoint.
 // Every wait is bounded as in gemm.cuh; a CTA whose wait expires stops issuing work, its partner's waits expire in turn.
 #pragma once
 #include "gemm.cuh"
@@ -25,14 +25,16 @@ struct PairSmem {
   static constexpr int kBBytes = 128 * kBKBytes;       // this CTA's half of the 256-wide B tile
   static constexpr int kStageBytes = kABytes + kBBytes;
   static constexpr int kSlabBytes = (EPI == EPI_F32) ? 16384 : 8192;
-  static constexpr int kStreams = (EPI == EPI_SWIGLU) ? 3 : 1;
+  static constexpr int kStreams = (EPI == EPI_SWIGLU) ? 3 : (EPI == EPI_SWIGLU_BWD) ? 2 : 1;
   static constexpr int kBufsPerGroup = (EPI == EPI_BF16) ? 2 : 1;
   static constexpr int kStagingBytes = 2 * kBufsPerGroup * kStreams * kSlabBytes;
   static constexpr int kBarrierBytes = 1536;  // barriers + the per-expert table of the grouped form (<= 257 ints)
-  static constexpr int kBudget = 232448 - 1024 - kBarrierBytes - kStagingBytes;
+  // EPI_SWIGLU_BWD: per epilogue group the saved gate / up of its next 64 columns (two 16 KB boxes)
+  static constexpr int kAuxBytes = (EPI == EPI_SWIGLU_BWD) ? 65536 : 0;
+  static constexpr int kBudget = 232448 - 1024 - kBarrierBytes - kStagingBytes - kAuxBytes;
   static constexpr int kStagesMax = kBudget / kStageBytes;
   static constexpr int kStages = kStagesMax > 6 ? 6 : kStagesMax;
-  static constexpr int kTotal = kStages * kStageBytes + kStagingBytes + kBarrierBytes + 1024;
+  static constexpr int kTotal = kStages * kStageBytes + kStagingBytes + kAuxBytes + kBarrierBytes + 1024;
   static_assert(kStages >= 4, "pipeline too shallow");
 };
 
@@ -57,11 +59,13 @@ gemm_pair_kernel(const __grid_constant__ GemmParams p) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* staging = smem + STAGES * S::kStageBytes;
-  uint64_t* bar_full = reinterpret_cast<uint64_t*>(staging + S::kStagingBytes);
+  uint8_t* aux_stage = staging + S::kStagingBytes;  // EPI_SWIGLU_BWD only
+  uint64_t* bar_full = reinterpret_cast<uint64_t*>(aux_stage + S::kAuxBytes);
   uint64_t* bar_empty = bar_full + STAGES;
   uint64_t* bar_tfull = bar_empty + STAGES;
   uint64_t* bar_tempty = bar_tfull + 2;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bar_tempty + 2);
+  uint64_t* bar_aux = bar_tempty + 2;  // [2]: one per epilogue group
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bar_aux + 2);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   int* etab = reinterpret_cast<int*>(tmem_slot + 2);  // GRP_M: first tile of expert e | experts before e with an odd tile count << 23
 
@@ -108,6 +112,8 @@ gemm_pair_kernel(const __grid_constant__ GemmParams p) {
       mbar_init(&bar_tfull[i], 1);
       mbar_init(&bar_tempty[i], 16);  // rank 0's: 8 epilogue warps of each CTA
     }
+    for (int i = 0; i < 2; ++i) mbar_init(&bar_aux[i], 1);
+    if (EPI == EPI_SWIGLU_BWD) tma_prefetch_desc(&p.tmAux);
     *abort_flag = 0;
     fence_mbar_init();
     for (int i = 0; i < p.nseg; ++i) {
@@ -292,6 +298,28 @@ gemm_pair_kernel(const __grid_constant__ GemmParams p) {
     int acc = 0;
     uint32_t acc_phase = 0;
     bool ok = true;
+    // Adjoint epilogue: group g owns the tile's columns [128 g, 128 g + 128) in two halves of 64; the saved gate / up of a
+    // half are staged as in gemm.cuh (two 128-row boxes, one buffer per group, taken into registers at the half's start),
+    // always one half ahead.
+    constexpr bool kAdj = (EPI == EPI_SWIGLU_BWD);
+    uint32_t aux_seq = 0;
+    int pre_id = pair_id, pre_half = 0;  // next half to stage (issuer only)
+    auto stage_next = [&]() {
+      while (pre_id < total_tiles) {
+        const Tile tt = decode(pre_id);
+        const int col = tt.nt * BN + group * 128 + pre_half * 64;
+        pre_half ^= 1;
+        if (pre_half == 0) pre_id += n_pairs;
+        if (col < p.N) {
+          uint8_t* dst = aux_stage + group * 32768;
+          mbar_expect_tx(&bar_aux[group], 32768);
+          tma_load_2d(dst, &p.tmAux, &bar_aux[group], col, tt.m0);                // rows / columns beyond the tensor: zeros
+          tma_load_2d(dst + 16384, &p.tmAux, &bar_aux[group], p.N + col, tt.m0);
+          return;
+        }
+      }
+    };
+    if (kAdj && issuer) stage_next();
     for (int id = pair_id; id < total_tiles && ok; id += n_pairs) {
       const Tile t = decode(id);
       const int nk = tile_kiters(t);
@@ -308,16 +336,32 @@ gemm_pair_kernel(const __grid_constant__ GemmParams p) {
       const int n_lim = kSwiglu ? p.half : p.N;
       int slabs = (n_lim - n0 + kSlabCols - 1) / kSlabCols;
       if (slabs > n_per_tile / kSlabCols) slabs = n_per_tile / kSlabCols;
-      const int last = ((slabs - 1 - group) >= 0) ? group + ((slabs - 1 - group) & ~1) : -1;
+      const int c_begin = kAdj ? 4 * group : group, c_step = kAdj ? 1 : 2, c_end = kAdj ? min(slabs, 4 * group + 4) : slabs;
+      const int last = (c_end > c_begin) ? c_begin + ((c_end - 1 - c_begin) / c_step) * c_step : -1;
       if (nk > 0 && last < 0) {
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive_cluster(tempty0);
       }
 
+      uint4 hg8[kAdj ? 8 : 1], hu8[kAdj ? 8 : 1];  // adjoint epilogue: saved gate / up of this row, the half's 64 columns
 #pragma unroll 1
-      for (int c = group; c < slabs; c += 2) {
+      for (int c = c_begin; c < c_end; c += c_step) {
         float v[32], u[32];
+        if (kAdj && ((c - c_begin) & 1) == 0) {
+          if (!mbar_wait(&bar_aux[group], aux_seq & 1, abort_flag, p.status, kStatusEpilogueTimeout)) ok = false;
+          const uint8_t* src = aux_stage + group * 32768 + r * 128;
+          const int sw = r & 7;
+#pragma unroll
+          for (int j = 0; j < (kAdj ? 8 : 0); ++j) {
+            hg8[j] = *reinterpret_cast<const uint4*>(src + ((j ^ sw) << 4));
+            hu8[j] = *reinterpret_cast<const uint4*>(src + 16384 + ((j ^ sw) << 4));
+          }
+          ++aux_seq;
+          ok = epi_bar_all(bar_id, ok);  // every thread of the group holds its rows: the buffer is free
+          if (!ok) break;
+          if (issuer) stage_next();
+        }
         if (nk > 0) {
           tmem_ld32(taddr + c * 32, v);
           if (kSwiglu) tmem_ld32(taddr + BN / 2 + c * 32, u);
@@ -344,6 +388,14 @@ gemm_pair_kernel(const __grid_constant__ GemmParams p) {
             const float u0 = __uint_as_float(pu[j] << 16), u1 = __uint_as_float(pu[j] & 0xffff0000u);
             ph[j] = pack_bf16x2(silu_f(g0) * u0, silu_f(g1) * u1);
           }
+        } else if (EPI == EPI_SWIGLU_BWD) {
+          uint4 hg[4], hu[4];  // this slab's 32 columns
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            hg[j] = ((c - c_begin) & 1) == 0 ? hg8[kAdj ? j : 0] : hg8[kAdj ? 4 + j : 0];
+            hu[j] = ((c - c_begin) & 1) == 0 ? hu8[kAdj ? j : 0] : hu8[kAdj ? 4 + j : 0];
+          }
+          swiglu_adjoint_slab(v, reinterpret_cast<const uint32_t*>(hg), reinterpret_cast<const uint32_t*>(hu), pk, pu);
         }
         if (kSwiglu && p.hidden_only) {  // as in gemm.cuh: one store per slab, two staging buffers in turn
           uint8_t* hbuf = sbuf0 + buf * S::kSlabBytes;
@@ -372,7 +424,7 @@ gemm_pair_kernel(const __grid_constant__ GemmParams p) {
         } else {
           stage_row_bf16(sbuf, r, pk);
           stage_row_bf16(sbuf + S::kSlabBytes, r, pu);
-          stage_row_bf16(sbuf + 2 * S::kSlabBytes, r, ph);
+          if (kSwiglu) stage_row_bf16(sbuf + 2 * S::kSlabBytes, r, ph);
         }
         fence_proxy_async_smem();
         epi_bar_sync(bar_id);
@@ -382,6 +434,9 @@ gemm_pair_kernel(const __grid_constant__ GemmParams p) {
             tma_store_3d(&p.tmC, sbuf, col, t.m0, 0);
             tma_store_3d(&p.tmC, sbuf + S::kSlabBytes, p.half + col, t.m0, 0);
             tma_store_3d(&p.tmC2, sbuf + 2 * S::kSlabBytes, col, t.m0, 0);
+          } else if (kAdj) {
+            tma_store_3d(&p.tmC, sbuf, col, t.m0, 0);                        // d_gate
+            tma_store_3d(&p.tmC, sbuf + S::kSlabBytes, p.N + col, t.m0, 0);  // d_up
           } else {
             tma_store_3d(&p.tmC, sbuf, col, t.m0, t.plane);
           }

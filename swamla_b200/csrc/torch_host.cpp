@@ -694,7 +694,7 @@ std::vector<Tensor> few_forward(const Sizes& d, const Tensor& x2d, const Tensor&
   Tensor ws = new_bytes(n, x2d);
   LMOE(lmoe_few_forward, &d.s, x2d.data_ptr(), wg.data_ptr(), wdn ? wdn->data_ptr() : nullptr, wup ? wup->data_ptr() : nullptr,
        wgus.data_ptr(), wds.data_ptr(), wgu.data_ptr(), wde.data_ptr(), bias.data_ptr<float>(), z_coef, y.data_ptr(),
-       z.data_ptr<float>(), ws.data_ptr(), n, at::cuda::getCurrentCUDAStream().stream());
+       z.data_ptr<float>(), ws.data_ptr(), n, status_word(wdn ? kLatentFwd : kMoeFwd), at::cuda::getCurrentCUDAStream().stream());
   return {y, z};
 }
 

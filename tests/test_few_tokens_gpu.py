@@ -37,7 +37,7 @@ def test_few_token_forward_matches_padded_path(name, T):
         z_ref = layer.get_aux_loss().clone()
         before = lib.lmoe_launch_count()
         y = layer.eval()(x)
-        assert (lib.lmoe_launch_count() - before == 4) == (T <= 64)
+        assert (lib.lmoe_launch_count() - before <= 4) == (T <= 64)
         y2 = layer(x)
     layer.check_status()
     assert torch.equal(y, y2)                                             # deterministic
