@@ -488,6 +488,16 @@ int lmoe_rmsnorm_fwd(const void* x, const float* weight, float eps, int64_t T, i
 int lmoe_add_bf16(const void* a, const void* b, void* out, int64_t n, void* stream);
 int lmoe_rmsnorm_bwd(const void* x, const float* weight, const float* rstd, const void* d_xn, const void* d_residual,
                      int64_t T, int D, void* dx, float* d_weight, void* workspace, size_t workspace_bytes, void* stream);
+/* The same kernels for rows and weights in either type (LMOE_BF16 / LMOE_F32): x, d_residual and dx share x_type; xn and d_xn
+ * have their own (the layers compute in bf16 whatever the residual stream is); d_weight in dw_type.  lmoe_add_f32_bf16:
+ * out = a + b, an fp32 stream and a bf16 branch.  Without them every step of an fp32 block pays for widened and narrowed
+ * copies of its activations (mla_block.py:83-85 under the autocast of train.py:1195). */
+int lmoe_rmsnorm_fwd_typed(const void* x, int x_type, const void* weight, int w_type, float eps, int64_t T, int D, void* xn,
+                           int xn_type, float* rstd, void* stream);
+int lmoe_rmsnorm_bwd_typed(const void* x, int x_type, const void* weight, int w_type, const float* rstd, const void* d_xn,
+                           int g_type, const void* d_residual, int64_t T, int D, void* dx, void* d_weight, int dw_type,
+                           void* workspace, size_t workspace_bytes, void* stream);
+int lmoe_add_f32_bf16(const float* a, const void* b, float* out, int64_t n, void* stream);
 
 /* ---- router bias update (after backward) ----
  * load = histogram(sel) (= counts); bias -= gamma * sign(load - T*K/E); history = .99 history + .01 load.

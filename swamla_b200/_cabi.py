@@ -114,6 +114,9 @@ SIGNATURES = {
     "lmoe_rmsnorm_fwd": (c_int, [P, P, c_float, c_int64, c_int, P, P, P]),
     "lmoe_add_bf16": (c_int, [P, P, P, c_int64, P]),
     "lmoe_rmsnorm_bwd": (c_int, [P, P, P, P, P, c_int64, c_int, P, P, P, c_size_t, P]),
+    "lmoe_rmsnorm_fwd_typed": (c_int, [P, c_int, P, c_int, c_float, c_int64, c_int, P, c_int, P, P]),
+    "lmoe_rmsnorm_bwd_typed": (c_int, [P, c_int, P, c_int, P, P, c_int, P, c_int64, c_int, P, P, c_int, P, c_size_t, P]),
+    "lmoe_add_f32_bf16": (c_int, [P, P, P, c_int64, P]),
     "lmoe_moe_wgrad_workspace_bytes": (c_size_t, [SP]),
     "lmoe_moe_shared_bwd": (c_int, [SP, P, P, P, P, P, P, c_int, P, c_size_t, P, P]),
     "lmoe_moe_xside_bwd": (c_int, [SP, P, P, P, P, P, P, P, c_int, P, c_size_t, P, P]),

@@ -6,9 +6,12 @@
 //   rmsnorm_bwd   dx[t] = rstd * (g - x * rstd^2 * mean(g * x)) + d_res[t],  g = d_xn * w     one kernel for the adjoint of the
 //                 d_w[d] = sum_t d_xn[t,d] * x[t,d] * rstd[t]                                  norm AND the residual branch
 //
-// bf16 rows, fp32 arithmetic, one warp per row with the row held in registers (D <= 2048).  The weight gradient is a
-// two-stage sum in a fixed order (per-warp registers -> per-block shared memory in warp order -> per-block partials ->
-// final kernel), so it is deterministic; no atomics.
+// Rows in bf16 or fp32 (the residual stream of mixed-precision training), fp32 arithmetic, one warp per row with the row held
+// in registers (D <= 2048).  HBM-bound by design, latency-bound in practice below some 10,000 rows: what counts is that
+// every load of a row is in flight at once and that no pass over the activations is spent on a conversion (with fp32 rows
+// converted before and after, the norm, its adjoint and the add of a 4,095-row block took 120 us in 11 launches; now four).
+// The weight gradient is a two-stage sum in a fixed order (per-warp registers -> the block's warps in order -> per-block
+// partials -> final kernel), so it is deterministic; no atomics.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -19,7 +22,7 @@
 namespace lmoe {
 
 constexpr int kNormWarps = 8;
-constexpr int kNormMaxChunks = 8;  // 16-byte chunks per lane: D <= 8 * 32 * 8 = 2048
+constexpr int kNormMaxChunks = 8;  // 8-element chunks per lane: D <= 8 * 32 * 8 = 2048
 constexpr int kNormMaxBlocks = 296;
 
 __device__ __forceinline__ void nrm_unpack(const uint4& v, float (&f)[8]) {
@@ -38,46 +41,85 @@ __device__ __forceinline__ uint4 nrm_pack(const float (&f)[8]) {
   for (int i = 0; i < 4; ++i) h[i] = __floats2bfloat162_rn(f[2 * i], f[2 * i + 1]);
   return v;
 }
+// Eight consecutive elements of a row in either type, kept as loaded until they are used.
+template <bool F32>
+struct Chunk {
+  uint4 v[F32 ? 2 : 1];
+  __device__ __forceinline__ void load(const void* base, long long chunk) {
+    const uint4* p = static_cast<const uint4*>(base) + chunk * (F32 ? 2 : 1);
+    v[0] = p[0];
+    if (F32) v[F32 ? 1 : 0] = p[1];
+  }
+  __device__ __forceinline__ void get(float (&f)[8]) const {
+    if (F32) {
+      const float* q = reinterpret_cast<const float*>(v);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) f[j] = q[F32 ? j : 0];
+    } else {
+      nrm_unpack(v[0], f);
+    }
+  }
+};
+template <bool F32>
+__device__ __forceinline__ void store_chunk(void* base, long long chunk, const float (&f)[8]) {
+  if (F32) {
+    float4* p = static_cast<float4*>(base) + chunk * 2;
+    p[0] = make_float4(f[0], f[1], f[2], f[3]);
+    p[1] = make_float4(f[4], f[5], f[6], f[7]);
+  } else {
+    static_cast<uint4*>(base)[chunk] = nrm_pack(f);
+  }
+}
+// Eight weights from chunk v of a bf16 or fp32 vector (L1-resident; the type is uniform over the launch).
+__device__ __forceinline__ void load_weight(const void* w, bool f32, int v, float (&f)[8]) {
+  if (f32) {
+    const float4 a = static_cast<const float4*>(w)[2 * v], b = static_cast<const float4*>(w)[2 * v + 1];
+    f[0] = a.x, f[1] = a.y, f[2] = a.z, f[3] = a.w, f[4] = b.x, f[5] = b.y, f[6] = b.z, f[7] = b.w;
+  } else {
+    nrm_unpack(static_cast<const uint4*>(w)[v], f);
+  }
+}
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
   return v;
 }
 
+// X32: type of x; Y32: type of xn.  CH chunks per lane cover the row.
+template <bool X32, bool Y32, int CH>
 __global__ void __launch_bounds__(kNormWarps * 32)
-rmsnorm_fwd_kernel(const uint4* __restrict__ x, const float* __restrict__ w, float eps, long long T, int vec_per_row,
-                   uint4* __restrict__ xn, float* __restrict__ rstd) {
+rmsnorm_fwd_kernel(const void* __restrict__ x, const void* __restrict__ w, bool w32, float eps, long long T, int vec_per_row,
+                   void* __restrict__ xn, float* __restrict__ rstd) {
   const int lane = threadIdx.x & 31;
   const float inv_d = 1.0f / static_cast<float>(vec_per_row * 8);
   for (long long t = static_cast<long long>(blockIdx.x) * kNormWarps + (threadIdx.x >> 5); t < T;
        t += static_cast<long long>(gridDim.x) * kNormWarps) {
-    uint4 row[kNormMaxChunks];
+    Chunk<X32> row[CH];
+#pragma unroll
+    for (int i = 0; i < CH; ++i)
+      if (lane + 32 * i < vec_per_row) row[i].load(x, t * vec_per_row + lane + 32 * i);
     float ss = 0.f;
 #pragma unroll
-    for (int i = 0; i < kNormMaxChunks; ++i) {
-      const int v = lane + 32 * i;
-      if (v < vec_per_row) {
-        row[i] = x[t * vec_per_row + v];
+    for (int i = 0; i < CH; ++i)
+      if (lane + 32 * i < vec_per_row) {
         float f[8];
-        nrm_unpack(row[i], f);
+        row[i].get(f);
 #pragma unroll
         for (int j = 0; j < 8; ++j) ss = fmaf(f[j], f[j], ss);
       }
-    }
     ss = warp_sum(ss);
     const float r = rsqrtf(ss * inv_d + eps);
     if (lane == 0) rstd[t] = r;
 #pragma unroll
-    for (int i = 0; i < kNormMaxChunks; ++i) {
+    for (int i = 0; i < CH; ++i) {
       const int v = lane + 32 * i;
       if (v < vec_per_row) {
-        float f[8], o[8];
-        nrm_unpack(row[i], f);
-        const float4 w0 = reinterpret_cast<const float4*>(w)[2 * v], w1 = reinterpret_cast<const float4*>(w)[2 * v + 1];
-        const float ww[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
+        float f[8], ww[8], o[8];
+        row[i].get(f);
+        load_weight(w, w32, v, ww);
 #pragma unroll
         for (int j = 0; j < 8; ++j) o[j] = ww[j] * (f[j] * r);
-        xn[t * vec_per_row + v] = nrm_pack(o);
+        store_chunk<Y32>(xn, t * vec_per_row + v, o);
       }
     }
   }
@@ -95,38 +137,64 @@ add_bf16_kernel(const uint4* __restrict__ a, const uint4* __restrict__ b, uint4*
     out[i] = nrm_pack(fa);
   }
 }
+// out = a + b with a wide stream and bf16 addends: no widened copy of b
+__global__ void __launch_bounds__(256)
+add_f32_bf16_kernel(const void* __restrict__ a, const void* __restrict__ b, void* __restrict__ out, long long n_vec) {
+  for (long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x; i < n_vec;
+       i += static_cast<long long>(gridDim.x) * blockDim.x) {
+    Chunk<true> ca;
+    Chunk<false> cb;
+    ca.load(a, i);
+    cb.load(b, i);
+    float fa[8], fb[8];
+    ca.get(fa);
+    cb.get(fb);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) fa[j] += fb[j];
+    store_chunk<true>(out, i, fa);
+  }
+}
 
-// partial[blockIdx.x][D]: this block's share of d_w.  Shared memory: D floats (dynamic).
+// partial[blockIdx.x][D]: this block's share of d_w.  Shared memory: one row of D floats per warp (dynamic).
+// X32: type of x, d_res and dx; G32: type of d_xn.
+template <bool X32, bool G32, int CH>
 __global__ void __launch_bounds__(kNormWarps * 32)
-rmsnorm_bwd_kernel(const uint4* __restrict__ x, const float* __restrict__ w, const float* __restrict__ rstd,
-                   const uint4* __restrict__ d_xn, const uint4* __restrict__ d_res, long long T, int vec_per_row,
-                   uint4* __restrict__ dx, float* __restrict__ partial) {
+rmsnorm_bwd_kernel(const void* __restrict__ x, const void* __restrict__ w, bool w32, const float* __restrict__ rstd,
+                   const void* __restrict__ d_xn, const void* __restrict__ d_res, long long T, int vec_per_row,
+                   void* __restrict__ dx, float* __restrict__ partial) {
   extern __shared__ float s_dw[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int D = vec_per_row * 8;
   const float inv_d = 1.0f / static_cast<float>(D);
-  float dw[kNormMaxChunks][8];
+  float dw[CH][8];
 #pragma unroll
-  for (int i = 0; i < kNormMaxChunks; ++i)
+  for (int i = 0; i < CH; ++i)
 #pragma unroll
     for (int j = 0; j < 8; ++j) dw[i][j] = 0.f;
 
   for (long long t = static_cast<long long>(blockIdx.x) * kNormWarps + warp; t < T;
        t += static_cast<long long>(gridDim.x) * kNormWarps) {
     const float r = rstd[t];
-    uint4 xr[kNormMaxChunks], gr[kNormMaxChunks];
-    float dot = 0.f;
+    Chunk<X32> xr[CH], rr[CH];
+    Chunk<G32> gr[CH];
 #pragma unroll
-    for (int i = 0; i < kNormMaxChunks; ++i) {
+    for (int i = 0; i < CH; ++i) {
       const int v = lane + 32 * i;
       if (v < vec_per_row) {
-        xr[i] = x[t * vec_per_row + v];
-        gr[i] = d_xn[t * vec_per_row + v];
-        float fx[8], fg[8];
-        nrm_unpack(xr[i], fx);
-        nrm_unpack(gr[i], fg);
-        const float4 w0 = reinterpret_cast<const float4*>(w)[2 * v], w1 = reinterpret_cast<const float4*>(w)[2 * v + 1];
-        const float ww[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
+        xr[i].load(x, t * vec_per_row + v);
+        gr[i].load(d_xn, t * vec_per_row + v);
+        if (d_res) rr[i].load(d_res, t * vec_per_row + v);
+      }
+    }
+    float dot = 0.f;
+#pragma unroll
+    for (int i = 0; i < CH; ++i) {
+      const int v = lane + 32 * i;
+      if (v < vec_per_row) {
+        float fx[8], fg[8], ww[8];
+        xr[i].get(fx);
+        gr[i].get(fg);
+        load_weight(w, w32, v, ww);
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
           dot = fmaf(fg[j] * ww[j], fx[j], dot);
@@ -137,53 +205,67 @@ rmsnorm_bwd_kernel(const uint4* __restrict__ x, const float* __restrict__ w, con
     dot = warp_sum(dot);
     const float c = r * r * r * dot * inv_d;  // rstd^3 * mean(g * x)
 #pragma unroll
-    for (int i = 0; i < kNormMaxChunks; ++i) {
+    for (int i = 0; i < CH; ++i) {
       const int v = lane + 32 * i;
       if (v < vec_per_row) {
-        float fx[8], fg[8], o[8];
-        nrm_unpack(xr[i], fx);
-        nrm_unpack(gr[i], fg);
-        const float4 w0 = reinterpret_cast<const float4*>(w)[2 * v], w1 = reinterpret_cast<const float4*>(w)[2 * v + 1];
-        const float ww[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
+        float fx[8], fg[8], ww[8], o[8];
+        xr[i].get(fx);
+        gr[i].get(fg);
+        load_weight(w, w32, v, ww);
 #pragma unroll
         for (int j = 0; j < 8; ++j) o[j] = fg[j] * ww[j] * r - fx[j] * c;
         if (d_res) {
           float fr[8];
-          nrm_unpack(d_res[t * vec_per_row + v], fr);
+          rr[i].get(fr);
 #pragma unroll
           for (int j = 0; j < 8; ++j) o[j] += fr[j];
         }
-        dx[t * vec_per_row + v] = nrm_pack(o);
+        store_chunk<X32>(dx, t * vec_per_row + v, o);
       }
     }
   }
-  // block sum of the weight-gradient partials, warp after warp (fixed order)
-  for (int wi = 0; wi < kNormWarps; ++wi) {
-    if (warp == wi) {
 #pragma unroll
-      for (int i = 0; i < kNormMaxChunks; ++i) {
-        const int v = lane + 32 * i;
-        if (v < vec_per_row) {
-#pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            const int d = v * 8 + j;
-            s_dw[d] = (wi == 0 ? 0.f : s_dw[d]) + dw[i][j];
-          }
-        }
-      }
+  for (int i = 0; i < CH; ++i) {
+    const int v = lane + 32 * i;
+    if (v < vec_per_row) {
+      float4* q = reinterpret_cast<float4*>(s_dw + warp * D + v * 8);
+      q[0] = make_float4(dw[i][0], dw[i][1], dw[i][2], dw[i][3]);
+      q[1] = make_float4(dw[i][4], dw[i][5], dw[i][6], dw[i][7]);
     }
-    __syncthreads();
   }
-  for (int d = threadIdx.x; d < D; d += blockDim.x) partial[static_cast<long long>(blockIdx.x) * D + d] = s_dw[d];
+  __syncthreads();
+  for (int d = threadIdx.x; d < D; d += blockDim.x) {
+    float s = s_dw[d];
+#pragma unroll
+    for (int wi = 1; wi < kNormWarps; ++wi) s += s_dw[wi * D + d];
+    partial[static_cast<long long>(blockIdx.x) * D + d] = s;
+  }
 }
 
-__global__ void __launch_bounds__(256)
-rmsnorm_dw_finalize_kernel(const float* __restrict__ partial, int blocks, int D, float* __restrict__ d_w) {
-  const int d = blockIdx.x * blockDim.x + threadIdx.x;
-  if (d >= D) return;
+// d_w[d] = sum over the blocks' partials: 32 columns per block, each warp sums a contiguous share of the blocks, then the
+// warps' sums are added in order.  (One thread per column over all 296 blocks took 11 us, a chain of dependent loads.)
+__global__ void __launch_bounds__(kNormWarps * 32)
+rmsnorm_dw_finalize_kernel(const float* __restrict__ partial, int blocks, int D, void* __restrict__ d_w, bool f32) {
+  __shared__ float s_sum[kNormWarps][32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int d = blockIdx.x * 32 + lane;
+  const int per = (blocks + kNormWarps - 1) / kNormWarps, b0 = warp * per, b1 = min(b0 + per, blocks);
   float s = 0.f;
-  for (int b = 0; b < blocks; ++b) s += partial[static_cast<long long>(b) * D + d];
-  d_w[d] = s;
+  if (d < D) {
+#pragma unroll 8
+    for (int b = b0; b < b1; ++b) s += partial[static_cast<long long>(b) * D + d];
+  }
+  s_sum[warp][lane] = s;
+  __syncthreads();
+  if (warp == 0 && d < D) {
+    float v = s_sum[0][lane];
+#pragma unroll
+    for (int wi = 1; wi < kNormWarps; ++wi) v += s_sum[wi][lane];
+    if (f32)
+      static_cast<float*>(d_w)[d] = v;
+    else
+      static_cast<__nv_bfloat16*>(d_w)[d] = __float2bfloat16_rn(v);
+  }
 }
 
 static inline int norm_blocks(long long T) {
@@ -193,6 +275,7 @@ static inline int norm_blocks(long long T) {
   return static_cast<int>(b);
 }
 static inline int norm_last_error() {
+  count_launch();
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : static_cast<int>(e);
 }
@@ -200,6 +283,7 @@ static inline bool norm_dims_ok(long long T, int D) {
   return T > 0 && D > 0 && (D & 7) == 0 && D <= kNormMaxChunks * 256;
 }
 static inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
+static inline bool is_type(int t) { return t == LMOE_BF16 || t == LMOE_F32; }
 
 }  // namespace lmoe
 
@@ -209,46 +293,80 @@ extern "C" size_t lmoe_rmsnorm_workspace_bytes(int D) {
   return D > 0 ? static_cast<size_t>(kNormMaxBlocks) * D * sizeof(float) : 0;
 }
 
-extern "C" int lmoe_rmsnorm_fwd(const void* x, const float* weight, float eps, int64_t T, int D, void* xn, float* rstd,
-                                void* stream) {
-  if (!x || !weight || !xn || !rstd) return LMOE_ERR_ARG;
+extern "C" int lmoe_rmsnorm_fwd_typed(const void* x, int x_type, const void* weight, int w_type, float eps, int64_t T, int D,
+                                      void* xn, int xn_type, float* rstd, void* stream) {
+  if (!x || !weight || !xn || !rstd || !is_type(x_type) || !is_type(w_type) || !is_type(xn_type)) return LMOE_ERR_ARG;
   if (!norm_dims_ok(T, D)) return LMOE_ERR_SHAPE;
   if (!aligned16(x) || !aligned16(xn) || !aligned16(weight)) return LMOE_ERR_ALIGN;
-  rmsnorm_fwd_kernel<<<norm_blocks(T), kNormWarps * 32, 0, static_cast<cudaStream_t>(stream)>>>(
-      static_cast<const uint4*>(x), weight, eps, T, D / 8, static_cast<uint4*>(xn), rstd);
-  count_launch();
+  auto pick = [&](auto narrow, auto wide) { return D <= 1024 ? narrow : wide; };
+  auto k = x_type == LMOE_BF16 ? (xn_type == LMOE_BF16 ? pick(rmsnorm_fwd_kernel<false, false, 4>, rmsnorm_fwd_kernel<false, false, 8>)
+                                                       : pick(rmsnorm_fwd_kernel<false, true, 4>, rmsnorm_fwd_kernel<false, true, 8>))
+                               : (xn_type == LMOE_BF16 ? pick(rmsnorm_fwd_kernel<true, false, 4>, rmsnorm_fwd_kernel<true, false, 8>)
+                                                       : pick(rmsnorm_fwd_kernel<true, true, 4>, rmsnorm_fwd_kernel<true, true, 8>));
+  long long blocks = (T + kNormWarps - 1) / kNormWarps;   // no per-block result here: a warp per row up to 16 blocks per SM
+  if (blocks > 148 * 16) blocks = 148 * 16;
+  k<<<static_cast<int>(blocks), kNormWarps * 32, 0, static_cast<cudaStream_t>(stream)>>>(x, weight, w_type == LMOE_F32, eps, T, D / 8, xn,
+                                                                                        rstd);
   return norm_last_error();
 }
 
+extern "C" int lmoe_rmsnorm_fwd(const void* x, const float* weight, float eps, int64_t T, int D, void* xn, float* rstd,
+                                void* stream) {
+  return lmoe_rmsnorm_fwd_typed(x, LMOE_BF16, weight, LMOE_F32, eps, T, D, xn, LMOE_BF16, rstd, stream);
+}
+
+static int add_blocks(long long n_vec) {
+  const long long blocks = (n_vec + 255) / 256;
+  return static_cast<int>(blocks > 148ll * 16 ? 148ll * 16 : blocks);
+}
 extern "C" int lmoe_add_bf16(const void* a, const void* b, void* out, int64_t n, void* stream) {
   if (!a || !b || !out) return LMOE_ERR_ARG;
   if (n <= 0 || (n & 7) != 0) return LMOE_ERR_SHAPE;
   if (!aligned16(a) || !aligned16(b) || !aligned16(out)) return LMOE_ERR_ALIGN;
-  const long long n_vec = n / 8;
-  long long blocks = (n_vec + 255) / 256;
-  if (blocks > 148ll * 16) blocks = 148ll * 16;
-  add_bf16_kernel<<<static_cast<int>(blocks), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-      static_cast<const uint4*>(a), static_cast<const uint4*>(b), static_cast<uint4*>(out), n_vec);
-  count_launch();
+  add_bf16_kernel<<<add_blocks(n / 8), 256, 0, static_cast<cudaStream_t>(stream)>>>(
+      static_cast<const uint4*>(a), static_cast<const uint4*>(b), static_cast<uint4*>(out), n / 8);
+  return norm_last_error();
+}
+extern "C" int lmoe_add_f32_bf16(const float* a, const void* b, float* out, int64_t n, void* stream) {
+  if (!a || !b || !out) return LMOE_ERR_ARG;
+  if (n <= 0 || (n & 7) != 0) return LMOE_ERR_SHAPE;
+  if (!aligned16(a) || !aligned16(b) || !aligned16(out)) return LMOE_ERR_ALIGN;
+  add_f32_bf16_kernel<<<add_blocks(n / 8), 256, 0, static_cast<cudaStream_t>(stream)>>>(a, b, out, n / 8);
+  return norm_last_error();
+}
+
+extern "C" int lmoe_rmsnorm_bwd_typed(const void* x, int x_type, const void* weight, int w_type, const float* rstd,
+                                      const void* d_xn, int g_type, const void* d_residual, int64_t T, int D, void* dx,
+                                      void* d_weight, int dw_type, void* workspace, size_t workspace_bytes, void* stream) {
+  if (!x || !weight || !rstd || !d_xn || !dx || !d_weight || !workspace) return LMOE_ERR_ARG;
+  if (!is_type(x_type) || !is_type(w_type) || !is_type(g_type) || !is_type(dw_type)) return LMOE_ERR_ARG;
+  if (!norm_dims_ok(T, D)) return LMOE_ERR_SHAPE;
+  if (workspace_bytes < lmoe_rmsnorm_workspace_bytes(D)) return LMOE_ERR_WORKSPACE;
+  if (!aligned16(x) || !aligned16(d_xn) || !aligned16(dx) || !aligned16(weight) || (d_residual && !aligned16(d_residual)))
+    return LMOE_ERR_ALIGN;
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  auto pick = [&](auto narrow, auto wide) { return D <= 1024 ? narrow : wide; };
+  auto k = x_type == LMOE_BF16 ? (g_type == LMOE_BF16 ? pick(rmsnorm_bwd_kernel<false, false, 4>, rmsnorm_bwd_kernel<false, false, 8>)
+                                                      : pick(rmsnorm_bwd_kernel<false, true, 4>, rmsnorm_bwd_kernel<false, true, 8>))
+                               : (g_type == LMOE_BF16 ? pick(rmsnorm_bwd_kernel<true, false, 4>, rmsnorm_bwd_kernel<true, false, 8>)
+                                                      : pick(rmsnorm_bwd_kernel<true, true, 4>, rmsnorm_bwd_kernel<true, true, 8>));
+  const size_t smem = static_cast<size_t>(kNormWarps) * D * sizeof(float);   // up to 64 KB
+  if (smem > 48 * 1024) {
+    const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+    if (e != cudaSuccess) return static_cast<int>(e);
+  }
+  const int blocks = norm_blocks(T);
+  k<<<blocks, kNormWarps * 32, smem, st>>>(x, weight, w_type == LMOE_F32, rstd, d_xn, d_residual, T, D / 8, dx,
+                                          static_cast<float*>(workspace));
+  if (int rc = norm_last_error()) return rc;
+  rmsnorm_dw_finalize_kernel<<<(D + 31) / 32, kNormWarps * 32, 0, st>>>(static_cast<const float*>(workspace), blocks, D, d_weight,
+                                                                       dw_type == LMOE_F32);
   return norm_last_error();
 }
 
 extern "C" int lmoe_rmsnorm_bwd(const void* x, const float* weight, const float* rstd, const void* d_xn,
                                 const void* d_residual, int64_t T, int D, void* dx, float* d_weight, void* workspace,
                                 size_t workspace_bytes, void* stream) {
-  if (!x || !weight || !rstd || !d_xn || !dx || !d_weight || !workspace) return LMOE_ERR_ARG;
-  if (!norm_dims_ok(T, D)) return LMOE_ERR_SHAPE;
-  if (workspace_bytes < lmoe_rmsnorm_workspace_bytes(D)) return LMOE_ERR_WORKSPACE;
-  if (!aligned16(x) || !aligned16(d_xn) || !aligned16(dx) || !aligned16(weight) || (d_residual && !aligned16(d_residual)))
-    return LMOE_ERR_ALIGN;
-  cudaStream_t st = static_cast<cudaStream_t>(stream);
-  const int blocks = norm_blocks(T);
-  rmsnorm_bwd_kernel<<<blocks, kNormWarps * 32, static_cast<size_t>(D) * sizeof(float), st>>>(
-      static_cast<const uint4*>(x), weight, rstd, static_cast<const uint4*>(d_xn), static_cast<const uint4*>(d_residual),
-      T, D / 8, static_cast<uint4*>(dx), static_cast<float*>(workspace));
-  count_launch();
-  if (int rc = norm_last_error()) return rc;
-  rmsnorm_dw_finalize_kernel<<<(D + 255) / 256, 256, 0, st>>>(static_cast<const float*>(workspace), blocks, D, d_weight);
-  count_launch();
-  return norm_last_error();
+  return lmoe_rmsnorm_bwd_typed(x, LMOE_BF16, weight, LMOE_F32, rstd, d_xn, LMOE_BF16, d_residual, T, D, dx, d_weight, LMOE_F32,
+                                workspace, workspace_bytes, stream);
 }

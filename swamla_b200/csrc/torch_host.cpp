@@ -823,6 +823,89 @@ class MoeFn : public torch::autograd::Function<MoeFn> {
   }
 };
 
+// ---------------------------------------------------------------- norm and residual either side of a feed-forward layer
+int lmoe_type(const Tensor& t) { return t.scalar_type() == at::kFloat ? LMOE_F32 : LMOE_BF16; }
+// bf16 and fp32 pass as they are; anything else in fp32
+Tensor rows_of(const Tensor& t) {
+  const Tensor d = t.detach();
+  return (d.scalar_type() == at::kFloat || d.scalar_type() == at::kBFloat16 ? d : d.to(at::kFloat)).contiguous();
+}
+
+// (xn, x_pass) = (rmsnorm(x) * weight, x).  x_pass is x itself, handed on to the residual add, so that the backward sees the
+// gradients of both branches in one call and adds them inside the norm's adjoint.
+class NormFn : public torch::autograd::Function<NormFn> {
+ public:
+  static variable_list forward(AutogradContext* ctx, const Tensor& x, const Tensor& weight, double eps, bool bf16_out) {
+    const Tensor xr = rows_of(x), w = rows_of(weight);
+    const int64_t D = x.size(-1), T = xr.numel() / D;
+    const bool wide = !bf16_out && xr.scalar_type() == at::kFloat;
+    Tensor xn = at::empty(x.sizes(), xr.options().dtype(wide ? at::kFloat : at::kBFloat16));
+    Tensor rstd = at::empty({T}, xr.options().dtype(at::kFloat));
+    LMOE(lmoe_rmsnorm_fwd_typed, xr.data_ptr(), lmoe_type(xr), w.data_ptr(), lmoe_type(w), static_cast<float>(eps), T, static_cast<int>(D),
+         xn.data_ptr(), lmoe_type(xn), rstd.data_ptr<float>(), at::cuda::getCurrentCUDAStream().stream());
+    ctx->set_materialize_grads(false);
+    ctx->save_for_backward({xr, w, rstd});
+    ctx->saved_data["t"] = dtypes_of({x, weight});
+    return {bf16_out ? xn : as_param(xn, x.scalar_type()), x};
+  }
+
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    try {
+      const auto sv = ctx->get_saved_variables();
+      const Tensor &x = sv[0], &w = sv[1], &rstd = sv[2];
+      const c10::cuda::CUDAGuard guard(x.device());
+      const auto t = ctx->saved_data["t"].toIntVector();
+      const auto x_type = static_cast<at::ScalarType>(t[0]), w_type = static_cast<at::ScalarType>(t[1]);
+      const int64_t D = x.size(-1), T = x.numel() / D;
+      const Tensor g = grads[0].defined() ? rows_of(grads[0]) : at::zeros_like(x);
+      Tensor r;
+      if (grads[1].defined()) r = rows_of(grads[1]).to(x.scalar_type()).contiguous();
+      Tensor dx = at::empty_like(x);
+      Tensor dw = at::empty({D}, x.options().dtype(w.scalar_type()));
+      Tensor ws = new_bytes(lmoe_rmsnorm_workspace_bytes(static_cast<int>(D)), x);
+      LMOE(lmoe_rmsnorm_bwd_typed, x.data_ptr(), lmoe_type(x), w.data_ptr(), lmoe_type(w), rstd.data_ptr<float>(), g.data_ptr(),
+           lmoe_type(g), r.defined() ? r.data_ptr() : nullptr, T, static_cast<int>(D), dx.data_ptr(), dw.data_ptr(), lmoe_type(dw),
+           ws.data_ptr(), static_cast<size_t>(ws.numel()), at::cuda::getCurrentCUDAStream().stream());
+      const Tensor none;
+      return {as_param(dx, x_type), as_param(dw, w_type), none, none};
+    } catch (const LmoeFailure& e) {
+      rethrow_as_python(e);
+    }
+  }
+};
+
+// out = a + b in a's dtype; both inputs receive the output's gradient, in their own dtype.
+class AddFn : public torch::autograd::Function<AddFn> {
+ public:
+  static variable_list forward(AutogradContext* ctx, const Tensor& a, const Tensor& b) {
+    ctx->saved_data["t"] = dtypes_of({a, b});
+    return {add(a, b)};
+  }
+  static Tensor add(const Tensor& a, const Tensor& b) {
+    const bool bf = b.scalar_type() == at::kBFloat16;
+    if (!bf || (a.scalar_type() != at::kBFloat16 && a.scalar_type() != at::kFloat)) return a.detach() + b.detach().to(a.scalar_type());
+    const Tensor ac = a.detach().contiguous(), bc = b.detach().contiguous();
+    Tensor out = at::empty_like(ac);
+    void* st = at::cuda::getCurrentCUDAStream().stream();
+    if (ac.scalar_type() == at::kFloat)
+      LMOE(lmoe_add_f32_bf16, ac.data_ptr<float>(), bc.data_ptr(), out.data_ptr<float>(), out.numel(), st);
+    else
+      LMOE(lmoe_add_bf16, ac.data_ptr(), bc.data_ptr(), out.data_ptr(), out.numel(), st);
+    return out;
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    const auto t = ctx->saved_data["t"].toIntVector();
+    auto cast = [&](int k) {
+      const auto d = static_cast<at::ScalarType>(t[k]);
+      if (!grads[0].defined() || grads[0].scalar_type() == d) return grads[0];
+      if (d != at::kBFloat16 || grads[0].scalar_type() != at::kFloat) return grads[0].to(d);
+      const c10::cuda::CUDAGuard guard(grads[0].device());
+      return grad_rows(grads[0], grads[0].view({-1, grads[0].size(-1)})).view(grads[0].sizes());
+    };
+    return {cast(0), cast(1)};
+  }
+};
+
 bool any_grad(std::initializer_list<const Tensor*> ts) {
   if (!at::GradMode::is_enabled()) return false;
   for (const Tensor* t : ts)
@@ -867,6 +950,16 @@ std::vector<Tensor> moe(const Tensor& x, const Tensor& wg, const Tensor& wgus, c
   }
   LatentOut r = moe_forward(d, o, f32_bias(bias), static_cast<float>(z_coef), false, forced_sel);
   return {as_param(r.y.view(x.sizes()), x.scalar_type()), r.z_loss, r.sel, r.counts};
+}
+
+std::vector<Tensor> norm_and_pass(const Tensor& x, const Tensor& weight, double eps, bool bf16_out) {
+  require_cuda(x, "fused norm");
+  const c10::cuda::CUDAGuard guard(x.device());
+  return NormFn::apply(x, weight, eps, bf16_out);
+}
+Tensor residual_add(const Tensor& a, const Tensor& b) {
+  const c10::cuda::CUDAGuard guard(a.device());
+  return any_grad({&a, &b}) ? AddFn::apply(a, b)[0] : AddFn::add(a, b);
 }
 
 py::dict dict_of(const Views& v) {
@@ -937,4 +1030,6 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     return LatentLayout(Sizes(T, D, L, E, K, F, Fs), false, false).bytes;
   });
   m.def("bias_update", &bias_update);
+  m.def("norm_and_pass", &norm_and_pass);
+  m.def("residual_add", &residual_add);
 }
