@@ -59,6 +59,15 @@ struct Chunk {
       nrm_unpack(v[0], f);
     }
   }
+  // The row as the norm sees it: in bf16, whatever the stream's type.  The router behind the norm decides by score order, so
+  // an fp32 stream that was not rounded here would select other experts than the same stream handed over in bf16.
+  __device__ __forceinline__ void get_rounded(float (&f)[8]) const {
+    get(f);
+    if (F32) {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) f[j] = __bfloat162float(__float2bfloat16_rn(f[j]));
+    }
+  }
 };
 template <bool F32>
 __device__ __forceinline__ void store_chunk(void* base, long long chunk, const float (&f)[8]) {
@@ -103,7 +112,7 @@ rmsnorm_fwd_kernel(const void* __restrict__ x, const void* __restrict__ w, bool 
     for (int i = 0; i < CH; ++i)
       if (lane + 32 * i < vec_per_row) {
         float f[8];
-        row[i].get(f);
+        row[i].get_rounded(f);
 #pragma unroll
         for (int j = 0; j < 8; ++j) ss = fmaf(f[j], f[j], ss);
       }
@@ -115,7 +124,7 @@ rmsnorm_fwd_kernel(const void* __restrict__ x, const void* __restrict__ w, bool 
       const int v = lane + 32 * i;
       if (v < vec_per_row) {
         float f[8], ww[8], o[8];
-        row[i].get(f);
+        row[i].get_rounded(f);
         load_weight(w, w32, v, ww);
 #pragma unroll
         for (int j = 0; j < 8; ++j) o[j] = ww[j] * (f[j] * r);
@@ -192,7 +201,7 @@ rmsnorm_bwd_kernel(const void* __restrict__ x, const void* __restrict__ w, bool 
       const int v = lane + 32 * i;
       if (v < vec_per_row) {
         float fx[8], fg[8], ww[8];
-        xr[i].get(fx);
+        xr[i].get_rounded(fx);
         gr[i].get(fg);
         load_weight(w, w32, v, ww);
 #pragma unroll
@@ -209,7 +218,7 @@ rmsnorm_bwd_kernel(const void* __restrict__ x, const void* __restrict__ w, bool 
       const int v = lane + 32 * i;
       if (v < vec_per_row) {
         float fx[8], fg[8], ww[8], o[8];
-        xr[i].get(fx);
+        xr[i].get_rounded(fx);
         gr[i].get(fg);
         load_weight(w, w32, v, ww);
 #pragma unroll

@@ -177,3 +177,35 @@ def test_fp32_residual_stream_is_not_rounded_to_bf16():
     assert (out.detach().cpu() - ref.detach()).abs().max().item() <= 2e-5          # bf16 rounding of x would be ~2e-2
     assert (xg.grad.cpu() - xr.grad).abs().max().item() <= 2e-5
     assert (x.to(torch.bfloat16).float() - x).abs().max().item() > 1e-3            # (what a bf16 residual would lose)
+
+
+def _mixed_block():
+    from swamla_b200.block import NormedResidualFFN
+    from swamla_b200.layer import create_moe_layer
+    w = inputs.WORKLOADS["tiny"]
+    torch.manual_seed(11)
+    with torch.device("cuda:0"):
+        block = NormedResidualFFN(create_moe_layer(w.config()), w.D)
+        for name, p in block.named_parameters():
+            if "experts." in name.replace("shared_experts", "shared"):
+                p.data = p.data.to(torch.bfloat16)
+        x = torch.randn(3, 171, w.D) * 3.0
+    return block, x
+
+
+def test_fp32_stream_selects_the_experts_of_its_bf16_rounding():
+    """The norm reads an fp32 stream as bf16: its output, and so every routing decision behind it, is that of the rounded
+    stream bit for bit (a score gap below the rounding would otherwise go to another expert)."""
+    block, x = _mixed_block()
+    block.train()
+    block(x)
+    sel = block.ffn.router._last_selected_experts.clone()
+    block(x.to(torch.bfloat16).float())
+    assert torch.equal(sel, block.ffn.router._last_selected_experts)
+    xn = [_host_norm(block, t) for t in (x, x.to(torch.bfloat16))]
+    assert torch.equal(xn[0], xn[1])
+
+
+def _host_norm(block, x):
+    from swamla_b200.functional import _host
+    return _host().norm_and_pass(x, block.ffn_norm.weight, block.ffn_norm.eps, True)[0]
