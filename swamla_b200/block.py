@@ -5,8 +5,8 @@ the RMSNorm (``models/normalization.py:25-39``) and the residual add as fused ro
 feed-forward module (here: ``LatentMoELayer`` / ``MoELayer``).  Forward: one kernel for the norm (one read of x, one
 write), the layer, one kernel for the add.  Backward: ONE kernel for the adjoint of the norm and the residual branch
 (``dx = norm_bwd(d_xn) + dy``), plus a deterministic two-stage sum for the weight gradient.  The residual stream keeps the
-input's dtype: under the reference's autocast training it is fp32 (train.py:1195, normalization.py:25-39) and is never rounded
-to bf16.  The autograd nodes are in ``csrc/torch_host.cpp``.  No CPU fallback.
+input's dtype: under the reference's autocast training it is fp32 (train.py:1195, normalization.py:25-39) and the residual
+branch is never rounded to bf16 (the norm's input is, as it is read).  The autograd nodes are in ``csrc/torch_host.cpp``.  No CPU fallback.
 """
 from __future__ import annotations
 
@@ -46,20 +46,25 @@ class NormedResidualFFN(nn.Module):
         self.ffn = ffn
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
+        _B, _S, _D = x.shape
+        norm, ffn = self.ffn_norm, self.ffn
         if torch.compiler.is_compiling():
-            return self._forward_opaque(x)
-        return self._forward(x)
-
-    def _forward(self, x):
-        ffn, norm = self._modules["ffn"], self._modules["ffn_norm"]
-        # this package's layers compute in bf16 whatever they are given: hand them bf16 and take bf16 back, instead of a
+            xn, x_pass = _norm_opaque(x, norm.weight, norm.eps)
+            return _add_opaque(x_pass, ffn(xn))
+        # this package's own layers compute in bf16 whatever they are given: hand them bf16 and take bf16 back, instead of a
         # widened copy each way (an active dropout keeps the stream's precision)
-        narrow = isinstance(ffn, (LatentMoELayer, MoELayer)) and not (ffn.training and ffn.dropout.p > 0.0)
+        narrow = type(ffn) in (LatentMoELayer, MoELayer) and not (ffn.training and ffn.dropout.p > 0.0)
         host = _host()
-        xn, x_pass = host.norm_and_pass(x, norm._parameters["weight"], norm.eps, narrow)
+        xn, x_pass = host.norm_and_pass(x, norm.weight, norm.eps, narrow)
         return host.residual_add(x_pass, ffn(xn))
 
-    # opaque to torch.compile (calls into the kernel library)
-    @torch.compiler.disable
-    def _forward_opaque(self, x):
-        return self._forward(x)
+
+# opaque to torch.compile (calls into the kernel library); the feed-forward module between them is compiled
+@torch.compiler.disable
+def _norm_opaque(x, weight, eps):
+    return _NormAndPass.apply(x, weight, eps)
+
+
+@torch.compiler.disable
+def _add_opaque(a, b):
+    return _host().residual_add(a, b)

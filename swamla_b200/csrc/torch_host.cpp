@@ -17,8 +17,10 @@
 #include <cuda_runtime.h>
 #include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/custom_function.h>
+#include <torch/csrc/jit/frontend/tracer.h>
 #include <torch/extension.h>
 
+#include <cstring>
 #include <map>
 #include <mutex>
 #include <utility>
@@ -62,7 +64,11 @@ const char* const kKindName[kKinds] = {"LatentMoE forward", "LatentMoE backward"
 int32_t* status_words() {
   static int32_t* words = [] {
     void* p = nullptr;
-    if (cudaHostAlloc(&p, 256, cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess)
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;  // the first call may be one that is being captured
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    const cudaError_t e = cudaHostAlloc(&p, 256, cudaHostAllocMapped | cudaHostAllocPortable);
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    if (e != cudaSuccess)
       throw LmoeFailure("no pinned memory for the device status words");
     std::memset(p, 0, 256);
     return static_cast<int32_t*>(p);
@@ -105,11 +111,27 @@ class Fork {
     }
     side_ = &s;
   }
+  // A stage that fails between to_side and to_main: what the side stream has been given still uses the call's buffers.
+  ~Fork() {
+    if (!open_) return;
+    std::lock_guard<std::mutex> lock(g_side_mutex);
+    if (cudaEventRecord(side_->ev, side_->stream) == cudaSuccess) cudaStreamWaitEvent(main_, side_->ev, 0);
+  }
+  Fork(const Fork&) = delete;
+  Fork& operator=(const Fork&) = delete;
   cudaStream_t side() const { return side_->stream; }
-  void to_side() { order(main_, side_->stream); }
-  void to_main() { order(side_->stream, main_); }
+  void to_side() {
+    open_ = true;
+    order(main_, side_->stream);
+  }
+  // more: the side stream goes on with work that a later to_main joins
+  void to_main(bool more = false) {
+    order(side_->stream, main_);
+    open_ = more;
+  }
 
  private:
+  bool open_ = false;
   void order(cudaStream_t first, cudaStream_t then) {
     std::lock_guard<std::mutex> lock(g_side_mutex);  // record and wait belong together: the event is shared
     C10_CUDA_CHECK(cudaEventRecord(side_->ev, first));
@@ -198,6 +220,10 @@ struct Caster {
     if (count > 0) LMOE(lmoe_cast_many_f32_to_bf16, count, src, dst, n, st);
   }
 };
+
+// t in another shape, not recorded as a view: an output of a custom function that autograd takes for a view refuses to be
+// changed in place (y += ..., an in-place dropout).
+Tensor shaped(const Tensor& t, at::IntArrayRef sizes) { return at::_unsafe_view(t, sizes); }
 
 // A gradient in its parameter's dtype.
 Tensor as_param(const Tensor& g, at::ScalarType d) { return g.scalar_type() == d ? g : g.to(d); }
@@ -358,7 +384,7 @@ LatentOut latent_forward(const Sizes& d, const LatentOps& o, const Tensor& bias,
     LMOE(lmoe_xproj_fwd, &d.s, o.x.data_ptr(), o.wg.data_ptr(), nullptr, logits, nullptr, status, st);
     LMOE(lmoe_xproj_fwd, &d.s, o.x.data_ptr(), nullptr, o.wdn.data_ptr(), nullptr, x_latent, status, side);
     LMOE(lmoe_topk_hist_fwd, &d.s, logits, bias.data_ptr<float>(), sel, weights, lse, tv + t_ws, ws_bytes, st);
-    if (forked) fork->to_main();
+    if (forked) fork->to_main(true);
     if (fp8) {  // the weights beside the latents: on the side stream, or in the same launches
       const int n = forked ? 1 : 3;
       LMOE(lmoe_fp8_amax, n, q, st);
@@ -370,7 +396,7 @@ LatentOut latent_forward(const Sizes& d, const LatentOps& o, const Tensor& bias,
     }
     LMOE(lmoe_route_gather_fwd, &d.s, sel, tv + t_ws, ws_bytes, z_coef, r.z_loss.data_ptr<float>(), &route,
          x_sorted ? gather_src : nullptr, gather_bytes, x_sorted, st);
-    if (fp8 && forked) fork->to_main();
+    if (fp8 && forked) fork->to_main(true);
     LMOE(lmoe_shared_gateup_fwd, &d.s, o.x.data_ptr(), o.wgus.data_ptr(), h1_s, act_cat, status, side);
   }
 
@@ -701,7 +727,9 @@ std::vector<Tensor> few_forward(const Sizes& d, const Tensor& x2d, const Tensor&
 // ---------------------------------------------------------------- autograd
 
 
+// torch.jit.trace would bake the results of a native call in as constants.
 void require_cuda(const Tensor& x, const char* what) {
+  if (torch::jit::tracer::isTracing()) throw LmoeFailure(std::string("the ") + what + " path cannot be recorded by torch.jit.trace");
   if (!x.is_cuda()) throw LmoeFailure(std::string("the ") + what + " path runs on a CUDA device only (no CPU fallback)");
 }
 
@@ -752,8 +780,7 @@ class LatentFn : public torch::autograd::Function<LatentFn> {
     ctx->saved_data["s"] = x.sizes().vec();
     ctx->saved_data["z"] = z_coef;
     ctx->mark_non_differentiable({r.sel, r.counts});
-    Tensor y = r.y.view(x.sizes());
-    return {as_param(y, x.scalar_type()), r.z_loss, r.sel, r.counts};
+    return {as_param(shaped(r.y, x.sizes()), x.scalar_type()), r.z_loss, r.sel, r.counts};
   }
 
   static variable_list backward(AutogradContext* ctx, variable_list grads) {
@@ -797,7 +824,7 @@ class MoeFn : public torch::autograd::Function<MoeFn> {
     ctx->saved_data["s"] = x.sizes().vec();
     ctx->saved_data["z"] = z_coef;
     ctx->mark_non_differentiable({r.sel, r.counts});
-    return {as_param(r.y.view(x.sizes()), x.scalar_type()), r.z_loss, r.sel, r.counts};
+    return {as_param(shaped(r.y, x.sizes()), x.scalar_type()), r.z_loss, r.sel, r.counts};
   }
 
   static variable_list backward(AutogradContext* ctx, variable_list grads) {
@@ -825,10 +852,16 @@ class MoeFn : public torch::autograd::Function<MoeFn> {
 
 // ---------------------------------------------------------------- norm and residual either side of a feed-forward layer
 int lmoe_type(const Tensor& t) { return t.scalar_type() == at::kFloat ? LMOE_F32 : LMOE_BF16; }
+bool aligned(const Tensor& t) { return reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0; }
 // bf16 and fp32 pass as they are; anything else in fp32
 Tensor rows_of(const Tensor& t) {
   const Tensor d = t.detach();
   return (d.scalar_type() == at::kFloat || d.scalar_type() == at::kBFloat16 ? d : d.to(at::kFloat)).contiguous();
+}
+// the norm's weight: a slice of a flat parameter need not start at the 16 bytes that the kernels read at once
+Tensor weight_of(const Tensor& t) {
+  const Tensor w = rows_of(t);
+  return aligned(w) ? w : w.clone();
 }
 
 // (xn, x_pass) = (rmsnorm(x) * weight, x).  x_pass is x itself, handed on to the residual add, so that the backward sees the
@@ -836,7 +869,8 @@ Tensor rows_of(const Tensor& t) {
 class NormFn : public torch::autograd::Function<NormFn> {
  public:
   static variable_list forward(AutogradContext* ctx, const Tensor& x, const Tensor& weight, double eps, bool bf16_out) {
-    const Tensor xr = rows_of(x), w = rows_of(weight);
+    const Tensor xr = rows_of(x), w = weight_of(weight);
+    TORCH_CHECK(x.dim() > 0 && weight.numel() == x.size(-1), "the norm's weight has another width than its input");
     const int64_t D = x.size(-1), T = xr.numel() / D;
     const bool wide = !bf16_out && xr.scalar_type() == at::kFloat;
     Tensor xn = at::empty(x.sizes(), xr.options().dtype(wide ? at::kFloat : at::kBFloat16));
@@ -885,6 +919,7 @@ class AddFn : public torch::autograd::Function<AddFn> {
     const bool bf = b.scalar_type() == at::kBFloat16;
     if (!bf || (a.scalar_type() != at::kBFloat16 && a.scalar_type() != at::kFloat)) return a.detach() + b.detach().to(a.scalar_type());
     const Tensor ac = a.detach().contiguous(), bc = b.detach().contiguous();
+    if (ac.scalar_type() == at::kFloat && !(aligned(ac) && aligned(bc))) return ac + bc;
     Tensor out = at::empty_like(ac);
     void* st = at::cuda::getCurrentCUDAStream().stream();
     if (ac.scalar_type() == at::kFloat)
@@ -900,16 +935,21 @@ class AddFn : public torch::autograd::Function<AddFn> {
       if (!grads[0].defined() || grads[0].scalar_type() == d) return grads[0];
       if (d != at::kBFloat16 || grads[0].scalar_type() != at::kFloat) return grads[0].to(d);
       const c10::cuda::CUDAGuard guard(grads[0].device());
-      return grad_rows(grads[0], grads[0].view({-1, grads[0].size(-1)})).view(grads[0].sizes());
+      Caster narrow;
+      Tensor g = narrow(grads[0]);
+      narrow.run(at::cuda::getCurrentCUDAStream().stream());
+      return g;
     };
     return {cast(0), cast(1)};
   }
 };
 
+// Whether the call needs an autograd node.  A forward-mode tangent counts whatever the grad mode is: the node refuses it
+// (no jvp), the direct path would drop it without a word.
 bool any_grad(std::initializer_list<const Tensor*> ts) {
-  if (!at::GradMode::is_enabled()) return false;
+  const bool grad = at::GradMode::is_enabled();
   for (const Tensor* t : ts)
-    if (t->requires_grad()) return true;
+    if ((grad && t->requires_grad()) || t->_fw_grad(/*level=*/0).defined()) return true;
   return false;
 }
 
@@ -957,8 +997,11 @@ std::vector<Tensor> norm_and_pass(const Tensor& x, const Tensor& weight, double 
   const c10::cuda::CUDAGuard guard(x.device());
   return NormFn::apply(x, weight, eps, bf16_out);
 }
-Tensor residual_add(const Tensor& a, const Tensor& b) {
+Tensor residual_add(const Tensor& a, const Tensor& b_in) {
   const c10::cuda::CUDAGuard guard(a.device());
+  // a feed-forward module may return its rows flattened; one whose result only broadcasts is added by PyTorch
+  const Tensor b = b_in.sizes() != a.sizes() && b_in.numel() == a.numel() ? b_in.reshape(a.sizes()) : b_in;
+  if (b.sizes() != a.sizes()) return a + b.to(a.scalar_type());
   return any_grad({&a, &b}) ? AddFn::apply(a, b)[0] : AddFn::add(a, b);
 }
 

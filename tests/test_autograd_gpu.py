@@ -1,0 +1,90 @@
+"""What a module's caller may do with its inputs and outputs under autograd: nothing that a plain module allows may break or,
+worse, be answered wrongly without a word."""
+import pytest
+import torch
+import torch.autograd.forward_ad as fwd_ad
+
+from oracle import inputs
+
+pytestmark = pytest.mark.gpu
+
+
+def _module(kind, dtype=torch.bfloat16):
+    from swamla_b200.block import NormedResidualFFN
+    from swamla_b200.layer import create_moe_layer
+    w = inputs.WORKLOADS["tiny_moe" if kind == "moe" else "tiny"]
+    torch.manual_seed(3)
+    with torch.device("cuda:0"):
+        m = create_moe_layer(w.config()).to(torch.bfloat16)
+        if kind == "block":
+            m = NormedResidualFFN(m, w.D)
+        x = torch.randn(2, 70, w.D, dtype=dtype)
+    return m, x
+
+
+KINDS = ["latent", "moe", "block"]
+
+
+@pytest.mark.parametrize("kind", KINDS)
+def test_output_may_be_changed_in_place(kind):
+    m, x = _module(kind)
+    xg = x.clone().requires_grad_(True)
+    m.train()(xg).sum().backward()
+    want, xg.grad = 3.0 * xg.grad, None
+    y = m(xg)
+    y.mul_(3.0)
+    y.sum().backward()
+    assert torch.allclose(xg.grad.float(), want.float(), rtol=2e-2, atol=2e-2 * want.float().abs().max().item())
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("kind", KINDS)
+def test_gradient_in_another_layout(kind, dtype):
+    m, x = _module(kind, dtype)
+    xg = x.clone().requires_grad_(True)
+    dy = torch.randn(70, 2, x.shape[-1], dtype=dtype, device=x.device)
+    m.train()(xg).backward(dy.transpose(0, 1).contiguous())
+    want, xg.grad = xg.grad, None
+    m(xg).transpose(0, 1).backward(dy)             # reaches the module with strides of the transpose
+    assert torch.equal(xg.grad, want)
+
+
+@pytest.mark.parametrize("grad", [True, False])
+@pytest.mark.parametrize("kind", KINDS)
+def test_forward_mode_is_refused(kind, grad):
+    m, x = _module(kind)
+    with fwd_ad.dual_level(), torch.set_grad_enabled(grad):
+        with pytest.raises((RuntimeError, NotImplementedError)):
+            m.eval()(fwd_ad.make_dual(x, torch.ones_like(x)))
+
+
+@pytest.mark.parametrize("kind", KINDS)
+def test_trace_is_refused(kind):
+    m, x = _module(kind)
+    with torch.no_grad(), pytest.raises(RuntimeError):
+        torch.jit.trace(m.eval(), (x,), check_trace=False)
+
+
+def test_block_takes_flattened_and_broadcast_branches():
+    from swamla_b200.block import NormedResidualFFN
+
+    class Branch(torch.nn.Module):
+        def __init__(self, f):
+            super().__init__()
+            self.f = f
+
+        def forward(self, t):
+            return self.f(t)
+
+    x = torch.randn(2, 5, 64, device="cuda:0")
+    flat = NormedResidualFFN(Branch(lambda t: t.flatten(0, 1).to(torch.bfloat16)), 64).cuda()
+    full = NormedResidualFFN(Branch(lambda t: t.to(torch.bfloat16)), 64).cuda()
+    one = NormedResidualFFN(Branch(lambda t: torch.ones(64, device=t.device)), 64).cuda()
+    for m in (flat, full):
+        xg = x.clone().requires_grad_(True)
+        y = m(xg)
+        y.sum().backward()
+        if m is flat:
+            want, want_grad = y.detach(), xg.grad
+    assert torch.equal(y, want) and torch.equal(xg.grad, want_grad)
+    assert torch.equal(one(x), x + 1.0)
