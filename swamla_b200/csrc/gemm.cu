@@ -370,6 +370,41 @@ static int launch_gemm_pair_grouped(const GemmCall& c) {
   return launch_pair_inst<false, false, EPI_BF16, GRP_M>(p, total, c.stream);
 }
 
+// Grouped-by-contraction GEMM (expert weight gradients) on CTA pairs: 256 x 256 tiles, half of the tile's B per CTA.
+// Bound by what an SM can pull in (one CTA per 128 x 256 tile: 48 KB per k-block, four stages; here 32 KB, six stages), so it
+// gains with the length of the contraction.  One CTA per tile -> pairs, us:
+//   128 experts, 6,144 rows each: 256 x 1,536 823 -> 658, 768 x 256 473 -> 416; 256 experts, 2,048 rows: 256 x 512 164 -> 142;
+//   32 experts, 384 rows: 1,024 x 2,048 57 -> 51; 128 experts, 96 rows: 256 x 512 14.7 -> 13.4
+// An output of a single pair tile per expert does not (256 x 256: 97.7 -> 99.8 with 256 experts, 18.4 -> 19.6 with 128 experts of
+// 384 rows): one CTA per tile then.  Rounding M up to 256 may cost an eighth over rounding it to 128 (M = 384 would load and
+// multiply a third for nothing).
+static bool pair_wgrad_applies(const GemmCall& c) {
+  const long long up256 = (c.M + 255) / 256 * 256, up128 = (c.M + 127) / 128 * 128;
+  return c.grp == GRP_K && c.esz == 2 && !c.a_rows && c.a_mn && c.b_mn && c.nseg == 1 && c.bn == 0 && c.epi == EPI_BF16 && c.groups > 0 &&
+         c.pad_offsets && pair_gemm_applies(c.M, c.N) && (c.M > 256 || c.N > 256) && 8 * up256 <= 9 * up128;
+}
+static int launch_gemm_pair_wgrad(const GemmCall& c) {
+  GemmParams p;
+  memset(&p, 0, sizeof(p));
+  if (!c.A[0] || !c.B[0]) return LMOE_ERR_ARG;
+  int rc = encode_2d(&p.tmA[0], c.A[0], c.M, c.padded_rows, c.lda[0], 64, 2);
+  if (rc) return rc;
+  rc = encode_2d(&p.tmB[0], c.B[0], c.N, c.padded_rows, c.ldb[0], 64, 2);
+  if (rc) return rc;
+  rc = encode_out(&p.tmC, c.C, false, c.N, c.M, c.groups, c.ldc, c.c_group_stride);
+  if (rc) return rc;
+  p.nseg = 1;
+  p.M = c.M;
+  p.N = c.N;
+  p.m_tiles = (c.M + 255) / 256;
+  p.n_tiles = (c.N + 255) / 256;
+  p.groups = c.groups;
+  p.split_k = 1;
+  p.pad_offsets = c.pad_offsets;
+  p.status = c.status;
+  return launch_pair_inst<true, true, EPI_BF16, GRP_K>(p, static_cast<long long>(p.m_tiles) * p.n_tiles * c.groups, c.stream);
+}
+
 int launch_gemm(const GemmCall& c) {
   // only a SwiGLU GEMM may leave out its main output (gate / up; see GemmParams::hidden_only)
   if (c.nseg < 1 || c.nseg > 3 || (!c.C && c.epi != EPI_SWIGLU) || c.M <= 0 || c.N <= 0) return LMOE_ERR_ARG;
@@ -388,6 +423,7 @@ int launch_gemm(const GemmCall& c) {
 
   const bool gather = c.a_rows != nullptr;
   if (pair_grouped_applies(c)) return launch_gemm_pair_grouped(c);
+  if (pair_wgrad_applies(c)) return launch_gemm_pair_wgrad(c);
   if (c.grp == GRP_NONE && esz == 2 && !gather && c.bn != 128 && pair_gemm_applies(c.M, swiglu ? 2 * c.N : c.N) &&
       (c.epi == EPI_BF16 || c.epi == EPI_F32 || (swiglu && !c.a_mn && !c.b_mn) || (swiglu_bwd && !c.a_mn && c.b_mn && c.nseg == 1)))
     return launch_gemm_pair(c);

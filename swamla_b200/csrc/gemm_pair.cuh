@@ -42,10 +42,13 @@ struct PairSmem {
 // consecutive 128-row tiles of the SAME expert (tiles 2j, 2j+1 of its run, from pad_offsets) and share that expert's
 // slice of the stacked B tensor.  An expert with an odd number of tiles ends with a pair whose second CTA recomputes
 // the first tile and stores nothing.
+// GRP == GRP_K (grouped over the contraction, both operands MN-major): output plane e is A[rows_e, :]^T * B[rows_e, :] over
+// expert e's padded rows (pad_offsets); one 256 x 256 tile of one expert per pair.  An expert without rows writes zeros.
 template <bool A_MN, bool B_MN, int EPI, int GRP = GRP_NONE>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1)
 gemm_pair_kernel(const __grid_constant__ GemmParams p) {
-  static_assert(GRP == GRP_NONE || (GRP == GRP_M && !A_MN), "grouped form: rows of a K-major A");
+  static_assert(GRP == GRP_NONE || (GRP == GRP_M && !A_MN) || (GRP == GRP_K && A_MN && B_MN && EPI == EPI_BF16),
+                "grouped forms: rows of a K-major A, or a contraction over rows");
   using S = PairSmem<EPI>;
   constexpr int BN = 256;
   constexpr int STAGES = S::kStages;
@@ -140,16 +143,18 @@ gemm_pair_kernel(const __grid_constant__ GemmParams p) {
   auto pairs_before = [&](int e) { return ((etab[e] & 0x7fffff) - (etab[0] & 0x7fffff) + (etab[e] >> 23)) >> 1; };
   // m_tiles counts 256-row tiles (dense) or is the layout's capacity in 128-row tiles (grouped: pairs come from etab)
   const int tiles_mn = (GRP == GRP_M ? pairs_before(p.groups) : p.m_tiles) * p.n_tiles;
-  const int total_tiles = tiles_mn * p.split_k;
+  const int total_tiles = tiles_mn * (GRP == GRP_K ? p.groups : p.split_k);
 
   struct Tile {
     int m0, nt, plane, kb, ke;
     int grp;   // GRP_M: expert of the pair
+    int krow0; // GRP_K: first padded row of the expert
     int live;  // GRP_M: 0 for the tile-less second CTA of an odd run (loads the first tile, stores nothing)
   };
   auto decode = [&](int id) {
     Tile t;
     t.grp = 0;
+    t.krow0 = 0;
     t.live = 1;
     if (GRP == GRP_M) {
       const int pid = id / p.n_tiles;
@@ -177,7 +182,11 @@ gemm_pair_kernel(const __grid_constant__ GemmParams p) {
     t.plane = 0;
     t.kb = 0;
     t.ke = p.seg_kiters[0];
-    if (p.split_k > 1) {
+    if (GRP == GRP_K) {
+      t.plane = outer;
+      t.krow0 = p.pad_offsets[outer];
+      t.ke = (p.pad_offsets[outer + 1] - t.krow0) / BK_E;
+    } else if (p.split_k > 1) {
       const int per = (p.seg_kiters[0] + p.split_k - 1) / p.split_k;
       t.kb = min(outer * per, p.seg_kiters[0]);
       t.ke = min(t.kb + per, p.seg_kiters[0]);
@@ -217,7 +226,7 @@ gemm_pair_kernel(const __grid_constant__ GemmParams p) {
             uint8_t* sb = sa + S::kABytes;
             if (rank == 0) mbar_expect_tx(&bar_full[stage], 2 * S::kStageBytes);
             const uint32_t full0 = mapa_shared(smem_u32(&bar_full[stage]), 0);
-            const int kcoord = kit * BK_E;
+            const int kcoord = t.krow0 + kit * BK_E;
             if (!A_MN) {
               tma_load_2d_pair(sa, &p.tmA[s], full0, kcoord, t.m0);
             } else {

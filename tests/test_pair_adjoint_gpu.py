@@ -77,3 +77,29 @@ def test_grouped_long_contraction(rows, b_mn):
             err = (got[lo:hi].float() - ref).abs()
             assert (err <= 2.0 ** -8 * ref.abs() + 2.0 ** -16 * ref.abs().max()).all()   # bf16 output rounding, fp32 sums
     assert (got[int(off[-1]):] == 0).all()                           # nothing beyond the tiles in use
+
+
+# whole tiles, several tiles, ragged edges (the second CTA's rows partly outside), an extent that stays with one CTA per tile
+@pytest.mark.parametrize("M,N", [(256, 256), (1024, 264), (504, 520), (256, 1536), (384, 256)])
+@pytest.mark.parametrize("rows", [[128, 0, 640, 64], [0, 0, 0, 129], [1, 256, 2000, 0]])   # empty experts, one k-block pair, long
+def test_grouped_weight_gradient(M, N, rows):
+    from swamla_b200 import _cabi
+    dev, E = "cuda:0", 4
+    pads = [(r + 127) // 128 * 128 for r in rows]
+    off = [sum(pads[:i]) for i in range(E + 1)]
+    P = off[-1] + 128                                                # one unused tile of capacity, never read
+    g = torch.Generator(dev).manual_seed(M + N)
+    a, b = (torch.randn(P, n, device=dev, generator=g).to(torch.bfloat16) for n in (M, N))
+    a[off[-1]:] = float("nan")
+    out = torch.full((E + 1, M, N), 3.0, dtype=torch.bfloat16, device=dev)
+    offd = torch.tensor(off, dtype=torch.int32, device=dev)
+    status = torch.zeros(1, dtype=torch.int32, device=dev)
+    _cabi.call("lmoe_grouped_wgrad_bf16", P, E, M, N, a.data_ptr(), b.data_ptr(), offd.data_ptr(), out.data_ptr(), status.data_ptr(),
+               torch.cuda.current_stream().cuda_stream)
+    torch.cuda.synchronize()
+    assert status.item() == 0
+    for e in range(E):
+        ref = a[off[e]:off[e + 1]].double().t() @ b[off[e]:off[e + 1]].double()
+        err = (out[e].double() - ref).abs()
+        assert (err <= 2.0 ** -8 * ref.abs() + 2.0 ** -16 * max(1.0, ref.abs().max().item())).all()   # bf16 rounding, fp32 sums
+    assert (out[E] == 3.0).all()                                     # nothing behind the last expert's plane
