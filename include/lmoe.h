@@ -241,7 +241,8 @@ int lmoe_swiglu_bwd(int64_t rows, int H, const void* h1, const void* d_hidden, v
                     const int32_t* n_tiles_dev, void* stream);
 /* Routed dgrads: d_hidden = d_y_sorted * w_down[e]^T, d_h1 = swiglu'(h1, d_hidden),
  * d_x_sorted = d_h1 * w_gate_up[e]^T.  All in the padded layout.  d_hidden may be NULL: the SwiGLU adjoint then
- * runs in the epilogue of the first GEMM and d_hidden is never written (also for lmoe_grouped_bwd_dgrad). */
+ * runs in the epilogue of the first GEMM, on the hardware tanh unit (sigmoid to 2^-12 absolute), and d_hidden is never
+ * written (also for lmoe_grouped_bwd_dgrad). */
 int lmoe_experts_bwd_dgrad(const lmoe_shape* s, const void* d_y_sorted, const void* h1, const void* w_gate_up,
                            const void* w_down, const lmoe_route* r, void* d_hidden, void* d_h1, void* d_x_sorted,
                            int32_t* status, void* stream);
@@ -323,9 +324,14 @@ int lmoe_gemm_swiglu_bf16(int M, int H, int K, const void* A, int64_t lda, const
 
 /* Backward of the non-latent layer's dense parts (autograd of models/moe.py:351-358); s->L is not used.
  * lmoe_moe_shared_bwd: d_h1_s = swiglu'(h1_s, dy * Wd_s) -> dgrad_cat[T, 2Fs+E][:, :2Fs] (the adjoint runs in the GEMM's
- * epilogue), d_w_down_s[D, Fs] = dy^T * hidden_s.  lmoe_moe_xside_bwd: dx_dense = [d_h1_s | d_logits] * [Wgu_s ; Wg] and the two
+ * epilogue and gives lmoe_swiglu_bwd's bits), d_w_down_s[D, Fs] = dy^T * hidden_s.  lmoe_moe_xside_bwd: dx_dense = [d_h1_s | d_logits] * [Wgu_s ; Wg] and the two
  * weight gradients that contract with x.  grad_type LMOE_F32 / LMOE_BF16. */
 size_t lmoe_moe_wgrad_workspace_bytes(const lmoe_shape* s);
+/* lmoe_grouped_bwd_dgrad for the experts of the non-latent layer: no d_hidden buffer, and d_h1 has the bits that
+ * lmoe_swiglu_bwd gives for the bf16 d_hidden (lmoe_grouped_bwd_dgrad without a buffer uses a coarser sigmoid). */
+int lmoe_moe_experts_bwd_dgrad(int64_t P, int E, int L, int F, const void* d_y_sorted, const void* h1, const void* w_gate_up,
+                               const void* w_down, const int32_t* tile_expert, const int32_t* n_tiles,
+                               const int32_t* pad_offsets, void* d_h1, void* d_x_sorted, int32_t* status, void* stream);
 int lmoe_moe_shared_bwd(const lmoe_shape* s, const void* dy, const void* w_down_s, const void* h1_s, const void* hidden_s,
                         void* dgrad_cat, void* d_w_down_s, int grad_type, void* workspace, size_t workspace_bytes,
                         int32_t* status, void* stream);
@@ -460,8 +466,8 @@ int lmoe_grouped_gateup_fp8(int64_t P, int E, int L, int F, const void* xq, cons
 int lmoe_grouped_gateup_fp8_amax(int64_t P, int E, int L, int F, const void* xq, const void* wq, const float* deq_x,
                                  const float* deq_w, const int32_t* tile_expert, const int32_t* n_tiles, void* h1, void* hidden,
                                  float* amax_hidden, int32_t* status, void* stream);
-/* Routed d_hidden with the SwiGLU adjoint in the epilogue: dyq[P,L], wdq[E,F,L] e4m3, h1[P,2F] -> d_h1[P,2F] bf16, and
- * amax_d_h1[0] = max(amax_d_h1[0], max |d_h1|) (may be NULL). */
+/* Routed d_hidden with the SwiGLU adjoint in the epilogue: dyq[P,L], wdq[E,F,L] e4m3, h1[P,2F] -> d_h1[P,2F] bf16 with the
+ * bits of lmoe_grouped_rows_fp8 + lmoe_swiglu_bwd, and amax_d_h1[0] = max(amax_d_h1[0], max |d_h1|) (may be NULL). */
 int lmoe_grouped_swiglu_bwd_fp8(int64_t P, int E, int L, int F, const void* dyq, const void* wdq, const float* deq_dy,
                                 const float* deq_wd, const int32_t* tile_expert, const int32_t* n_tiles, const void* h1,
                                 void* d_h1, float* amax_d_h1, int32_t* status, void* stream);

@@ -118,6 +118,7 @@ SIGNATURES = {
     "lmoe_rmsnorm_bwd_typed": (c_int, [P, c_int, P, c_int, P, P, c_int, P, c_int64, c_int, P, P, c_int, P, c_size_t, P]),
     "lmoe_add_f32_bf16": (c_int, [P, P, P, c_int64, P]),
     "lmoe_moe_wgrad_workspace_bytes": (c_size_t, [SP]),
+    "lmoe_moe_experts_bwd_dgrad": (c_int, [c_int64, c_int, c_int, c_int, P, P, P, P, P, P, P, P, P, P, P]),
     "lmoe_moe_shared_bwd": (c_int, [SP, P, P, P, P, P, P, c_int, P, c_size_t, P, P]),
     "lmoe_moe_xside_bwd": (c_int, [SP, P, P, P, P, P, P, P, c_int, P, c_size_t, P, P]),
     "lmoe_router_bias_update_counted": (c_int, [c_int, P, c_float, P, P, P, P]),

@@ -287,6 +287,7 @@ static int launch_gemm_pair(const GemmCall& c) {
   p.split_k = split;
   p.half = c.N;
   p.hidden_only = c.C ? 0 : 1;
+  p.exact_sigmoid = c.exact_sigmoid ? 1 : 0;
   p.status = c.status;
   const long long total = static_cast<long long>(m_tiles) * n_tiles * split;
   const int key = c.a_mn | (c.b_mn << 1) | (c.epi << 2);
@@ -538,6 +539,7 @@ int launch_gemm(const GemmCall& c) {
   p.split_k = split;
   p.half = c.N;
   p.hidden_only = c.C ? 0 : 1;
+  p.exact_sigmoid = c.exact_sigmoid ? 1 : 0;
   p.tile_expert = c.tile_expert;
   p.n_m_tiles = c.n_m_tiles;
   p.b_group_rows = c.b_group_rows;

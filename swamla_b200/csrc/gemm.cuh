@@ -70,6 +70,7 @@ struct alignas(64) GemmParams {
   const float* deq_a;      // e4m3: per-tensor de-scale factors (amax / 448) of A and B, device scalars
   const float* deq_b;
   float* amax;             // e4m3 operands, SwiGLU epilogues: max |hidden| / max |d_h1| (bf16-rounded), device scalar or NULL
+  int exact_sigmoid;       // EPI_SWIGLU_BWD, bf16 operands: sigmoid_exact instead of sigmoid_fast (e4m3 operands: always)
   const void* aux;         // EPI_SWIGLU_BWD: h1 [rows, 2*N] bf16 (gate | up), row stride ld_aux elements
   long long ld_aux;
   CUtensorMap tmAux;       // EPI_SWIGLU_BWD: the same tensor as 128-row boxes of 64 columns (128-byte swizzle), staged by TMA
@@ -115,7 +116,9 @@ struct GemmSmem {
 
 // sigmoid(g) = 0.5 + 0.5 * tanh(g / 2) on the hardware tanh unit: ONE special-function instruction per value
 // (exp2 + reciprocal take two, and a full-precision division many more; the SwiGLU epilogues are bound by instruction
-// issue, not by memory).  tanh.approx.f32 has a relative error of 2^-11, an eighth of a bf16 ulp.
+// issue, not by memory).  tanh.approx.f32 has a relative error of 2^-11: an ABSOLUTE error of at most 2^-12 of the sigmoid.
+// That is an eighth of a bf16 ulp of it for g >= 0; for negative g the sum cancels and the relative error grows with
+// 1 / sigmoid(g): up to 1.4 % at g = -4, 10 % at g = -6.
 __device__ __forceinline__ float sigmoid_fast(float g) {
   float t;
   asm("tanh.approx.f32 %0, %1;" : "=f"(t) : "f"(0.5f * g));
@@ -123,6 +126,18 @@ __device__ __forceinline__ float sigmoid_fast(float g) {
 }
 // silu(g) = g * sigmoid(g)
 __device__ __forceinline__ float silu_f(float g) { return g * sigmoid_fast(g); }
+// Accurate to a few fp32 ulps at every g: 1 / (1 + __expf(-g)) with the bits of lmoe_swiglu_bwd, for the adjoints that are
+// held to them.  The quotient is the hardware reciprocal and one Newton step with an fma residual (Markstein, IBM J. Res. Dev.
+// 34, 1990): equal to 1.0f / x for every float of [1, 2^126) (all 1.06e9 compared).  Above, at gates below -87, the quotient is
+// subnormal and stays the hardware's; the step would turn the 0 of x = inf into a NaN.  The division itself has a branch per
+// value: with it the adjoint of the largest e4m3 training step (131,072 tokens) cost 0.42 ms of 7.1.
+__device__ __forceinline__ float sigmoid_exact(float g) {
+  const float x = 1.0f + __expf(-g);
+  float r;
+  asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(x));
+  const float n = fmaf(r, fmaf(-x, r, 1.0f), r);
+  return x < 0x1p126f ? n : r;
+}
 
 // Named barrier over the 128 threads of one epilogue group (barrier id 1 or 2).
 __device__ __forceinline__ void epi_bar_sync(int id) { asm volatile("bar.sync %0, 128;" ::"r"(id) : "memory"); }
@@ -173,6 +188,8 @@ __device__ __forceinline__ void stage_row_f32(uint8_t* buf, int r, const float (
 // SwiGLU adjoint of 32 columns of one row: v = d_hidden (fp32 accumulator), wg / wu = saved gate / up (bf16 pairs) ->
 // pg = d_gate, pu = d_up.  d_hidden is rounded to bf16 first (what a stored d_hidden would hold), then
 //   d_up = dh * g * sig(g),  d_gate = dh * u * sig(g) * (1 + g * (1 - sig(g)))
+// EXACT: the bits of lmoe_swiglu_bwd on the stored d_hidden.
+template <bool EXACT>
 __device__ __forceinline__ void swiglu_adjoint_slab(const float (&v)[32], const uint32_t* wg, const uint32_t* wu,
                                                     uint32_t (&pg)[16], uint32_t (&pu)[16]) {
 #pragma unroll
@@ -184,7 +201,7 @@ __device__ __forceinline__ void swiglu_adjoint_slab(const float (&v)[32], const 
     float dg[2], du[2];
 #pragma unroll
     for (int k = 0; k < 2; ++k) {
-      const float sg = sigmoid_fast(g[k]);
+      const float sg = EXACT ? sigmoid_exact(g[k]) : sigmoid_fast(g[k]);
       du[k] = dh[k] * g[k] * sg;
       dg[k] = dh[k] * uu[k] * sg * (1.0f + g[k] * (1.0f - sg));
     }
@@ -588,7 +605,10 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_kernel(const __grid_cons
 #pragma unroll
           for (int j = 0; j < 16; ++j) pk[j] = pack_bf16x2(v[2 * j], v[2 * j + 1]);
         } else if (EPI == EPI_SWIGLU_BWD) {
-          swiglu_adjoint_slab(v, reinterpret_cast<const uint32_t*>(hg), reinterpret_cast<const uint32_t*>(hu), pk, pu);
+          if (ESZ == 1 || p.exact_sigmoid)
+            swiglu_adjoint_slab<true>(v, reinterpret_cast<const uint32_t*>(hg), reinterpret_cast<const uint32_t*>(hu), pk, pu);
+          else
+            swiglu_adjoint_slab<false>(v, reinterpret_cast<const uint32_t*>(hg), reinterpret_cast<const uint32_t*>(hu), pk, pu);
         } else if (EPI == EPI_SWIGLU) {
 #pragma unroll
           for (int j = 0; j < 16; ++j) {

@@ -404,7 +404,10 @@ gemm_pair_kernel(const __grid_constant__ GemmParams p) {
             hg[j] = ((c - c_begin) & 1) == 0 ? hg8[kAdj ? j : 0] : hg8[kAdj ? 4 + j : 0];
             hu[j] = ((c - c_begin) & 1) == 0 ? hu8[kAdj ? j : 0] : hu8[kAdj ? 4 + j : 0];
           }
-          swiglu_adjoint_slab(v, reinterpret_cast<const uint32_t*>(hg), reinterpret_cast<const uint32_t*>(hu), pk, pu);
+          if (p.exact_sigmoid)
+            swiglu_adjoint_slab<true>(v, reinterpret_cast<const uint32_t*>(hg), reinterpret_cast<const uint32_t*>(hu), pk, pu);
+          else
+            swiglu_adjoint_slab<false>(v, reinterpret_cast<const uint32_t*>(hg), reinterpret_cast<const uint32_t*>(hu), pk, pu);
         }
         if (kSwiglu && p.hidden_only) {  // as in gemm.cuh: one store per slab, two staging buffers in turn
           uint8_t* hbuf = sbuf0 + buf * S::kSlabBytes;

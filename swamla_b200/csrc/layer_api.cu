@@ -380,11 +380,10 @@ extern "C" int lmoe_grouped_wgrad_bf16(int64_t P, int E, int M, int N, const voi
   return launch_gemm(c);
 }
 
-extern "C" int lmoe_grouped_bwd_dgrad(int64_t P, int E, int L, int F, const void* d_y_sorted, const void* h1,
-                                      const void* w_gate_up, const void* w_down, const int32_t* tile_expert,
-                                      const int32_t* n_tiles, const int32_t* pad_offsets, void* d_hidden, void* d_h1,
-                                      void* d_x_sorted,
-                                      int32_t* status, void* stream) {
+static int grouped_bwd_dgrad(int64_t P, int E, int L, int F, const void* d_y_sorted, const void* h1, const void* w_gate_up,
+                             const void* w_down, const int32_t* tile_expert, const int32_t* n_tiles,
+                             const int32_t* pad_offsets, void* d_hidden, void* d_h1, void* d_x_sorted, bool exact_sigmoid,
+                             int32_t* status, void* stream) {
   if (!d_y_sorted || !h1 || !w_gate_up || !w_down || !tile_expert || !n_tiles || !d_h1 || !d_x_sorted)
     return LMOE_ERR_ARG;
   if (P <= 0 || (P % LMOE_ROW_PAD) != 0 || E <= 0 || (L % 64) != 0 || (F % 64) != 0) return LMOE_ERR_SHAPE;
@@ -425,6 +424,7 @@ extern "C" int lmoe_grouped_bwd_dgrad(int64_t P, int E, int L, int F, const void
     f.ldc = 2ll * F;
     f.aux = h1;
     f.ld_aux = 2ll * F;
+    f.exact_sigmoid = exact_sigmoid;
     if (int rc = launch_gemm(f)) return rc;
   }
   // d_x_sorted[P,L] = d_h1[P,2F] * Wgu[e]^T : Wgu[e] is [L,2F] = [N,K] row-major -> K-major B
@@ -440,6 +440,22 @@ extern "C" int lmoe_grouped_bwd_dgrad(int64_t P, int E, int L, int F, const void
   b.ldc = L;
   b.b_group_rows = L;
   return launch_gemm(b);
+}
+
+extern "C" int lmoe_grouped_bwd_dgrad(int64_t P, int E, int L, int F, const void* d_y_sorted, const void* h1,
+                                      const void* w_gate_up, const void* w_down, const int32_t* tile_expert,
+                                      const int32_t* n_tiles, const int32_t* pad_offsets, void* d_hidden, void* d_h1,
+                                      void* d_x_sorted, int32_t* status, void* stream) {
+  return grouped_bwd_dgrad(P, E, L, F, d_y_sorted, h1, w_gate_up, w_down, tile_expert, n_tiles, pad_offsets, d_hidden, d_h1,
+                           d_x_sorted, false, status, stream);
+}
+
+extern "C" int lmoe_moe_experts_bwd_dgrad(int64_t P, int E, int L, int F, const void* d_y_sorted, const void* h1,
+                                          const void* w_gate_up, const void* w_down, const int32_t* tile_expert,
+                                          const int32_t* n_tiles, const int32_t* pad_offsets, void* d_h1, void* d_x_sorted,
+                                          int32_t* status, void* stream) {
+  return grouped_bwd_dgrad(P, E, L, F, d_y_sorted, h1, w_gate_up, w_down, tile_expert, n_tiles, pad_offsets, nullptr, d_h1,
+                           d_x_sorted, true, status, stream);
 }
 
 extern "C" int lmoe_experts_bwd_dgrad(const lmoe_shape* s, const void* d_y_sorted, const void* h1, const void* w_gate_up,
@@ -587,6 +603,7 @@ extern "C" int lmoe_moe_shared_bwd(const lmoe_shape* s, const void* dy, const vo
                      stream);
   b.aux = h1_s;
   b.ld_aux = 2ll * s->Fs;
+  b.exact_sigmoid = true;
   if (int rc = launch_gemm(b)) return rc;
   const int split = wgrad_split(s->D, s->Fs, s->T);
   float* ws = static_cast<float*>(workspace);

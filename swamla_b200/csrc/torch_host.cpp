@@ -714,8 +714,8 @@ MoeGrads moe_backward(const Sizes& d, const MoeOps& o, const Tensor& dy, const f
   LMOE(lmoe_combine_bwd, &d.s, dy.data_ptr(), sv + at_.y_sorted, weights, &route, d_ys, d_w, side);
   fork.to_main();
   // routed experts
-  LMOE(lmoe_grouped_bwd_dgrad, P, d.E, d.D, d.F, d_ys, sv + at_.h1, o.wgu.data_ptr(), o.wde.data_ptr(), route.tile_expert,
-       route.n_tiles, route.pad_offsets, nullptr, d_h1, d_xs, status, st);
+  LMOE(lmoe_moe_experts_bwd_dgrad, P, d.E, d.D, d.F, d_ys, sv + at_.h1, o.wgu.data_ptr(), o.wde.data_ptr(), route.tile_expert,
+       route.n_tiles, route.pad_offsets, d_h1, d_xs, status, st);
   // [router adjoint (+ z-loss) -> cat[:, 2Fs:]; the entry point places d_logits after 2Fs + L columns] beside
   // [routed weight gradients]
   lmoe_shape cat_shape = d.s;

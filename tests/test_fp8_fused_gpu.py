@@ -89,10 +89,4 @@ def test_e4m3_gemm_epilogues_with_adjoint_and_amax(T):
     torch.cuda.synchronize()
     assert status.item() == 0
     assert amax.item() == got[:used].float().abs().max().item()
-    # Both round the same d_hidden to bf16 first.  The epilogue's sigmoid s comes from tanh.approx (2^-11 relative, so s is off
-    # by at most 2^-12), and d/ds of d_gate = dh * u * s * (1 + g * (1 - s)) and d_up = dh * g * s is at most
-    # dh * (1 + |g|)(1 + |u|); two bf16 roundings of nearly equal values differ by at most one ulp, 2^-7 relative.
-    a, b, dh = got[:used].float(), ref[:used].float(), d_hid[:used].float().abs().repeat(1, 2)
-    gu = h1[:used].float().abs()
-    scale = dh * (1.0 + gu[:, :F] + gu[:, F:] + gu[:, :F] * gu[:, F:]).repeat(1, 2)
-    assert ((a - b).abs() <= 2.0 ** -7 * b.abs() + 2.0 ** -11 * scale + 1e-30).all()
+    assert torch.equal(got[:used], ref[:used])                       # the same d_hidden, the same adjoint
