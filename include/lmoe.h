@@ -203,8 +203,8 @@ int lmoe_combine_out_fwd(const lmoe_shape* s, const void* y_sorted, const lmoe_r
 
 /* Whole forward of a few tokens (generation) in three or four launches without the padded layout: T <= LMOE_FEW_TOKENS, every other
  * dimension as lmoe_few_applies says.  With w_down = w_up = NULL and L = D: the non-latent layer (models/moe.py:344-372).
- * Same stages and rounding points as the entry points above (models/moe.py:702-734), fp32 sums in another order; the
- * expert weights are bf16 whatever the layer's precision for large batches.  Nothing is kept for a backward. */
+ * Same stages and rounding points as the entry points above (models/moe.py:702-734), fp32 sums in another order.  bf16
+ * expert weights only: a layer with e4m3 experts does not take it.  Nothing is kept for a backward. */
 #define LMOE_FEW_TOKENS 64
 int lmoe_few_applies(const lmoe_shape* s);
 size_t lmoe_few_workspace_bytes(const lmoe_shape* s);

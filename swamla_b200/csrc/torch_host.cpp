@@ -988,7 +988,7 @@ std::vector<Tensor> latent_moe(const Tensor& x, const Tensor& wg, const Tensor& 
     return LatentFn::apply(x, wg, wdn, wup, wgus, wds, wgu, wde, bias, top_k, z_coef, fp8);
   const LatentOps o = latent_ops(x, wg, wdn, wup, wgus, wds, wgu, wde);
   const Sizes d = latent_sizes(o.x, o.wgu, o.wds, top_k);
-  if (evaluation && d.T <= LMOE_FEW_TOKENS && lmoe_few_applies(&d.s)) {
+  if (evaluation && !fp8 && d.T <= LMOE_FEW_TOKENS && lmoe_few_applies(&d.s)) {  // (its experts are bf16)
     auto yz = few_forward(d, o.x, o.wg, &o.wdn, &o.wup, o.wgus, o.wds, o.wgu, o.wde, f32_bias(bias), static_cast<float>(z_coef));
     return {as_param(yz[0].view(x.sizes()), x.scalar_type()), yz[1]};
   }

@@ -138,7 +138,7 @@ def latent_moe(x: torch.Tensor, w_gate, w_down, w_up, w_gate_up_s, w_down_s, w_g
                z_coef: float, fp8: bool = False, evaluation: bool = False):
     """Functional form on a [..., D] activation.  Returns (y like x, aux_loss scalar, sel [T,K] int32, counts [E] int32).
     ``fp8``: run the routed expert GEMMs in e4m3 with per-tensor scaling (latent and routed hidden dims % 128 == 0).
-    ``evaluation``: without gradients, a few tokens may take the path of ``lmoe_few_forward`` (bf16 expert weights, no
+    ``evaluation``: without gradients and without ``fp8``, a few tokens may take the path of ``lmoe_few_forward`` (no
     routing tables: only (y, aux_loss) is returned then)."""
     if _testing.SINK is not None or _testing.FORCE_SEL is not None:
         return LatentMoEFunction.apply(x, w_gate, w_down, w_up, w_gate_up_s, w_down_s, w_gate_up, w_down_e, expert_bias,

@@ -65,3 +65,24 @@ def test_gradients_and_training_mode_keep_the_padded_path():
     assert lib.lmoe_launch_count() - before > 4
     y.sum().backward()
     assert x.grad is not None and layer.down_proj.weight.grad is not None
+
+
+@pytest.mark.parametrize("T", [1, 64, 65])
+def test_e4m3_layer_keeps_its_precision_at_every_size(T):
+    """An e4m3 layer in evaluation gives the training forward's bits: the same token's output does not depend on whether the
+    call holds few enough tokens for the bf16 kernels."""
+    from swamla_b200.layer import create_moe_layer
+    w = inputs.WORKLOADS["cfg1"]
+    cfg = w.config()
+    cfg.moe_fp8 = True
+    torch.manual_seed(T)
+    with torch.device("cuda:0"):
+        layer = create_moe_layer(cfg).to(torch.bfloat16)
+        x = torch.randn(1, T, w.D).to(torch.bfloat16)
+    assert layer.fp8_experts
+    with torch.no_grad():
+        want = layer.train()(x)
+        want_aux = layer.get_aux_loss()
+        got = layer.eval()(x)
+    layer.check_status()
+    assert torch.equal(got, want) and torch.equal(layer.get_aux_loss(), want_aux)
