@@ -548,16 +548,17 @@ __global__ void __launch_bounds__(kFewThreads) few_out_kernel(const FewParams p)
         for (int u = 0; u < 6; ++u) {
           const int s = (tok0 + tok) * p.K + min(k0 + u, p.K - 1);
           yv[u] = *reinterpret_cast<const uint4*>(p.y_slot + static_cast<long long>(s) * p.L + v * 8);
-          wk[u] = k0 + u < p.K ? p.weights[s] : 0.f;
+          wk[u] = p.weights[s];
         }
 #pragma unroll
         for (int u = 0; u < 6; ++u) {
           const uint32_t yw[4] = {yv[u].x, yv[u].y, yv[u].z, yv[u].w};
+          if (k0 + u < p.K)  // (a weight of zero instead would turn an infinite row into NaN)
 #pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            acc[2 * j] = fmaf(wk[u], bf_lo(yw[j]), acc[2 * j]);
-            acc[2 * j + 1] = fmaf(wk[u], bf_hi(yw[j]), acc[2 * j + 1]);
-          }
+            for (int j = 0; j < 4; ++j) {
+              acc[2 * j] = fmaf(wk[u], bf_lo(yw[j]), acc[2 * j]);
+              acc[2 * j + 1] = fmaf(wk[u], bf_hi(yw[j]), acc[2 * j + 1]);
+            }
         }
       }
       s_routed[i] = make_uint4(pack_bf16x2(acc[0], acc[1]), pack_bf16x2(acc[2], acc[3]), pack_bf16x2(acc[4], acc[5]),

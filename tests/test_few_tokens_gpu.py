@@ -86,3 +86,26 @@ def test_e4m3_layer_keeps_its_precision_at_every_size(T):
         got = layer.eval()(x)
     layer.check_status()
     assert torch.equal(got, want) and torch.equal(layer.get_aux_loss(), want_aux)
+
+
+@pytest.mark.parametrize("K", [1, 6, 7, 16])                             # the combine takes six slots at a time
+def test_infinite_expert_output_stays_infinite(K):
+    """The last slot's expert overflows bf16 in one latent column: infinities in the output, as on the padded path, no NaN."""
+    from types import SimpleNamespace
+    from swamla_b200.layer import create_moe_layer
+    cfg = SimpleNamespace(n_embd=128, latent_n_experts=32, latent_n_activated=K, latent_dim=64, expert_dim=256, latent_ratio=4,
+                          n_shared_experts=1, bias=False, dropout=0.0, use_latent_moe=True)
+    torch.manual_seed(K)
+    with torch.device("cuda:0"):
+        layer = create_moe_layer(cfg).to(torch.bfloat16).train()
+        x = torch.randn(1, 1, 128).to(torch.bfloat16)
+    with torch.no_grad():
+        layer(x)
+        e = int(layer.router._last_selected_experts[0, K - 1])
+        xl = (x[0, 0] @ layer.down_proj.weight.t()).float()
+        layer.experts.gate_up_weight[e] = (xl / xl.square().sum())[:, None]      # gate = up = 1: every hidden value 0.73
+        layer.experts.down_weight[e, :, 0] = 1e38
+        want = layer(x)
+        got = layer.eval()(x)
+    assert want.isinf().any() and not want.isnan().any()
+    assert torch.equal(got.isinf(), want.isinf()) and not got.isnan().any()
