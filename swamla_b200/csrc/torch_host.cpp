@@ -1046,7 +1046,9 @@ py::tuple latent_fwd_raw(const Tensor& x, const Tensor& wg, const Tensor& wdn, c
   Views views;
   LatentOut r = latent_forward(latent_sizes(o.x, o.wgu, o.wds, top_k), o, f32_bias(bias), static_cast<float>(z_coef), fp8,
                                true, forced_sel, capture ? &views : nullptr);
-  return py::make_tuple(as_param(r.y.view(x.sizes()), x.scalar_type()), r.z_loss, r.sel, r.counts, r.saved, dict_of(views));
+  const Tensor y = as_param(r.y.view(x.sizes()), x.scalar_type());
+  py::gil_scoped_acquire gil;
+  return py::make_tuple(y, r.z_loss, r.sel, r.counts, r.saved, dict_of(views));
 }
 
 py::tuple latent_bwd_raw(const c10::optional<Tensor>& dy, const c10::optional<Tensor>& d_z, const Tensor& x, const Tensor& wg,
@@ -1065,6 +1067,7 @@ py::tuple latent_bwd_raw(const c10::optional<Tensor>& dy, const c10::optional<Te
                           as_param(g.wdn, wdn.scalar_type()), as_param(g.wup, wup.scalar_type()),
                           as_param(g.wgus, wgus.scalar_type()), as_param(g.wds, wds.scalar_type()),
                           as_param(g.wgu, wgu.scalar_type()), as_param(g.wde, wde.scalar_type())};
+  py::gil_scoped_acquire gil;
   return py::make_tuple(out, dict_of(views));
 }
 
@@ -1087,16 +1090,19 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
       PyErr_SetString(g_error_class ? g_error_class : PyExc_RuntimeError, e.what());
     }
   });
+  // Whatever launches does so without the interpreter lock, as PyTorch's own operators do: a launch blocks while the device's
+  // queue is full, and what empties it may be another thread's to launch.
+  using NoGil = py::call_guard<py::gil_scoped_release>;
   m.def("set_error_class", [](py::object cls) { g_error_class = cls.inc_ref().ptr(); });
   m.def("poll_status", &poll_status);
-  m.def("latent_moe", &latent_moe);
-  m.def("moe", &moe);
-  m.def("latent_fwd_raw", &latent_fwd_raw);
-  m.def("latent_bwd_raw", &latent_bwd_raw);
+  m.def("latent_moe", &latent_moe, NoGil());
+  m.def("moe", &moe, NoGil());
+  m.def("latent_fwd_raw", &latent_fwd_raw, NoGil());
+  m.def("latent_bwd_raw", &latent_bwd_raw, NoGil());
   m.def("latent_saved_bytes", [](int64_t T, int64_t D, int64_t L, int64_t E, int64_t K, int64_t F, int64_t Fs) {
     return LatentLayout(Sizes(T, D, L, E, K, F, Fs), false, false).bytes;
   });
-  m.def("bias_update", &bias_update);
-  m.def("norm_and_pass", &norm_and_pass);
-  m.def("residual_add", &residual_add);
+  m.def("bias_update", &bias_update, NoGil());
+  m.def("norm_and_pass", &norm_and_pass, NoGil());
+  m.def("residual_add", &residual_add, NoGil());
 }

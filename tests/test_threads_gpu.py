@@ -1,0 +1,106 @@
+"""The layers' native calls from several host threads and on streams other than the default one."""
+import threading
+import time
+
+import pytest
+import torch
+
+from oracle import inputs
+
+pytestmark = pytest.mark.gpu
+KINDS = ["latent", "fp8", "moe", "block"]
+
+
+def _module(kind, seed):
+    from swamla_b200.block import NormedResidualFFN
+    from swamla_b200.layer import create_moe_layer
+    w = inputs.WORKLOADS["tiny_moe_ragged" if kind == "moe" else "tiny_fp8" if kind == "fp8" else "tiny_ragged"]
+    cfg = w.config()
+    cfg.moe_fp8 = kind == "fp8"
+    torch.manual_seed(seed)
+    with torch.device("cuda:0"):
+        m = create_moe_layer(cfg).to(torch.bfloat16)
+        if kind == "block":
+            m = NormedResidualFFN(m, w.D)
+        xs = [torch.randn(2, t, w.D, dtype=torch.float32 if kind == "block" else torch.bfloat16) for t in (3, 61, 190, 700)]
+    return m.train(), xs
+
+
+def _steps(m, xs, turns):
+    """A forward and backward per input, and an evaluation; everything that comes out."""
+    layer = getattr(m, "ffn", m)
+    out = []
+    for _ in range(turns):
+        for x in xs:
+            xg = x.clone().requires_grad_(True)
+            m.zero_grad(set_to_none=True)
+            y = m(xg)
+            (y.float().square().mean() + layer.get_aux_loss()).backward()
+            out += [y.detach(), xg.grad, *[p.grad for p in m.parameters()]]
+            layer.router.update_bias_from_last_forward()
+            out.append(layer.router.expert_bias.clone())
+            with torch.no_grad():
+                out.append(m.eval()(x))
+            m.train()
+    return out
+
+
+@pytest.mark.parametrize("kind", KINDS)
+def test_threads_on_their_own_streams_give_the_serial_bits(kind):
+    n, turns = 3, 4
+    want = [_steps(*_module(kind, i), turns) for i in range(n)]
+    torch.cuda.synchronize()
+    jobs, got, errors = [_module(kind, i) for i in range(n)], [None] * n, []
+    torch.cuda.synchronize()
+
+    def work(i):
+        try:
+            s = torch.cuda.Stream()
+            with torch.cuda.stream(s):
+                got[i] = _steps(*jobs[i], turns)
+            s.synchronize()
+        except Exception as e:                                           # pragma: no cover
+            errors.append(e)
+
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(n)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not errors, errors
+    for a, b in zip(want, got):
+        assert len(a) == len(b) and all(torch.equal(p, q) for p, q in zip(a, b))
+
+
+@pytest.mark.parametrize("kind", ["latent", "moe", "block"])
+def test_a_launch_that_waits_for_the_queue_lets_other_threads_run(kind):
+    """Behind a one-second kernel the queue fills up and a launch blocks until it ends; the interpreter lock must be free."""
+    m, xs = _module(kind, 0)
+    x, stop, gaps = xs[2], threading.Event(), []
+    with torch.no_grad():
+        m(x)
+    torch.cuda.synchronize()
+
+    def tick():
+        last = time.perf_counter()
+        while not stop.is_set():
+            time.sleep(0.001)
+            now = time.perf_counter()
+            gaps.append(now - last)
+            last = now
+
+    t = threading.Thread(target=tick)
+    t.start()
+    try:
+        torch.cuda._sleep(2_000_000_000)                                 # about a second of a kernel that ends by itself
+        t0 = time.perf_counter()
+        with torch.no_grad():
+            for _ in range(400):                                         # ten launches and more each
+                m(x)
+        blocked = time.perf_counter() - t0
+    finally:
+        stop.set()
+        t.join()
+        torch.cuda.synchronize()
+    assert blocked > 0.5, "the queue never filled up"
+    assert max(gaps) < 0.3 * blocked, (max(gaps), blocked)
