@@ -20,6 +20,7 @@
 #include <torch/csrc/jit/frontend/tracer.h>
 #include <torch/extension.h>
 
+#include <atomic>
 #include <cstring>
 #include <map>
 #include <mutex>
@@ -56,35 +57,55 @@ void check(int rc, const char* what) {
 }
 
 // ---------------------------------------------------------------- device status words
-// One int32 per kind of call, in mapped pinned memory: a kernel whose bounded wait gives up writes its code straight to
-// the host, which reads the word at its next call.  Never freed: kernels of any stream may still hold the address.
+// One int32 per device and kind of call, in mapped pinned memory: a kernel whose bounded wait gives up writes its code
+// straight to the host, which reads the word at its next call.  Never freed: kernels of any stream may still hold the address.
 enum Kind : int { kLatentFwd = 0, kLatentBwd = 1, kMoeFwd = 2, kMoeBwd = 3, kKinds = 4 };
 const char* const kKindName[kKinds] = {"LatentMoE forward", "LatentMoE backward", "MoE forward", "MoE backward"};
+constexpr int kStatusDevices = 64;
+constexpr int kStatusStride = 16;  // int32 per word: a cache line each
+std::atomic<bool> g_device_used[kStatusDevices];
 
 int32_t* status_words() {
   static int32_t* words = [] {
+    constexpr size_t bytes = kStatusDevices * kKinds * kStatusStride * sizeof(int32_t);
     void* p = nullptr;
     cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;  // the first call may be one that is being captured
     cudaThreadExchangeStreamCaptureMode(&mode);
-    const cudaError_t e = cudaHostAlloc(&p, 256, cudaHostAllocMapped | cudaHostAllocPortable);
+    const cudaError_t e = cudaHostAlloc(&p, bytes, cudaHostAllocMapped | cudaHostAllocPortable);
     cudaThreadExchangeStreamCaptureMode(&mode);
     if (e != cudaSuccess)
       throw LmoeFailure("no pinned memory for the device status words");
-    std::memset(p, 0, 256);
+    std::memset(p, 0, bytes);
     return static_cast<int32_t*>(p);
   }();
   return words;
 }
-int32_t* status_word(Kind k) { return status_words() + 16 * k; }  // a cache line each
+int32_t* status_word(int device, Kind k) { return status_words() + (device * kKinds + k) * kStatusStride; }
+// The word of a call that is about to launch on the current device.
+int32_t* status_word(Kind k) {
+  const int device = c10::cuda::current_device();
+  TORCH_CHECK(device >= 0 && device < kStatusDevices, "device ordinal out of range");
+  g_device_used[device].store(true, std::memory_order_relaxed);
+  return status_word(device, k);
+}
+std::vector<int> devices_used() {
+  std::vector<int> v;
+  for (int d = 0; d < kStatusDevices; ++d)
+    if (g_device_used[d].load(std::memory_order_relaxed)) v.push_back(d);
+  return v;
+}
 
 // Throws for the first word that a kernel has written; the word is cleared.
 void poll_status() {
-  for (int k = 0; k < kKinds; ++k) {
-    volatile int32_t* w = status_word(static_cast<Kind>(k));
-    const int32_t code = *w;
-    if (code != 0) {
-      *w = 0;
-      throw LmoeFailure("device status " + std::to_string(code) + " in " + kKindName[k] + ": " + lmoe_status_string(code));
+  for (int d = 0; d < kStatusDevices; ++d) {
+    if (!g_device_used[d].load(std::memory_order_relaxed)) continue;
+    for (int k = 0; k < kKinds; ++k) {
+      int32_t* w = status_word(d, static_cast<Kind>(k));
+      if (__atomic_load_n(w, __ATOMIC_RELAXED) == 0) continue;
+      const int32_t code = __atomic_exchange_n(w, 0, __ATOMIC_RELAXED);
+      if (code != 0)
+        throw LmoeFailure("device status " + std::to_string(code) + " in " + kKindName[k] + " on cuda:" + std::to_string(d) + ": " +
+                          lmoe_status_string(code));
     }
   }
 }
@@ -1095,6 +1116,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   using NoGil = py::call_guard<py::gil_scoped_release>;
   m.def("set_error_class", [](py::object cls) { g_error_class = cls.inc_ref().ptr(); });
   m.def("poll_status", &poll_status);
+  m.def("devices_used", &devices_used);
   m.def("latent_moe", &latent_moe, NoGil());
   m.def("moe", &moe, NoGil());
   m.def("latent_fwd_raw", &latent_fwd_raw, NoGil());

@@ -34,14 +34,24 @@ def post(status: torch.Tensor, label: str) -> None:
 
 
 def poll(block: bool = False) -> None:
-    """Raises ``LmoeError`` if a completed step reported a non-zero device status."""
+    """Raises ``LmoeError`` if a completed step reported a non-zero device status; ``block`` waits for the queued steps of
+    every device first (not while the current stream is being captured, when nothing may be waited for)."""
     global _pending
+    host = None
     if block:
         from . import functional
-        torch.cuda.synchronize()
-        functional._host().poll_status()
-    if not _pending or torch.cuda.is_current_stream_capturing():
+        host = functional._native            # not loaded: no single-GPU step has been queued
+    devices = host.devices_used() if host is not None else []
+    if not (_pending or devices) or torch.cuda.is_current_stream_capturing():
         return
+    failure = None
+    for d in devices:                        # whichever device is current: the words are written by the steps' own ones
+        torch.cuda.synchronize(d)
+    if devices:
+        try:
+            host.poll_status()
+        except _cabi.LmoeError as e:         # raised when the entries below have been looked at
+            failure = e
     keep, bad = [], None
     for ev, host, label in _pending:
         if block:
@@ -54,6 +64,8 @@ def poll(block: bool = False) -> None:
         else:
             keep.append((ev, host, label))
     _pending = keep
+    if failure is not None:
+        raise failure
     if bad is not None:
         code, label = bad
         raise _cabi.LmoeError(f"device status {code} in {label}: {_cabi.status_string(code)}")

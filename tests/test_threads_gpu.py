@@ -104,3 +104,20 @@ def test_a_launch_that_waits_for_the_queue_lets_other_threads_run(kind):
         torch.cuda.synchronize()
     assert blocked > 0.5, "the queue never filled up"
     assert max(gaps) < 0.3 * blocked, (max(gaps), blocked)
+
+
+def test_a_failure_names_its_device_and_is_reported_once():
+    from swamla_b200 import _cabi, _testing
+    m, xs = _module("latent", 0)
+    sink = {}
+    _testing.SINK = sink
+    try:
+        m(xs[0])
+    finally:
+        _testing.SINK = None
+    torch.cuda.synchronize()
+    sink["status"].fill_(101)                # what a kernel writes when its wait gives up
+    with pytest.raises(_cabi.LmoeError, match="101 in LatentMoE forward on cuda:0"):
+        m.check_status()
+    m.check_status()
+    m(xs[0])
