@@ -15,6 +15,9 @@ namespace lmoe {
 
 constexpr int kTopkWarps = 8;       // warps of a top-k block, and the fewest of one that also counts
 constexpr int kMaxTopkWarps = 32;
+constexpr int kMaxChunkTokens = 128;  // tokens of a block
+// z_partial: the fp32 sum of lse^2 over eight consecutive tokens each, whatever the block's size; the rest of the sum is fp64.
+constexpr int kZGroup = 8;
 
 // One warp per token, `per_warp` consecutive tokens each.  With chunk_hist the block also counts its selections:
 // chunk_hist[blockIdx.x][E] is the first pass of the routing tables (whole numbers: the order of the shared-memory
@@ -24,34 +27,39 @@ __global__ void __launch_bounds__(kMaxTopkWarps * 32)
 gate_topk_kernel(const float* __restrict__ logits, const float* __restrict__ bias, int T, int E, int K, int* __restrict__ sel,
                  float* __restrict__ weights, float* __restrict__ lse_out, float* __restrict__ z_partial, int per_warp,
                  int* __restrict__ chunk_hist) {
-  __shared__ float s_lse2[kMaxTopkWarps];
+  __shared__ float s_lse2[kMaxChunkTokens];
   __shared__ int s_hist[32 * PER];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
   if (chunk_hist) {
     for (int e = threadIdx.x; e < E; e += blockDim.x) s_hist[e] = 0;
     __syncthreads();
   }
-  float lse2 = 0.f;
   for (int r = 0; r < per_warp; ++r) {
-    const int t = (blockIdx.x * warps + warp) * per_warp + r;
-    if (t >= T) break;
+    const int slot = warp * per_warp + r, t = blockIdx.x * warps * per_warp + slot;
+    if (t >= T) {
+      if (lane == 0) s_lse2[slot] = 0.f;
+      continue;
+    }
     int idx;
     float aff, aff_sum, lse;
     topk_row<PER>(logits + static_cast<long long>(t) * E, bias, E, K, lane, idx, aff, aff_sum, lse);
-    lse2 += lse * lse;
-    if (lane == 0) lse_out[t] = lse;
+    if (lane == 0) {
+      s_lse2[slot] = lse * lse;
+      lse_out[t] = lse;
+    }
     if (lane < K) {
       sel[static_cast<long long>(t) * K + lane] = idx;
       weights[static_cast<long long>(t) * K + lane] = aff / (aff_sum + 1e-9f);
       if (chunk_hist) atomicAdd(&s_hist[idx], 1);
     }
   }
-  if (lane == 0) s_lse2[warp] = lse2;
   __syncthreads();
-  if (threadIdx.x == 0) {
+  const int groups = warps * per_warp / kZGroup;
+  if (static_cast<int>(threadIdx.x) < groups) {
+    const int g = blockIdx.x * groups + threadIdx.x;
     float s = 0.f;
-    for (int i = 0; i < warps; ++i) s += s_lse2[i];
-    z_partial[blockIdx.x] = s;
+    for (int i = 0; i < kZGroup; ++i) s += s_lse2[threadIdx.x * kZGroup + i];
+    if (g * kZGroup < T) z_partial[g] = s;
   }
   if (chunk_hist)
     for (int e = threadIdx.x; e < E; e += blockDim.x) chunk_hist[static_cast<long long>(blockIdx.x) * E + e] = s_hist[e];
@@ -223,7 +231,6 @@ route_scatter_kernel(const int* __restrict__ sel, int n, int E, const int* __res
 // it K times).  Blocks beyond the last chunk, and every block besides its chunk, publish the tables and zero the pad rows of
 // experts b, b + gridDim.x, ...; block 0 also adds up the z-loss.
 constexpr int kDirectChunks = 128;
-constexpr int kMaxChunkTokens = 128;
 constexpr int kMaskWords = kMaxChunkTokens / 32;
 
 __global__ void __launch_bounds__(256)
@@ -317,7 +324,9 @@ route_gather_kernel(const int* __restrict__ sel, int T, int E, int K, int tokens
       r.n_tiles[0] = s_poff[E] / LMOE_ROW_PAD;
     }
     double acc = 0.0;
-    for (int i = tid; i < chunks; i += 256) acc += static_cast<double>(z_partial[i]);
+    const int n_z = (T + kZGroup - 1) / kZGroup;
+#pragma unroll 8
+    for (int i = tid; i < n_z; i += 256) acc += static_cast<double>(z_partial[i]);
     s_z[tid] = acc;
     __syncthreads();
     for (int o = 128; o > 0; o >>= 1) {
@@ -439,7 +448,7 @@ extern "C" int lmoe_gate_topk_fwd(const lmoe_shape* s, const float* logits, cons
   if (!logits || !expert_bias || !sel || !weights || !lse || !z_partial || !z_loss) return LMOE_ERR_ARG;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   launch_topk(s, logits, expert_bias, sel, weights, lse, z_partial, kTopkWarps, 1, nullptr, st);
-  const int blocks = (s->T + kTopkWarps - 1) / kTopkWarps;
+  const int blocks = (s->T + kZGroup - 1) / kZGroup;
   count_launch();
   zloss_finalize_kernel<<<1, 256, 0, st>>>(z_partial, blocks, z_coef / static_cast<float>(s->T), z_loss);
   cudaError_t e = cudaGetLastError();
@@ -467,8 +476,8 @@ static RouteChunks route_chunks(int T) {
 
 extern "C" size_t lmoe_route_fwd_workspace_bytes(const lmoe_shape* s) {
   if (check_shape(s)) return 0;
-  const size_t chunks = static_cast<size_t>(route_chunks(s->T).n);
-  return (chunks * s->E + (chunks + 3) / 4 * 4) * sizeof(int);
+  const size_t chunks = static_cast<size_t>(route_chunks(s->T).n), z = (static_cast<size_t>(s->T) + kZGroup - 1) / kZGroup;
+  return (chunks * s->E + (z + 3) / 4 * 4) * sizeof(int);
 }
 
 extern "C" int lmoe_topk_hist_fwd(const lmoe_shape* s, const float* logits, const float* expert_bias, int32_t* sel,

@@ -6,9 +6,10 @@ import torch
 pytestmark = pytest.mark.gpu
 
 
-# one token, one top-k block and its neighbours, the last size with one token per warp, the last one without the scan
-# kernel and its neighbour, several tokens per warp with a ragged last chunk; expert counts of both top-k kernels
-@pytest.mark.parametrize("T", [1, 7, 8, 9, 1024, 1025, 4096, 4097, 20001])
+# one token, one top-k block of eight warps and its neighbours, the last size with such blocks and its neighbour (16 warps), the
+# last one without the scan kernel and its neighbour, one token per warp with a ragged last chunk; two, three and four tokens per
+# warp (chunks of two, three and four mask words) with ragged last chunks, and more chunks than 1,024
+@pytest.mark.parametrize("T", [1, 7, 8, 9, 1024, 1025, 4096, 4097, 20001, 32769, 65567, 131089, 140007])
 @pytest.mark.parametrize("E,K", [(128, 12), (256, 16), (32, 3), (40, 5), (256, 32)])
 def test_fused_routing_equals_separate_entry_points(T, E, K):
     from swamla_b200 import _cabi
@@ -21,6 +22,7 @@ def test_fused_routing_equals_separate_entry_points(T, E, K):
     g = torch.Generator(dev).manual_seed(T + E)
     logits = torch.randn(T, E, device=dev, generator=g)
     logits[:, : E // 4] += 1.0                                   # uneven load; some experts stay empty at small T
+    logits[3::32] += 3000.0                                      # squares that absorb small ones: the z-loss sum's grouping shows
     bias = 0.1 * torch.randn(E, device=dev, generator=g)
     src = torch.randn(T, L, device=dev, generator=g).to(torch.bfloat16)
     got = []
@@ -52,10 +54,7 @@ def test_fused_routing_equals_separate_entry_points(T, E, K):
         got.append(dict(t, sel=sel, w=w, lse=lse, z=z, rows=rows))
     a, b = got
     for k in a:
-        if k != "z":
-            assert torch.equal(a[k], b[k]), k
-    # the z-loss sums the same fp32 squares in another grouping: at most T roundings of 2^-24 relative
-    assert abs(a["z"].item() - b["z"].item()) <= 2.0 ** -24 * 32 * abs(a["z"].item())
+        assert torch.equal(a[k], b[k]), k
 
 
 @pytest.mark.parametrize("M,H", [(1, 64), (129, 96), (300, 160), (1024, 1024)])   # one-CTA and CTA-pair kernels, ragged tiles
