@@ -309,6 +309,7 @@ extern "C" int lmoe_grouped_swiglu_bwd_fp8(int64_t P, int E, int L, int F, const
   a.n_m_tiles = n_tiles;
   a.deq_a = deq_dy;
   a.deq_b = deq_wd;
+  a.exact_sigmoid = true;
   a.amax = amax_d_h1;
   a.status = status;
   a.stream = static_cast<cudaStream_t>(stream);

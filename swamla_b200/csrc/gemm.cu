@@ -104,9 +104,9 @@ static bool g_prof_enabled = false;
 static std::vector<std::pair<cudaEvent_t, cudaEvent_t>> g_prof_events;
 
 // ---------------------------------------------------------------- dispatch
-template <bool A_MN, bool B_MN, int BN, int EPI, int GRP, int ESZ>
+template <bool A_MN, bool B_MN, int BN, int EPI, int GRP, int ESZ, bool EXACT = false>
 static int launch_inst(const GemmParams& p, int grid, cudaStream_t stream) {
-  auto kfn = gemm_kernel<A_MN, B_MN, BN, EPI, GRP, ESZ>;
+  auto kfn = gemm_kernel<A_MN, B_MN, BN, EPI, GRP, ESZ, EXACT>;
   constexpr int smem = GemmSmem<BN, EPI, GRP>::kTotal;
   static PerDeviceOnce once;  // one per template instantiation
   if (int rc = once.run([&] {
@@ -140,6 +140,10 @@ static int launch_inst(const GemmParams& p, int grid, cudaStream_t stream) {
 #define LMOE_CASE(am, bm, bn, epi, grp, esz)          \
   case LMOE_KEY(am, bm, (bn == 256), epi, grp, esz):  \
     return launch_inst<(am != 0), (bm != 0), bn, epi, grp, esz>(p, grid, stream);
+#define LMOE_CASE_ADJOINT(am, bm, grp)                                                                            \
+  case LMOE_KEY(am, bm, 0, EPI_SWIGLU_BWD, grp, 2):                                                               \
+    return c.exact_sigmoid ? launch_inst<(am != 0), (bm != 0), 128, EPI_SWIGLU_BWD, grp, 2, true>(p, grid, stream) \
+                           : launch_inst<(am != 0), (bm != 0), 128, EPI_SWIGLU_BWD, grp, 2>(p, grid, stream);
 #define LMOE_CASE_BN(am, bm, epi, grp, esz) LMOE_CASE(am, bm, 128, epi, grp, esz) LMOE_CASE(am, bm, 256, epi, grp, esz)
 #define LMOE_CASE_MAJORS(epi, grp, esz)                                                                      \
   LMOE_CASE_BN(0, 0, epi, grp, esz) LMOE_CASE_BN(0, 1, epi, grp, esz) LMOE_CASE_BN(1, 0, epi, grp, esz) \
@@ -159,12 +163,13 @@ static int dispatch(const GemmCall& c, int bn, const GemmParams& p, int grid, cu
     // grouped over the contraction (routed wgrads)
     LMOE_CASE_BN(1, 1, EPI_BF16, GRP_K, 2)
     // dgrad with the SwiGLU adjoint in the epilogue (routed and shared)
-    LMOE_CASE(0, 0, 128, EPI_SWIGLU_BWD, GRP_M, 2)
-    LMOE_CASE(0, 1, 128, EPI_SWIGLU_BWD, GRP_NONE, 2)
+    LMOE_CASE_ADJOINT(0, 0, GRP_M)
+    LMOE_CASE_ADJOINT(0, 1, GRP_NONE)
     // ---- e4m3 ----
     LMOE_CASE_MAJORS(EPI_BF16, GRP_NONE, 1)
     LMOE_CASE(0, 1, 256, EPI_SWIGLU, GRP_M, 1)
-    LMOE_CASE(0, 0, 128, EPI_SWIGLU_BWD, GRP_M, 1)
+    case LMOE_KEY(0, 0, 0, EPI_SWIGLU_BWD, GRP_M, 1):
+      return launch_inst<false, false, 128, EPI_SWIGLU_BWD, GRP_M, 1, true>(p, grid, stream);
     LMOE_CASE_BN(0, 1, EPI_BF16, GRP_M, 1)
     LMOE_CASE_BN(0, 0, EPI_BF16, GRP_M, 1)
     LMOE_CASE_BN(1, 1, EPI_BF16, GRP_K, 1)
@@ -186,9 +191,9 @@ static bool pair_gemm_enabled() {
 
 bool pair_gemm_applies(int M, int N) { return pair_gemm_enabled() && M >= 256 && N >= 256; }
 
-template <bool A_MN, bool B_MN, int EPI, int GRP = GRP_NONE>
+template <bool A_MN, bool B_MN, int EPI, int GRP = GRP_NONE, bool EXACT = false>
 static int launch_pair_inst(const GemmParams& p, long long total_tiles, cudaStream_t stream) {
-  auto kfn = gemm_pair_kernel<A_MN, B_MN, EPI, GRP>;
+  auto kfn = gemm_pair_kernel<A_MN, B_MN, EPI, GRP, EXACT>;
   constexpr int smem = PairSmem<EPI>::kTotal;
   static PerDeviceOnce once;  // one per template instantiation
   static int max_pairs_dev[kMaxDevices] = {};
@@ -287,7 +292,6 @@ static int launch_gemm_pair(const GemmCall& c) {
   p.split_k = split;
   p.half = c.N;
   p.hidden_only = c.C ? 0 : 1;
-  p.exact_sigmoid = c.exact_sigmoid ? 1 : 0;
   p.status = c.status;
   const long long total = static_cast<long long>(m_tiles) * n_tiles * split;
   const int key = c.a_mn | (c.b_mn << 1) | (c.epi << 2);
@@ -301,7 +305,9 @@ static int launch_gemm_pair(const GemmCall& c) {
     case 2 | (EPI_F32 << 2): return launch_pair_inst<false, true, EPI_F32>(p, total, c.stream);
     case 3 | (EPI_F32 << 2): return launch_pair_inst<true, true, EPI_F32>(p, total, c.stream);
     case 0 | (EPI_SWIGLU << 2): return launch_pair_inst<false, false, EPI_SWIGLU>(p, total, c.stream);
-    case 2 | (EPI_SWIGLU_BWD << 2): return launch_pair_inst<false, true, EPI_SWIGLU_BWD>(p, total, c.stream);
+    case 2 | (EPI_SWIGLU_BWD << 2):
+      return c.exact_sigmoid ? launch_pair_inst<false, true, EPI_SWIGLU_BWD, GRP_NONE, true>(p, total, c.stream)
+                             : launch_pair_inst<false, true, EPI_SWIGLU_BWD>(p, total, c.stream);
     default: return LMOE_ERR_ARG;
   }
 }
@@ -539,7 +545,6 @@ int launch_gemm(const GemmCall& c) {
   p.split_k = split;
   p.half = c.N;
   p.hidden_only = c.C ? 0 : 1;
-  p.exact_sigmoid = c.exact_sigmoid ? 1 : 0;
   p.tile_expert = c.tile_expert;
   p.n_m_tiles = c.n_m_tiles;
   p.b_group_rows = c.b_group_rows;

@@ -70,7 +70,6 @@ struct alignas(64) GemmParams {
   const float* deq_a;      // e4m3: per-tensor de-scale factors (amax / 448) of A and B, device scalars
   const float* deq_b;
   float* amax;             // e4m3 operands, SwiGLU epilogues: max |hidden| / max |d_h1| (bf16-rounded), device scalar or NULL
-  int exact_sigmoid;       // EPI_SWIGLU_BWD, bf16 operands: sigmoid_exact instead of sigmoid_fast (e4m3 operands: always)
   const void* aux;         // EPI_SWIGLU_BWD: h1 [rows, 2*N] bf16 (gate | up), row stride ld_aux elements
   long long ld_aux;
   CUtensorMap tmAux;       // EPI_SWIGLU_BWD: the same tensor as 128-row boxes of 64 columns (128-byte swizzle), staged by TMA
@@ -210,8 +209,9 @@ __device__ __forceinline__ void swiglu_adjoint_slab(const float (&v)[32], const 
   }
 }
 
-// ESZ = operand element size in bytes: 2 (bf16) or 1 (e4m3).
-template <bool A_MN, bool B_MN, int BN, int EPI, int GRP, int ESZ = 2>
+// ESZ = operand element size in bytes: 2 (bf16) or 1 (e4m3).  EXACT: which sigmoid EPI_SWIGLU_BWD takes; an instance of its
+// own, because a branch on a launch parameter cost the other one 1 % of a training step (2,190 -> 2,209 us with 256 experts).
+template <bool A_MN, bool B_MN, int BN, int EPI, int GRP, int ESZ = 2, bool EXACT = false>
 __global__ void __launch_bounds__(kGemmThreads, 1) gemm_kernel(const __grid_constant__ GemmParams p) {
   using S = GemmSmem<BN, EPI, GRP>;
   constexpr int STAGES = S::kStages;
@@ -605,10 +605,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_kernel(const __grid_cons
 #pragma unroll
           for (int j = 0; j < 16; ++j) pk[j] = pack_bf16x2(v[2 * j], v[2 * j + 1]);
         } else if (EPI == EPI_SWIGLU_BWD) {
-          if (ESZ == 1 || p.exact_sigmoid)
-            swiglu_adjoint_slab<true>(v, reinterpret_cast<const uint32_t*>(hg), reinterpret_cast<const uint32_t*>(hu), pk, pu);
-          else
-            swiglu_adjoint_slab<false>(v, reinterpret_cast<const uint32_t*>(hg), reinterpret_cast<const uint32_t*>(hu), pk, pu);
+          swiglu_adjoint_slab<EXACT>(v, reinterpret_cast<const uint32_t*>(hg), reinterpret_cast<const uint32_t*>(hu), pk, pu);
         } else if (EPI == EPI_SWIGLU) {
 #pragma unroll
           for (int j = 0; j < 16; ++j) {

@@ -31,7 +31,7 @@ struct GemmCall {
   long long ldc2 = 0;
   const void* aux = nullptr;     // EPI_SWIGLU_BWD: h1 [rows, 2N] bf16; C is then d_h1 [rows, 2N]
   long long ld_aux = 0;
-  bool exact_sigmoid = false;    // EPI_SWIGLU_BWD: see GemmParams::exact_sigmoid
+  bool exact_sigmoid = false;    // EPI_SWIGLU_BWD: sigmoid_exact instead of sigmoid_fast (e4m3 operands: always set)
   float* amax = nullptr;         // e4m3 grouped GEMMs: amax[0] = max(amax[0], max |what the epilogue forms|), see gemm.cuh
   // Gathered A (bf16, nseg == 1, GRP_M with K-major A or GRP_K): A[0] is the SOURCE tensor [a_src_rows, K or M]
   // and padded row i reads its row a_rows[i * a_rows_stride] / a_rows_div; a negative entry reads row a_zero_row,

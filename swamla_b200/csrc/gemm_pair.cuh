@@ -44,7 +44,8 @@ struct PairSmem {
 // the first tile and stores nothing.
 // GRP == GRP_K (grouped over the contraction, both operands MN-major): output plane e is A[rows_e, :]^T * B[rows_e, :] over
 // expert e's padded rows (pad_offsets); one 256 x 256 tile of one expert per pair.  An expert without rows writes zeros.
-template <bool A_MN, bool B_MN, int EPI, int GRP = GRP_NONE>
+// EXACT: as in gemm.cuh.
+template <bool A_MN, bool B_MN, int EPI, int GRP = GRP_NONE, bool EXACT = false>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1)
 gemm_pair_kernel(const __grid_constant__ GemmParams p) {
   static_assert(GRP == GRP_NONE || (GRP == GRP_M && !A_MN) || (GRP == GRP_K && A_MN && B_MN && EPI == EPI_BF16),
@@ -404,10 +405,7 @@ gemm_pair_kernel(const __grid_constant__ GemmParams p) {
             hg[j] = ((c - c_begin) & 1) == 0 ? hg8[kAdj ? j : 0] : hg8[kAdj ? 4 + j : 0];
             hu[j] = ((c - c_begin) & 1) == 0 ? hu8[kAdj ? j : 0] : hu8[kAdj ? 4 + j : 0];
           }
-          if (p.exact_sigmoid)
-            swiglu_adjoint_slab<true>(v, reinterpret_cast<const uint32_t*>(hg), reinterpret_cast<const uint32_t*>(hu), pk, pu);
-          else
-            swiglu_adjoint_slab<false>(v, reinterpret_cast<const uint32_t*>(hg), reinterpret_cast<const uint32_t*>(hu), pk, pu);
+          swiglu_adjoint_slab<EXACT>(v, reinterpret_cast<const uint32_t*>(hg), reinterpret_cast<const uint32_t*>(hu), pk, pu);
         }
         if (kSwiglu && p.hidden_only) {  // as in gemm.cuh: one store per slab, two staging buffers in turn
           uint8_t* hbuf = sbuf0 + buf * S::kSlabBytes;
