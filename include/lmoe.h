@@ -504,6 +504,14 @@ int lmoe_rmsnorm_bwd_typed(const void* x, int x_type, const void* weight, int w_
                            int g_type, const void* d_residual, int64_t T, int D, void* dx, void* d_weight, int dw_type,
                            void* workspace, size_t workspace_bytes, void* stream);
 int lmoe_add_f32_bf16(const float* a, const void* b, float* out, int64_t n, void* stream);
+/* The pair that the layers run.  The forward also writes what the adjoint needs into buffers of the caller's (either may be
+ * NULL): x_keep[T, D] bf16, the rows of an fp32 x as the norm sees them, and w_keep[D] fp32.  The adjoint takes the kept rows
+ * and d_residual and dx in the stream's type s_type. */
+int lmoe_rmsnorm_fwd_keep(const void* x, int x_type, const void* weight, int w_type, float eps, int64_t T, int D, void* xn,
+                          int xn_type, float* rstd, void* x_keep, float* w_keep, void* stream);
+int lmoe_rmsnorm_bwd_kept(const void* x_bf16, const void* weight, int w_type, const float* rstd, const void* d_xn, int g_type,
+                          const void* d_residual, int s_type, int64_t T, int D, void* dx, void* d_weight, int dw_type,
+                          void* workspace, size_t workspace_bytes, void* stream);
 
 /* ---- router bias update (after backward) ----
  * load = histogram(sel) (= counts); bias -= gamma * sign(load - T*K/E); history = .99 history + .01 load.

@@ -116,6 +116,8 @@ SIGNATURES = {
     "lmoe_rmsnorm_bwd": (c_int, [P, P, P, P, P, c_int64, c_int, P, P, P, c_size_t, P]),
     "lmoe_rmsnorm_fwd_typed": (c_int, [P, c_int, P, c_int, c_float, c_int64, c_int, P, c_int, P, P]),
     "lmoe_rmsnorm_bwd_typed": (c_int, [P, c_int, P, c_int, P, P, c_int, P, c_int64, c_int, P, P, c_int, P, c_size_t, P]),
+    "lmoe_rmsnorm_fwd_keep": (c_int, [P, c_int, P, c_int, c_float, c_int64, c_int, P, c_int, P, P, P, P]),
+    "lmoe_rmsnorm_bwd_kept": (c_int, [P, P, c_int, P, P, c_int, P, c_int, c_int64, c_int, P, P, c_int, P, c_size_t, P]),
     "lmoe_add_f32_bf16": (c_int, [P, P, P, c_int64, P]),
     "lmoe_moe_wgrad_workspace_bytes": (c_size_t, [SP]),
     "lmoe_moe_experts_bwd_dgrad": (c_int, [c_int64, c_int, c_int, c_int, P, P, P, P, P, P, P, P, P, P, P]),

@@ -95,11 +95,20 @@ __device__ __forceinline__ float warp_sum(float v) {
 }
 
 // X32: type of x; Y32: type of xn.  CH chunks per lane cover the row.
+// x_keep, w_keep (may be NULL): what the adjoint needs, in buffers of the call's own, so that the stream and a bf16 weight may
+// be changed in place before it runs: the rounded row (an fp32 x; the adjoint then reads half the bytes that this writes more)
+// and the weight in fp32.
 template <bool X32, bool Y32, int CH>
 __global__ void __launch_bounds__(kNormWarps * 32)
 rmsnorm_fwd_kernel(const void* __restrict__ x, const void* __restrict__ w, bool w32, float eps, long long T, int vec_per_row,
-                   void* __restrict__ xn, float* __restrict__ rstd) {
+                   void* __restrict__ xn, float* __restrict__ rstd, void* __restrict__ x_keep, float* __restrict__ w_keep) {
   const int lane = threadIdx.x & 31;
+  if (w_keep && blockIdx.x == 0)
+    for (int v = threadIdx.x; v < vec_per_row; v += blockDim.x) {
+      float ww[8];
+      load_weight(w, w32, v, ww);
+      store_chunk<true>(w_keep, v, ww);
+    }
   const float inv_d = 1.0f / static_cast<float>(vec_per_row * 8);
   for (long long t = static_cast<long long>(blockIdx.x) * kNormWarps + (threadIdx.x >> 5); t < T;
        t += static_cast<long long>(gridDim.x) * kNormWarps) {
@@ -129,6 +138,7 @@ rmsnorm_fwd_kernel(const void* __restrict__ x, const void* __restrict__ w, bool 
 #pragma unroll
         for (int j = 0; j < 8; ++j) o[j] = ww[j] * (f[j] * r);
         store_chunk<Y32>(xn, t * vec_per_row + v, o);
+        if (X32 && x_keep) store_chunk<false>(x_keep, t * vec_per_row + v, f);
       }
     }
   }
@@ -165,8 +175,8 @@ add_f32_bf16_kernel(const void* __restrict__ a, const void* __restrict__ b, void
 }
 
 // partial[blockIdx.x][D]: this block's share of d_w.  Shared memory: one row of D floats per warp (dynamic).
-// X32: type of x, d_res and dx; G32: type of d_xn.
-template <bool X32, bool G32, int CH>
+// X32: type of x; S32: type of the stream's gradients, d_res and dx; G32: type of d_xn.
+template <bool X32, bool S32, bool G32, int CH>
 __global__ void __launch_bounds__(kNormWarps * 32)
 rmsnorm_bwd_kernel(const void* __restrict__ x, const void* __restrict__ w, bool w32, const float* __restrict__ rstd,
                    const void* __restrict__ d_xn, const void* __restrict__ d_res, long long T, int vec_per_row,
@@ -184,7 +194,8 @@ rmsnorm_bwd_kernel(const void* __restrict__ x, const void* __restrict__ w, bool 
   for (long long t = static_cast<long long>(blockIdx.x) * kNormWarps + warp; t < T;
        t += static_cast<long long>(gridDim.x) * kNormWarps) {
     const float r = rstd[t];
-    Chunk<X32> xr[CH], rr[CH];
+    Chunk<X32> xr[CH];
+    Chunk<S32> rr[CH];
     Chunk<G32> gr[CH];
 #pragma unroll
     for (int i = 0; i < CH; ++i) {
@@ -229,7 +240,7 @@ rmsnorm_bwd_kernel(const void* __restrict__ x, const void* __restrict__ w, bool 
 #pragma unroll
           for (int j = 0; j < 8; ++j) o[j] += fr[j];
         }
-        store_chunk<X32>(dx, t * vec_per_row + v, o);
+        store_chunk<S32>(dx, t * vec_per_row + v, o);
       }
     }
   }
@@ -302,11 +313,11 @@ extern "C" size_t lmoe_rmsnorm_workspace_bytes(int D) {
   return D > 0 ? static_cast<size_t>(kNormMaxBlocks) * D * sizeof(float) : 0;
 }
 
-extern "C" int lmoe_rmsnorm_fwd_typed(const void* x, int x_type, const void* weight, int w_type, float eps, int64_t T, int D,
-                                      void* xn, int xn_type, float* rstd, void* stream) {
+extern "C" int lmoe_rmsnorm_fwd_keep(const void* x, int x_type, const void* weight, int w_type, float eps, int64_t T, int D,
+                                     void* xn, int xn_type, float* rstd, void* x_keep, float* w_keep, void* stream) {
   if (!x || !weight || !xn || !rstd || !is_type(x_type) || !is_type(w_type) || !is_type(xn_type)) return LMOE_ERR_ARG;
   if (!norm_dims_ok(T, D)) return LMOE_ERR_SHAPE;
-  if (!aligned16(x) || !aligned16(xn) || !aligned16(weight)) return LMOE_ERR_ALIGN;
+  if (!aligned16(x) || !aligned16(xn) || !aligned16(weight) || !aligned16(x_keep) || !aligned16(w_keep)) return LMOE_ERR_ALIGN;
   auto pick = [&](auto narrow, auto wide) { return D <= 1024 ? narrow : wide; };
   auto k = x_type == LMOE_BF16 ? (xn_type == LMOE_BF16 ? pick(rmsnorm_fwd_kernel<false, false, 4>, rmsnorm_fwd_kernel<false, false, 8>)
                                                        : pick(rmsnorm_fwd_kernel<false, true, 4>, rmsnorm_fwd_kernel<false, true, 8>))
@@ -315,8 +326,13 @@ extern "C" int lmoe_rmsnorm_fwd_typed(const void* x, int x_type, const void* wei
   long long blocks = (T + kNormWarps - 1) / kNormWarps;   // no per-block result here: a warp per row up to 16 blocks per SM
   if (blocks > 148 * 16) blocks = 148 * 16;
   k<<<static_cast<int>(blocks), kNormWarps * 32, 0, static_cast<cudaStream_t>(stream)>>>(x, weight, w_type == LMOE_F32, eps, T, D / 8, xn,
-                                                                                        rstd);
+                                                                                        rstd, x_keep, w_keep);
   return norm_last_error();
+}
+
+extern "C" int lmoe_rmsnorm_fwd_typed(const void* x, int x_type, const void* weight, int w_type, float eps, int64_t T, int D,
+                                      void* xn, int xn_type, float* rstd, void* stream) {
+  return lmoe_rmsnorm_fwd_keep(x, x_type, weight, w_type, eps, T, D, xn, xn_type, rstd, nullptr, nullptr, stream);
 }
 
 extern "C" int lmoe_rmsnorm_fwd(const void* x, const float* weight, float eps, int64_t T, int D, void* xn, float* rstd,
@@ -344,21 +360,27 @@ extern "C" int lmoe_add_f32_bf16(const float* a, const void* b, float* out, int6
   return norm_last_error();
 }
 
-extern "C" int lmoe_rmsnorm_bwd_typed(const void* x, int x_type, const void* weight, int w_type, const float* rstd,
-                                      const void* d_xn, int g_type, const void* d_residual, int64_t T, int D, void* dx,
-                                      void* d_weight, int dw_type, void* workspace, size_t workspace_bytes, void* stream) {
+static int rmsnorm_bwd(const void* x, int x_type, const void* weight, int w_type, const float* rstd, const void* d_xn, int g_type,
+                       const void* d_residual, int s_type, int64_t T, int D, void* dx, void* d_weight, int dw_type,
+                       void* workspace, size_t workspace_bytes, void* stream) {
   if (!x || !weight || !rstd || !d_xn || !dx || !d_weight || !workspace) return LMOE_ERR_ARG;
-  if (!is_type(x_type) || !is_type(w_type) || !is_type(g_type) || !is_type(dw_type)) return LMOE_ERR_ARG;
+  if (!is_type(x_type) || !is_type(w_type) || !is_type(g_type) || !is_type(s_type) || !is_type(dw_type)) return LMOE_ERR_ARG;
+  if (x_type == LMOE_F32 && s_type != LMOE_F32) return LMOE_ERR_ARG;
   if (!norm_dims_ok(T, D)) return LMOE_ERR_SHAPE;
   if (workspace_bytes < lmoe_rmsnorm_workspace_bytes(D)) return LMOE_ERR_WORKSPACE;
   if (!aligned16(x) || !aligned16(d_xn) || !aligned16(dx) || !aligned16(weight) || (d_residual && !aligned16(d_residual)))
     return LMOE_ERR_ALIGN;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   auto pick = [&](auto narrow, auto wide) { return D <= 1024 ? narrow : wide; };
-  auto k = x_type == LMOE_BF16 ? (g_type == LMOE_BF16 ? pick(rmsnorm_bwd_kernel<false, false, 4>, rmsnorm_bwd_kernel<false, false, 8>)
-                                                      : pick(rmsnorm_bwd_kernel<false, true, 4>, rmsnorm_bwd_kernel<false, true, 8>))
-                               : (g_type == LMOE_BF16 ? pick(rmsnorm_bwd_kernel<true, false, 4>, rmsnorm_bwd_kernel<true, false, 8>)
-                                                      : pick(rmsnorm_bwd_kernel<true, true, 4>, rmsnorm_bwd_kernel<true, true, 8>));
+  const bool g32 = g_type == LMOE_F32;
+  auto k = s_type == LMOE_BF16
+               ? (g32 ? pick(rmsnorm_bwd_kernel<false, false, true, 4>, rmsnorm_bwd_kernel<false, false, true, 8>)
+                      : pick(rmsnorm_bwd_kernel<false, false, false, 4>, rmsnorm_bwd_kernel<false, false, false, 8>))
+               : x_type == LMOE_BF16
+                     ? (g32 ? pick(rmsnorm_bwd_kernel<false, true, true, 4>, rmsnorm_bwd_kernel<false, true, true, 8>)
+                            : pick(rmsnorm_bwd_kernel<false, true, false, 4>, rmsnorm_bwd_kernel<false, true, false, 8>))
+                     : (g32 ? pick(rmsnorm_bwd_kernel<true, true, true, 4>, rmsnorm_bwd_kernel<true, true, true, 8>)
+                            : pick(rmsnorm_bwd_kernel<true, true, false, 4>, rmsnorm_bwd_kernel<true, true, false, 8>));
   const size_t smem = static_cast<size_t>(kNormWarps) * D * sizeof(float);   // up to 64 KB
   if (smem > 48 * 1024) {
     const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
@@ -371,6 +393,20 @@ extern "C" int lmoe_rmsnorm_bwd_typed(const void* x, int x_type, const void* wei
   rmsnorm_dw_finalize_kernel<<<(D + 31) / 32, kNormWarps * 32, 0, st>>>(static_cast<const float*>(workspace), blocks, D, d_weight,
                                                                        dw_type == LMOE_F32);
   return norm_last_error();
+}
+
+extern "C" int lmoe_rmsnorm_bwd_typed(const void* x, int x_type, const void* weight, int w_type, const float* rstd,
+                                      const void* d_xn, int g_type, const void* d_residual, int64_t T, int D, void* dx,
+                                      void* d_weight, int dw_type, void* workspace, size_t workspace_bytes, void* stream) {
+  return rmsnorm_bwd(x, x_type, weight, w_type, rstd, d_xn, g_type, d_residual, x_type, T, D, dx, d_weight, dw_type, workspace,
+                     workspace_bytes, stream);
+}
+
+extern "C" int lmoe_rmsnorm_bwd_kept(const void* x_bf16, const void* weight, int w_type, const float* rstd, const void* d_xn,
+                                     int g_type, const void* d_residual, int s_type, int64_t T, int D, void* dx, void* d_weight,
+                                     int dw_type, void* workspace, size_t workspace_bytes, void* stream) {
+  return rmsnorm_bwd(x_bf16, LMOE_BF16, weight, w_type, rstd, d_xn, g_type, d_residual, s_type, T, D, dx, d_weight, dw_type,
+                     workspace, workspace_bytes, stream);
 }
 
 extern "C" int lmoe_rmsnorm_bwd(const void* x, const float* weight, const float* rstd, const void* d_xn,

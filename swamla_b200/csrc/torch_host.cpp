@@ -910,21 +910,28 @@ Tensor weight_of(const Tensor& t) {
 }
 
 // (xn, x_pass) = (rmsnorm(x) * weight, x).  x_pass is x itself, handed on to the residual add, so that the backward sees the
-// gradients of both branches in one call and adds them inside the norm's adjoint.
+// gradients of both branches in one call and adds them inside the norm's adjoint.  `keep`: a backward may follow; it reads
+// copies that the norm's kernel wrote (an fp32 stream's rows as the norm saw them, a bf16 weight in fp32), so that either may be
+// changed in place in between.  What is bf16 rows or an fp32 weight is kept as it is, under autograd's check.
 class NormFn : public torch::autograd::Function<NormFn> {
  public:
-  static variable_list forward(AutogradContext* ctx, const Tensor& x, const Tensor& weight, double eps, bool bf16_out) {
+  static variable_list forward(AutogradContext* ctx, const Tensor& x, const Tensor& weight, double eps, bool bf16_out, bool keep) {
     const Tensor xr = rows_of(x), w = weight_of(weight);
     TORCH_CHECK(x.dim() > 0 && weight.numel() == x.size(-1), "the norm's weight has another width than its input");
     const int64_t D = x.size(-1), T = xr.numel() / D;
     const bool wide = !bf16_out && xr.scalar_type() == at::kFloat;
     Tensor xn = at::empty(x.sizes(), xr.options().dtype(wide ? at::kFloat : at::kBFloat16));
     Tensor rstd = at::empty({T}, xr.options().dtype(at::kFloat));
-    LMOE(lmoe_rmsnorm_fwd_typed, xr.data_ptr(), lmoe_type(xr), w.data_ptr(), lmoe_type(w), static_cast<float>(eps), T, static_cast<int>(D),
-         xn.data_ptr(), lmoe_type(xn), rstd.data_ptr<float>(), at::cuda::getCurrentCUDAStream().stream());
+    Tensor x_keep, w_keep;
+    if (keep && xr.scalar_type() == at::kFloat) x_keep = at::empty(xr.sizes(), xr.options().dtype(at::kBFloat16));
+    if (keep && w.scalar_type() == at::kBFloat16) w_keep = at::empty({D}, w.options().dtype(at::kFloat));
+    LMOE(lmoe_rmsnorm_fwd_keep, xr.data_ptr(), lmoe_type(xr), w.data_ptr(), lmoe_type(w), static_cast<float>(eps), T, static_cast<int>(D),
+         xn.data_ptr(), lmoe_type(xn), rstd.data_ptr<float>(), x_keep.defined() ? x_keep.data_ptr() : nullptr,
+         w_keep.defined() ? w_keep.data_ptr<float>() : nullptr, at::cuda::getCurrentCUDAStream().stream());
     ctx->set_materialize_grads(false);
-    ctx->save_for_backward({xr, w, rstd});
+    ctx->save_for_backward({x_keep.defined() ? x_keep : xr, w_keep.defined() ? w_keep : w, rstd});
     ctx->saved_data["t"] = dtypes_of({x, weight});
+    ctx->saved_data["s"] = std::vector<int64_t>{static_cast<int64_t>(xr.scalar_type()), static_cast<int64_t>(w.scalar_type())};
     return {bf16_out ? xn : as_param(xn, x.scalar_type()), x};
   }
 
@@ -935,18 +942,20 @@ class NormFn : public torch::autograd::Function<NormFn> {
       const c10::cuda::CUDAGuard guard(x.device());
       const auto t = ctx->saved_data["t"].toIntVector();
       const auto x_type = static_cast<at::ScalarType>(t[0]), w_type = static_cast<at::ScalarType>(t[1]);
+      const auto s = ctx->saved_data["s"].toIntVector();  // the types that the forward's kernel took
+      const auto stream_type = static_cast<at::ScalarType>(s[0]), dw_type = static_cast<at::ScalarType>(s[1]);
       const int64_t D = x.size(-1), T = x.numel() / D;
       const Tensor g = grads[0].defined() ? rows_of(grads[0]) : at::zeros_like(x);
       Tensor r;
-      if (grads[1].defined()) r = rows_of(grads[1]).to(x.scalar_type()).contiguous();
-      Tensor dx = at::empty_like(x);
-      Tensor dw = at::empty({D}, x.options().dtype(w.scalar_type()));
+      if (grads[1].defined()) r = rows_of(grads[1]).to(stream_type).contiguous();
+      Tensor dx = at::empty(x.sizes(), x.options().dtype(stream_type));
+      Tensor dw = at::empty({D}, x.options().dtype(dw_type));
       Tensor ws = new_bytes(lmoe_rmsnorm_workspace_bytes(static_cast<int>(D)), x);
-      LMOE(lmoe_rmsnorm_bwd_typed, x.data_ptr(), lmoe_type(x), w.data_ptr(), lmoe_type(w), rstd.data_ptr<float>(), g.data_ptr(),
-           lmoe_type(g), r.defined() ? r.data_ptr() : nullptr, T, static_cast<int>(D), dx.data_ptr(), dw.data_ptr(), lmoe_type(dw),
+      LMOE(lmoe_rmsnorm_bwd_kept, x.data_ptr(), w.data_ptr(), lmoe_type(w), rstd.data_ptr<float>(), g.data_ptr(), lmoe_type(g),
+           r.defined() ? r.data_ptr() : nullptr, lmoe_type(dx), T, static_cast<int>(D), dx.data_ptr(), dw.data_ptr(), lmoe_type(dw),
            ws.data_ptr(), static_cast<size_t>(ws.numel()), at::cuda::getCurrentCUDAStream().stream());
       const Tensor none;
-      return {as_param(dx, x_type), as_param(dw, w_type), none, none};
+      return {as_param(dx, x_type), as_param(dw, w_type), none, none, none};
     } catch (const LmoeFailure& e) {
       rethrow_as_python(e);
     }
@@ -1040,7 +1049,7 @@ std::vector<Tensor> moe(const Tensor& x, const Tensor& wg, const Tensor& wgus, c
 std::vector<Tensor> norm_and_pass(const Tensor& x, const Tensor& weight, double eps, bool bf16_out) {
   require_cuda(x, "fused norm");
   const c10::cuda::CUDAGuard guard(x.device());
-  return NormFn::apply(x, weight, eps, bf16_out);
+  return NormFn::apply(x, weight, eps, bf16_out, any_grad({&x, &weight}));
 }
 Tensor residual_add(const Tensor& a, const Tensor& b_in) {
   const c10::cuda::CUDAGuard guard(a.device());

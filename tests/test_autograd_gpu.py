@@ -88,3 +88,34 @@ def test_block_takes_flattened_and_broadcast_branches():
             want, want_grad = y.detach(), xg.grad
     assert torch.equal(y, want) and torch.equal(xg.grad, want_grad)
     assert torch.equal(one(x), x + 1.0)
+
+
+@pytest.mark.parametrize("what", ["stream", "bf16 weight"])
+@pytest.mark.parametrize("width", [256, 2048])
+def test_block_s_inputs_may_change_before_the_backward(what, width):
+    """An fp32 stream (the norm keeps its rows in bf16) and a bf16 norm weight (kept in fp32) changed in place between the two
+    directions: the gradients are those of the values that the forward saw."""
+    from swamla_b200.block import NormedResidualFFN
+    torch.manual_seed(5)
+    m = NormedResidualFFN(torch.nn.Linear(width, width), width).cuda()
+    with torch.no_grad():
+        m.ffn_norm.weight.normal_(1.0, 0.1)
+    if what == "bf16 weight":
+        m.ffn_norm.to(torch.bfloat16)
+    x = torch.randn(3, 37, width, device="cuda:0")
+    dy = torch.randn_like(x)
+    got = []
+    for change in (False, True):
+        m.zero_grad()
+        leaf = x.clone().requires_grad_(True)
+        h = 1.0 * leaf
+        kept = m.ffn_norm.weight.detach().clone()
+        y = m(h)
+        if change:
+            with torch.no_grad():
+                (h if what == "stream" else m.ffn_norm.weight).mul_(3.0)
+        y.backward(dy)
+        with torch.no_grad():
+            m.ffn_norm.weight.copy_(kept)
+        got.append((leaf.grad, m.ffn_norm.weight.grad.clone()))
+    assert all(torch.equal(a, b) for a, b in zip(*got))
