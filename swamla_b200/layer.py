@@ -376,13 +376,14 @@ class MoELayer(nn.Module):
     def forward(self, x: torch.Tensor) -> torch.Tensor:
         moe = functional_moe.moe_opaque if torch.compiler.is_compiling() else functional_moe.moe
         status_monitor.poll()
+        batch_size, seq_len, _d_model = x.shape
         w_gate_up_s, w_down_s = _merged_shared_weights(self.shared_experts)
         out = moe(x, self.router.gate.weight, w_gate_up_s, w_down_s, self.experts.gate_up_weight, self.experts.down_weight,
                   self.router.expert_bias, self.n_activated, self.router.z_loss_coef, not self.training)
         y, self.aux_loss = out[0], out[1]                                 # moe.py:358
         if self.training:                                                 # moe.py:237-240
             self.router._last_selected_experts, self.router._last_counts = out[2], out[3]
-            self.router._last_num_tokens = x.shape[0] * x.shape[1]
+            self.router._last_num_tokens = batch_size * seq_len
             if self.dropout.p > 0.0:
                 y = self.dropout(y)                                       # moe.py:367
         return y
