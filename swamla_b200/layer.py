@@ -9,6 +9,7 @@ from __future__ import annotations
 
 import torch
 import torch.nn as nn
+from torch.nn.modules.module import _has_any_global_hook
 
 from . import _cabi, functional_moe, status as status_monitor
 from .functional import latent_moe, latent_moe_opaque, make_shape, _host, _stream
@@ -159,6 +160,16 @@ def _merged_shared_weights(shared_experts):
     return gate_up, down
 
 
+def _hooked(m: nn.Module) -> bool:
+    return bool(m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks or _has_any_global_hook())
+
+
+def _drops(d: nn.Module) -> bool:
+    """Whether a layer's dropout module has anything to do: a plain, unhooked dropout of rate 0 or in evaluation mode has not, and
+    calling it costs a small step a few microseconds.  Its own mode counts: it may be left active in an evaluated layer."""
+    return (d.p > 0.0 and d.training) or _hooked(d) if type(d) is nn.Dropout else True
+
+
 class LatentMoELayer(nn.Module):
     """LatentMoE feed-forward layer; see the module docstring.  ``models/moe.py:603-866``."""
 
@@ -269,9 +280,8 @@ class LatentMoELayer(nn.Module):
             if training:
                 router._last_selected_experts, router._last_counts = out[2], out[3]
                 router._last_num_tokens = batch_size * seq_len
-                if self.dropout.p > 0.0:
-                    y = self.dropout(y)
-            return y
+            dropout = self._modules["dropout"]
+            return dropout(y) if _drops(dropout) else y                   # moe.py:732
         x_flat = x.reshape(-1, d_model)
         args = (x_flat, *self._arguments(), self.n_activated, router.z_loss_coef)
         if self.ep_size > 1 and self.ep_mode == "p2p_dedup":
@@ -374,7 +384,8 @@ class MoELayer(nn.Module):
         status_monitor.poll(block=True)
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
-        moe = functional_moe.moe_opaque if torch.compiler.is_compiling() else functional_moe.moe
+        compiling = torch.compiler.is_compiling()
+        moe = functional_moe.moe_opaque if compiling else functional_moe.moe
         status_monitor.poll()
         batch_size, seq_len, _d_model = x.shape
         w_gate_up_s, w_down_s = _merged_shared_weights(self.shared_experts)
@@ -384,9 +395,7 @@ class MoELayer(nn.Module):
         if self.training:                                                 # moe.py:237-240
             self.router._last_selected_experts, self.router._last_counts = out[2], out[3]
             self.router._last_num_tokens = batch_size * seq_len
-            if self.dropout.p > 0.0:
-                y = self.dropout(y)                                       # moe.py:367
-        return y
+        return self.dropout(y) if compiling or _drops(self.dropout) else y    # moe.py:367
 
     def get_aux_loss(self) -> torch.Tensor:
         return self.aux_loss

@@ -25,3 +25,35 @@ def test_other_ranks_of_input_are_refused(kind):
         for m in (layer.train(), layer.eval()):
             with torch.no_grad(), pytest.raises(ValueError):
                 m(bad)
+
+
+@pytest.mark.parametrize("tokens", [1, 50])                            # the few-token path and the padded one
+@pytest.mark.parametrize("kind", KINDS)
+def test_dropout_follows_its_own_mode(kind, tokens):
+    layer, x = _layer(kind, 0.5)
+    x = x[:, :tokens]
+    with torch.no_grad():
+        plain = layer.eval()(x)
+        layer.dropout.train()                                          # left active in an evaluated layer
+        y = layer(x)
+        zero = (y == 0) & (plain != 0)
+        assert 0.3 < zero.float().mean().item() < 0.7
+        assert torch.equal(y[~zero], 2.0 * plain[~zero])
+        layer.train().dropout.eval()                                   # and the other way round
+        assert (layer(x) != 0).float().mean().item() > 0.99
+
+
+@pytest.mark.parametrize("kind", KINDS)
+def test_dropout_may_be_replaced_or_hooked(kind):
+    from swamla_b200.block import NormedResidualFFN
+    layer, x = _layer(kind)
+    seen = []
+    handle = layer.dropout.register_forward_hook(lambda m, a, out: seen.append(out.shape))
+    with torch.no_grad():
+        want = layer.train()(x)
+        layer.eval()(x)
+        handle.remove()
+        assert len(seen) == 2
+        layer.dropout = torch.nn.Identity()
+        assert torch.equal(layer.train()(x), want)
+        NormedResidualFFN(layer, x.shape[-1]).cuda()(x)
