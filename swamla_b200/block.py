@@ -14,7 +14,7 @@ import torch
 import torch.nn as nn
 
 from .functional import _host
-from .layer import LatentMoELayer, MoELayer
+from .layer import LatentMoELayer, MoELayer, _drops, _hooked
 
 
 class _NormAndPass:
@@ -51,12 +51,16 @@ class NormedResidualFFN(nn.Module):
         if torch.compiler.is_compiling():
             xn, x_pass = _norm_opaque(x, norm.weight, norm.eps)
             return _add_opaque(x_pass, ffn(xn))
-        # this package's own layers compute in bf16 whatever they are given: hand them bf16 and take bf16 back, instead of a
-        # widened copy each way (an active dropout keeps the stream's precision)
-        narrow = type(ffn) in (LatentMoELayer, MoELayer) and not (ffn.training and ffn.dropout.p > 0.0)
         host = _host()
-        xn, x_pass = host.norm_and_pass(x, norm.weight, norm.eps, narrow)
+        xn, x_pass = host.norm_and_pass(x, norm.weight, norm.eps, _takes_bf16(ffn))
         return host.residual_add(x_pass, ffn(xn))
+
+
+def _takes_bf16(ffn) -> bool:
+    """Whether the feed-forward module is handed bf16 and gives bf16 back, instead of a widened copy each way: this package's
+    own layers compute in bf16 whatever they are given.  Not where something else sees or changes the tensors in the stream's
+    precision: an active dropout, a hook, a replaced ``forward``."""
+    return type(ffn) in (LatentMoELayer, MoELayer) and "forward" not in ffn.__dict__ and not _hooked(ffn) and not _drops(ffn.dropout)
 
 
 # opaque to torch.compile (calls into the kernel library); the feed-forward module between them is compiled

@@ -57,3 +57,41 @@ def test_dropout_may_be_replaced_or_hooked(kind):
         layer.dropout = torch.nn.Identity()
         assert torch.equal(layer.train()(x), want)
         NormedResidualFFN(layer, x.shape[-1]).cuda()(x)
+
+
+@pytest.mark.parametrize("how", ["forward hook", "pre-hook", "global hook", "forward"])
+@pytest.mark.parametrize("kind", KINDS)
+def test_whoever_looks_at_the_feed_forward_module_sees_the_stream_s_precision(kind, how):
+    from swamla_b200.block import NormedResidualFFN
+    layer, x = _layer(kind)
+    block, x = NormedResidualFFN(layer, x.shape[-1]).cuda(), x.float()
+    with torch.no_grad():
+        plain = block(x)
+    seen = []
+    add = 2.0 ** -13                                                   # lost if the branch were rounded to bf16 after it
+
+    def hook(m, args, out):
+        if m is layer:
+            seen.extend([args[0].dtype, out.dtype])
+            return out + add
+
+    if how == "forward hook":
+        handle = layer.register_forward_hook(hook)
+    elif how == "pre-hook":
+        handle = layer.register_forward_pre_hook(lambda m, args: seen.append(args[0].dtype))
+    elif how == "global hook":
+        handle = torch.nn.modules.module.register_module_forward_hook(hook)
+    else:
+        inner = layer.forward
+        layer.forward = lambda t: hook(layer, (t,), inner(t))
+    try:
+        with torch.no_grad():
+            y = block(x)
+    finally:
+        if how != "forward":
+            handle.remove()
+    assert seen and set(seen) == {torch.float32}
+    if how != "pre-hook":
+        assert ((y - plain) - add).abs().max().item() <= 2.0 ** -21   # fp32 roundings of values of a few units
+    else:
+        assert torch.equal(y, plain)
