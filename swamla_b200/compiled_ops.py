@@ -3,8 +3,10 @@ layer (the reference compiles the whole model by default, ``train.py:936-942``).
 
 Two opaque operators, ``swamla_b200::latent_moe_fwd`` and ``swamla_b200::latent_moe_bwd``, each with a fake (shape-only)
 implementation for tracing, tied together with ``register_autograd``.  Their real implementations are the two directions
-of the native host path that the eager call runs too, so compiled and eager execution launch the same kernels and give the
-same bits.
+of the native host path that the eager call runs too.  A third, ``swamla_b200::latent_moe_eval``, is the evaluated layer
+without gradients, whose eager call may take the few-token kernels and keeps nothing for a backward.  So compiled and eager
+execution give the same bits in every mode, and launch the same kernels but for a training-mode forward without gradients,
+which keeps what a backward would read.
 
 An operator's outputs may alias neither its inputs nor one another, so the forward operator returns only tensors it
 creates (what the backward needs travels as one allocation) and the backward operator takes the layer's inputs
@@ -81,6 +83,24 @@ def _backward(ctx, *grads):
 
 
 latent_moe_fwd.register_autograd(_backward, setup_context=_setup_context)
+
+
+@torch.library.custom_op("swamla_b200::latent_moe_eval", mutates_args=())
+def latent_moe_eval(x: Tensor, w_gate: Tensor, w_down: Tensor, w_up: Tensor, w_gate_up_s: Tensor, w_down_s: Tensor,
+                    w_gate_up: Tensor, w_down_e: Tensor, expert_bias: Tensor, top_k: int, z_coef: float) -> Tuple[Tensor, Tensor]:
+    out = Fn._host().latent_moe(x, w_gate, w_down, w_up, w_gate_up_s, w_down_s, w_gate_up, w_down_e, expert_bias, top_k, z_coef,
+                                False, True)
+    return out[0], out[1]
+
+
+@latent_moe_eval.register_fake
+def _(x, w_gate, w_down, w_up, w_gate_up_s, w_down_s, w_gate_up, w_down_e, expert_bias, top_k, z_coef):
+    return x.new_empty(x.shape), x.new_empty((), dtype=torch.float32)
+
+
+def latent_moe_eval_compiled(x2d, *args):
+    """(y, aux_loss) of an evaluated layer without gradients; arguments of ``latent_moe_compiled``."""
+    return torch.ops.swamla_b200.latent_moe_eval(x2d, *args)
 
 
 def latent_moe_compiled(x2d, w_gate, w_down, w_up, w_gate_up_s, w_down_s, w_gate_up, w_down_e, expert_bias, top_k: int,

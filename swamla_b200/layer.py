@@ -13,7 +13,7 @@ from torch.nn.modules.module import _has_any_global_hook
 
 from . import _cabi, functional_moe, status as status_monitor
 from .functional import latent_moe, latent_moe_opaque, make_shape, _host, _stream
-from .compiled_ops import latent_moe_compiled
+from .compiled_ops import latent_moe_compiled, latent_moe_eval_compiled
 
 
 def _ep_size(group) -> int:
@@ -305,8 +305,12 @@ class LatentMoELayer(nn.Module):
             y, z_loss, sel, counts = latent_moe_ep(*args, self.ep_group)   # counts: load summed over all ranks
         elif compiling and not self.fp8_experts:
             # torch.compile (the reference's default, train.py:936-942): custom operators with fake implementations
-            # keep one graph across the layer; they run the same kernels as the eager call below
-            y, z_loss, sel, counts = latent_moe_compiled(*args)
+            # keep one graph across the layer, with the bits of the eager call
+            grad = torch.is_grad_enabled() and any(t.requires_grad for t in args[:8])
+            if self.training or grad:
+                y, z_loss, sel, counts = latent_moe_compiled(*args)
+            else:
+                y, z_loss = latent_moe_eval_compiled(*args)
         else:
             y, z_loss, sel, counts = (latent_moe_opaque if compiling else latent_moe)(*args, fp8=self.fp8_experts)
         self.aux_loss = z_loss                                            # moe.py:719
