@@ -295,7 +295,7 @@ struct LatentLayout {
   }
 };
 // scal: [amax, amax / 448] per quantised tensor
-enum Scal : int { kSx = 0, kSwgu = 1, kSwd = 2, kSh = 3, kSdy = 4, kSdh1 = 5 };
+enum Scal : int { kSx = 0, kSwgu = 1, kSwd = 2, kSh = 3, kSdy = 4, kSdh1 = 5, kScals = 6 };
 float* amax_of(float* scal, Scal k) { return scal + 2 * k; }
 float* deq_of(float* scal, Scal k) { return scal + 2 * k + 1; }
 
@@ -496,10 +496,13 @@ LatentGrads latent_backward(const Sizes& d, const LatentOps& o, const Tensor& dy
   const size_t t_dw = c.take(T * d.K * 4), t_dys = c.take(P * d.L * (fp8 ? 1 : 2)), t_dh1 = c.take(P * 2 * d.F * 2);
   const size_t t_dxs = c.take(P * d.L * 2);
   const size_t t_dh1q = fp8 ? c.take(P * 2 * d.F) : 0;
-  float* scal = fp8 ? reinterpret_cast<float*>(static_cast<char*>(saved.data_ptr()) + at_.scal) : nullptr;
-  if (fp8) C10_CUDA_CHECK(cudaMemsetAsync(amax_of(scal, kSdy), 0, 4 * sizeof(float), stream.stream()));
+  const size_t t_scal = fp8 ? c.take(kScals * 2 * sizeof(float)) : 0;
   Tensor tmp = new_bytes(c.bytes, o.x);
   char *tv = base_of(tmp), *sv = base_of(saved);
+  // the forward's scales are read; the backward's own are scratch (what is saved may be read by another backward at the time)
+  float* scal = fp8 ? reinterpret_cast<float*>(sv + at_.scal) : nullptr;
+  float* d_scal = fp8 ? reinterpret_cast<float*>(tv + t_scal) : nullptr;
+  if (fp8) C10_CUDA_CHECK(cudaMemsetAsync(d_scal, 0, kScals * 2 * sizeof(float), stream.stream()));
 
   float* logits = reinterpret_cast<float*>(sv + at_.logits);
   float* weights = reinterpret_cast<float*>(sv + at_.weights);
@@ -518,7 +521,7 @@ LatentGrads latent_backward(const Sizes& d, const LatentOps& o, const Tensor& dy
        status, st);
   fork.to_side();
   if (fp8)
-    LMOE(lmoe_fp8_combine_bwd, &d.s, d_routed, y_sorted, weights, &route, amax_of(scal, kSdy), deq_of(scal, kSdy), d_ys, d_w, side);
+    LMOE(lmoe_fp8_combine_bwd, &d.s, d_routed, y_sorted, weights, &route, amax_of(d_scal, kSdy), deq_of(d_scal, kSdy), d_ys, d_w, side);
   else
     LMOE(lmoe_combine_bwd, &d.s, d_routed, y_sorted, weights, &route, d_ys, d_w, side);
   LMOE(lmoe_combine_out_bwd_wgrad, &d.s, dy.data_ptr(), act_cat, g.wup.data_ptr(), g.wds.data_ptr(), gtype, ws, ws_bytes,
@@ -528,19 +531,19 @@ LatentGrads latent_backward(const Sizes& d, const LatentOps& o, const Tensor& dy
   if (fp8) {
     void *xq = sv + at_.xq, *hq = sv + at_.hq, *wguq = sv + at_.wguq, *wdq = sv + at_.wdq, *dyq = d_ys, *dh1q = tv + t_dh1q;
     // d_h1 = swiglu'(h1, d_y * Wd[e]^T): the down weights [E, F, L] read as [N = F rows, K = L] (K-major operand)
-    LMOE(lmoe_grouped_swiglu_bwd_fp8, P, d.E, d.L, d.F, dyq, wdq, deq_of(scal, kSdy), deq_of(scal, kSwd), route.tile_expert,
-         route.n_tiles, h1, d_h1, amax_of(scal, kSdh1), status, st);
-    const lmoe_fp8_tensor h = {d_h1, dh1q, P, 2 * d.F, route.n_tiles, amax_of(scal, kSdh1), deq_of(scal, kSdh1)};
+    LMOE(lmoe_grouped_swiglu_bwd_fp8, P, d.E, d.L, d.F, dyq, wdq, deq_of(d_scal, kSdy), deq_of(scal, kSwd), route.tile_expert,
+         route.n_tiles, h1, d_h1, amax_of(d_scal, kSdh1), status, st);
+    const lmoe_fp8_tensor h = {d_h1, dh1q, P, 2 * d.F, route.n_tiles, amax_of(d_scal, kSdh1), deq_of(d_scal, kSdh1)};
     LMOE(lmoe_fp8_cast, 1, &h, st);
     // d_x_sorted = d_h1 * Wgu[e]^T: the gate_up weights [E, L, 2F] read as [N = L rows, K = 2F]
-    LMOE(lmoe_grouped_rows_fp8, P, d.E, 2 * d.F, d.L, dh1q, wguq, 0, deq_of(scal, kSdh1), deq_of(scal, kSwgu),
+    LMOE(lmoe_grouped_rows_fp8, P, d.E, 2 * d.F, d.L, dh1q, wguq, 0, deq_of(d_scal, kSdh1), deq_of(scal, kSwgu),
          route.tile_expert, route.n_tiles, d_xs, status, st);
     fork.to_side();
     LMOE(lmoe_unpermute_sum_bwd, &d.s, d_xs, &route, cat, side);
     LMOE(lmoe_gate_topk_bwd, &d.s, logits, sel, weights, d_w, lse, dz, z_coef, cat, side);
-    LMOE(lmoe_grouped_wgrad_fp8, P, d.E, d.L, 2 * d.F, xq, dh1q, deq_of(scal, kSx), deq_of(scal, kSdh1), route.pad_offsets,
+    LMOE(lmoe_grouped_wgrad_fp8, P, d.E, d.L, 2 * d.F, xq, dh1q, deq_of(scal, kSx), deq_of(d_scal, kSdh1), route.pad_offsets,
          g.wgu.data_ptr(), status, st);
-    LMOE(lmoe_grouped_wgrad_fp8, P, d.E, d.F, d.L, hq, dyq, deq_of(scal, kSh), deq_of(scal, kSdy), route.pad_offsets,
+    LMOE(lmoe_grouped_wgrad_fp8, P, d.E, d.F, d.L, hq, dyq, deq_of(scal, kSh), deq_of(d_scal, kSdy), route.pad_offsets,
          g.wde.data_ptr(), status, st);
     fork.to_main();
   } else {

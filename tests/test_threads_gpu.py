@@ -121,3 +121,17 @@ def test_a_failure_names_its_device_and_is_reported_once():
         m.check_status()
     m.check_status()
     m(xs[0])
+
+
+@pytest.mark.parametrize("kind", ["latent", "fp8", "moe"])
+def test_a_backward_leaves_what_the_forward_saved_as_it_is(kind):
+    """Another backward of the same graph may read it at the same time; a second one gives the first one's bits."""
+    m, xs = _module(kind, 1)
+    x = xs[2].clone().requires_grad_(True)
+    saved = []
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: saved.append(t) or t, lambda t: t):
+        y = m(x)
+    before = [t.clone() for t in saved]
+    grads = [torch.autograd.grad(y, [x, *m.parameters()], torch.ones_like(y), retain_graph=True, allow_unused=True) for _ in range(2)]
+    assert saved and all(torch.equal(a, b) for a, b in zip(saved, before))
+    assert all(a is b or torch.equal(a, b) for a, b in zip(*grads))
