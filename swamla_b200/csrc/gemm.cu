@@ -25,6 +25,14 @@ typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t,
                                   CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 
 static EncodeTiledFn encode_fn() {
+  // The driver encodes a map for the calling thread's current context.  A thread that has made no runtime call that needs
+  // one (an autograd thread whose buffers all came from PyTorch's cache) has none yet: cudaSetDevice makes it current, also
+  // while a stream is being captured.
+  thread_local bool bound = false;
+  if (!bound) {
+    int dev = 0;
+    bound = cudaGetDevice(&dev) == cudaSuccess && cudaSetDevice(dev) == cudaSuccess;
+  }
   static EncodeTiledFn fn = nullptr;
   static std::once_flag once;
   std::call_once(once, [] {

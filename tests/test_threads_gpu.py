@@ -135,3 +135,35 @@ def test_a_backward_leaves_what_the_forward_saved_as_it_is(kind):
     grads = [torch.autograd.grad(y, [x, *m.parameters()], torch.ones_like(y), retain_graph=True, allow_unused=True) for _ in range(2)]
     assert saved and all(torch.equal(a, b) for a, b in zip(saved, before))
     assert all(a is b or torch.equal(a, b) for a, b in zip(*grads))
+
+
+@pytest.mark.parametrize("kind", ["latent", "fp8", "moe", "block", "backward"])
+def test_first_call_of_a_thread(kind):
+    """A thread whose first CUDA call is the layer's, with every buffer from PyTorch's cache, has no current context before it."""
+    from swamla_b200 import functional
+    m, xs = _module("latent" if kind == "backward" else kind, 0)
+    x = xs[3].repeat(1, 2, 1)                                           # 2,800 tokens: nothing goes to the side stream first
+    args = (*m._arguments(), m.n_activated, 1e-3, False) if kind == "backward" else None
+    with torch.no_grad():
+        if kind == "backward":
+            fwd = functional._host().latent_fwd_raw(x, *args, None, False)
+            call = lambda: functional._host().latent_bwd_raw(fwd[0], None, x, *args[:7], fwd[2], fwd[4], *args[8:], False)[0][0]
+        else:
+            call = lambda: m(x)
+        want = call()
+        call()                                                         # (its buffers go back to the cache)
+    torch.cuda.synchronize()
+    got = []
+
+    def work():
+        torch.set_grad_enabled(False)
+        try:
+            got.append(call())
+        except Exception as e:                                           # pragma: no cover
+            got.append(e)
+
+    t = threading.Thread(target=work)
+    t.start()
+    t.join()
+    assert isinstance(got[0], torch.Tensor), got[0]
+    assert torch.equal(got[0], want)
