@@ -18,6 +18,7 @@ CSRC = os.path.join(HERE, "csrc")
 OBJ = os.path.join(CSRC, "_obj")
 LIB = os.path.join(HERE, "liblmoe.so")
 HOST = os.path.join(HERE, "_host.so")
+HOST_STAMP = os.path.join(OBJ, "host_stamp.txt")
 INCLUDE = os.path.join(os.path.dirname(HERE), "include")
 
 NVCC_FLAGS = [
@@ -49,6 +50,20 @@ def _deps_mtime() -> float:
     return latest
 
 
+def _host_versions() -> str:
+    """What ``_host.so`` is bound to besides its sources."""
+    from importlib.metadata import version
+    return f"torch {version('torch')}, python {sys.version.split()[0]}"
+
+
+def _host_fits() -> bool:
+    try:
+        with open(HOST_STAMP) as f:
+            return f.read() == _host_versions()
+    except OSError:
+        return False
+
+
 def _build_host() -> None:
     """``csrc/torch_host.cpp`` -> ``_host.so``: a Python module against the installed PyTorch's headers and libraries,
     linked to ``liblmoe.so`` beside it."""
@@ -66,13 +81,17 @@ def _build_host() -> None:
     r = subprocess.run(cmd, capture_output=True, text=True)
     if r.returncode != 0:
         raise RuntimeError(f"g++ failed for torch_host.cpp:\n{r.stdout}\n{r.stderr}")
+    with open(HOST_STAMP, "w") as f:
+        f.write(_host_versions())
 
 
 def build(force: bool = False, verbose: bool = False) -> str:
     newest = _deps_mtime()
-    if not force and all(os.path.exists(p) and os.path.getmtime(p) >= newest for p in (LIB, HOST)):
-        return LIB
     os.makedirs(OBJ, exist_ok=True)
+    if not force and all(os.path.exists(p) and os.path.getmtime(p) >= newest for p in (LIB, HOST)):
+        if not _host_fits():          # PyTorch or Python has changed since
+            _build_host()
+        return LIB
     nvcc = _nvcc()
 
     def compile_one(src: str) -> str:

@@ -34,7 +34,11 @@ def _host():
     global _native
     if _native is None:
         _cabi.load()
-        from . import _host as native
+        try:
+            from . import _host as native
+        except ImportError as e:
+            raise _cabi.LmoeError(f"swamla_b200/_host.so is missing or was built for another PyTorch or Python ({e}): build it with "
+                                  "`python -m swamla_b200.build` (there is no CPU or PyTorch fallback for this path)") from e
         native.set_error_class(_cabi.LmoeError)
         _native = native
     return _native
