@@ -906,10 +906,10 @@ Tensor rows_of(const Tensor& t) {
   const Tensor d = t.detach();
   return (d.scalar_type() == at::kFloat || d.scalar_type() == at::kBFloat16 ? d : d.to(at::kFloat)).contiguous();
 }
-// the norm's weight: a slice of a flat parameter need not start at the 16 bytes that the kernels read at once
-Tensor weight_of(const Tensor& t) {
-  const Tensor w = rows_of(t);
-  return aligned(w) ? w : w.clone();
+// ... where the 16 bytes that the kernels read at once begin: a slice of a flat parameter or of another gradient need not
+Tensor aligned_rows_of(const Tensor& t) {
+  const Tensor r = rows_of(t);
+  return aligned(r) ? r : r.clone();
 }
 
 // (xn, x_pass) = (rmsnorm(x) * weight, x).  x_pass is x itself, handed on to the residual add, so that the backward sees the
@@ -919,7 +919,7 @@ Tensor weight_of(const Tensor& t) {
 class NormFn : public torch::autograd::Function<NormFn> {
  public:
   static variable_list forward(AutogradContext* ctx, const Tensor& x, const Tensor& weight, double eps, bool bf16_out, bool keep) {
-    const Tensor xr = rows_of(x), w = weight_of(weight);
+    const Tensor xr = rows_of(x), w = aligned_rows_of(weight);
     TORCH_CHECK(x.dim() > 0 && weight.numel() == x.size(-1), "the norm's weight has another width than its input");
     const int64_t D = x.size(-1), T = xr.numel() / D;
     const bool wide = !bf16_out && xr.scalar_type() == at::kFloat;
@@ -948,9 +948,9 @@ class NormFn : public torch::autograd::Function<NormFn> {
       const auto s = ctx->saved_data["s"].toIntVector();  // the types that the forward's kernel took
       const auto stream_type = static_cast<at::ScalarType>(s[0]), dw_type = static_cast<at::ScalarType>(s[1]);
       const int64_t D = x.size(-1), T = x.numel() / D;
-      const Tensor g = grads[0].defined() ? rows_of(grads[0]) : at::zeros_like(x);
+      const Tensor g = grads[0].defined() ? aligned_rows_of(grads[0]) : at::zeros_like(x);
       Tensor r;
-      if (grads[1].defined()) r = rows_of(grads[1]).to(stream_type).contiguous();
+      if (grads[1].defined()) r = aligned_rows_of(grads[1].to(stream_type));
       Tensor dx = at::empty(x.sizes(), x.options().dtype(stream_type));
       Tensor dw = at::empty({D}, x.options().dtype(dw_type));
       Tensor ws = new_bytes(lmoe_rmsnorm_workspace_bytes(static_cast<int>(D)), x);
@@ -990,7 +990,7 @@ class AddFn : public torch::autograd::Function<AddFn> {
     auto cast = [&](int k) {
       const auto d = static_cast<at::ScalarType>(t[k]);
       if (!grads[0].defined() || grads[0].scalar_type() == d) return grads[0];
-      if (d != at::kBFloat16 || grads[0].scalar_type() != at::kFloat) return grads[0].to(d);
+      if (d != at::kBFloat16 || grads[0].scalar_type() != at::kFloat || !aligned(grads[0])) return grads[0].to(d);
       const c10::cuda::CUDAGuard guard(grads[0].device());
       Caster narrow;
       Tensor g = narrow(grads[0]);

@@ -119,3 +119,21 @@ def test_block_s_inputs_may_change_before_the_backward(what, width):
             m.ffn_norm.weight.copy_(kept)
         got.append((leaf.grad, m.ffn_norm.weight.grad.clone()))
     assert all(torch.equal(a, b) for a, b in zip(*got))
+
+
+@pytest.mark.parametrize("own", [True, False])
+def test_block_takes_a_gradient_that_begins_anywhere(own):
+    """An fp32 upstream gradient that is contiguous but does not begin at 16 bytes (a slice of a flat buffer)."""
+    from swamla_b200.block import NormedResidualFFN
+    m, x = _module("block", torch.float32)
+    if not own:                                     # (an element-wise branch: a library GEMM may choose by alignment)
+        m = NormedResidualFFN(torch.nn.Tanh(), x.shape[-1]).cuda()
+    dy = torch.randn(x.numel() + 1, device=x.device)[1:].view(x.shape)
+    assert dy.is_contiguous() and dy.data_ptr() % 16
+    grads = []
+    for g in (dy, dy.clone()):
+        xg = x.clone().requires_grad_(True)
+        m.zero_grad()
+        m.train()(xg).backward(g)
+        grads.append([xg.grad, *[p.grad.clone() for p in m.parameters()]])
+    assert all(torch.equal(a, b) for a, b in zip(*grads))
