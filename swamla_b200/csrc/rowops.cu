@@ -498,6 +498,7 @@ extern "C" int lmoe_combine_bwd_rows(const void* d_routed, const void* y_rows, c
 
 extern "C" int lmoe_cast_f32_to_bf16(const float* src, void* dst, int64_t n, void* stream) {
   if (!src || !dst || n <= 0) return LMOE_ERR_ARG;
+  if ((reinterpret_cast<uintptr_t>(src) & 15) != 0 || (reinterpret_cast<uintptr_t>(dst) & 7) != 0) return LMOE_ERR_ALIGN;
   const long long n4 = n / 4;
   const int tail = static_cast<int>(n - n4 * 4);
   cast_f32_bf16_kernel<<<grid_for(n4 > 0 ? n4 : 1, 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(

@@ -215,14 +215,22 @@ struct Sizes {
   }
 };
 
+void check_device(const Tensor& t, at::Device device) {
+  if (t.device() != device) throw LmoeFailure("a tensor of the layer is on " + t.device().str() + ", its input on " + device.str());
+}
+
 // bf16, contiguous forms of the operands; everything that is fp32 is converted by one launch.
+// All on one device: a pointer to another one's memory, or to the host's, would only be found out by a kernel.
 struct Caster {
+  explicit Caster(const Tensor& x) : device(x.device()) {}
+  const at::Device device;
   const float* src[LMOE_CAST_MANY_MAX];
   void* dst[LMOE_CAST_MANY_MAX];
   int64_t n[LMOE_CAST_MANY_MAX];
   std::vector<Tensor> keep;
   int count = 0;
   Tensor operator()(const Tensor& t) {
+    check_device(t, device);
     if (t.scalar_type() == at::kBFloat16) return t.is_contiguous() ? t.detach() : t.detach().contiguous();
     Tensor f = t.detach();
     if (f.scalar_type() != at::kFloat) f = f.to(at::kFloat);
@@ -257,7 +265,8 @@ bool tma_gather_enabled() {
   return on;
 }
 
-Tensor f32_bias(const Tensor& b) {
+Tensor f32_bias(const Tensor& b, const Tensor& x) {
+  check_device(b, x.device());
   return b.scalar_type() == at::kFloat && b.is_contiguous() ? b : b.detach().to(at::kFloat).contiguous();
 }
 
@@ -790,7 +799,7 @@ at::ScalarType lin_dtype_of(std::initializer_list<at::ScalarType> dts) {
 
 LatentOps latent_ops(const Tensor& x, const Tensor& wg, const Tensor& wdn, const Tensor& wup, const Tensor& wgus,
                      const Tensor& wds, const Tensor& wgu, const Tensor& wde) {
-  Caster cast;
+  Caster cast(x);
   LatentOps o{cast(x).view({-1, x.size(-1)}), cast(wg), cast(wdn), cast(wup), cast(wgus), cast(wds), cast(wgu), cast(wde)};
   cast.run(at::cuda::getCurrentCUDAStream().stream());
   return o;
@@ -804,7 +813,7 @@ std::vector<int64_t> dtypes_of(const std::vector<Tensor>& ts) {
 
 Tensor grad_rows(const Tensor& dy, const Tensor& like2d) {
   if (!dy.defined()) return at::zeros_like(like2d);
-  Caster cast;
+  Caster cast(like2d);
   Tensor d = cast(dy);
   cast.run(at::cuda::getCurrentCUDAStream().stream());
   return d.view({like2d.size(0), like2d.size(1)});
@@ -818,7 +827,7 @@ class LatentFn : public torch::autograd::Function<LatentFn> {
                                int64_t top_k, double z_coef, bool fp8) {
     const LatentOps o = latent_ops(x, wg, wdn, wup, wgus, wds, wgu, wde);
     const Sizes d = latent_sizes(o.x, o.wgu, o.wds, top_k);
-    LatentOut r = latent_forward(d, o, f32_bias(bias), static_cast<float>(z_coef), fp8, true, c10::nullopt, nullptr);
+    LatentOut r = latent_forward(d, o, f32_bias(bias, x), static_cast<float>(z_coef), fp8, true, c10::nullopt, nullptr);
     ctx->set_materialize_grads(false);
     // e4m3: the quantised copies in `saved` replace the bf16 expert weights
     const Tensor none = fp8 ? Tensor() : o.wgu;
@@ -860,11 +869,11 @@ class MoeFn : public torch::autograd::Function<MoeFn> {
   static variable_list forward(AutogradContext* ctx, const Tensor& x, const Tensor& wg, const Tensor& wgus, const Tensor& wds,
                                const Tensor& wgu, const Tensor& wde, const Tensor& bias, int64_t top_k, double z_coef,
                                const c10::optional<Tensor>& forced) {
-    Caster cast;
+    Caster cast(x);
     const MoeOps o{cast(x).view({-1, x.size(-1)}), cast(wg), cast(wgus), cast(wds), cast(wgu), cast(wde)};
     cast.run(at::cuda::getCurrentCUDAStream().stream());
     const Sizes d = moe_sizes(o.x, o.wgu, o.wds, top_k);
-    LatentOut r = moe_forward(d, o, f32_bias(bias), static_cast<float>(z_coef), true, forced);
+    LatentOut r = moe_forward(d, o, f32_bias(bias, x), static_cast<float>(z_coef), true, forced);
     ctx->set_materialize_grads(false);
     ctx->save_for_backward({o.x, o.wg, o.wgus, o.wds, o.wgu, o.wde, r.sel, r.saved});
     ctx->saved_data["i"] = std::vector<int64_t>{d.E, d.K, d.F, d.Fs};
@@ -975,6 +984,7 @@ class AddFn : public torch::autograd::Function<AddFn> {
   static Tensor add(const Tensor& a, const Tensor& b) {
     const bool bf = b.scalar_type() == at::kBFloat16;
     if (!bf || (a.scalar_type() != at::kBFloat16 && a.scalar_type() != at::kFloat)) return a.detach() + b.detach().to(a.scalar_type());
+    check_device(b, a.device());
     const Tensor ac = a.detach().contiguous(), bc = b.detach().contiguous();
     if (ac.scalar_type() == at::kFloat && !(aligned(ac) && aligned(bc))) return ac + bc;
     Tensor out = at::empty_like(ac);
@@ -992,7 +1002,7 @@ class AddFn : public torch::autograd::Function<AddFn> {
       if (!grads[0].defined() || grads[0].scalar_type() == d) return grads[0];
       if (d != at::kBFloat16 || grads[0].scalar_type() != at::kFloat || !aligned(grads[0])) return grads[0].to(d);
       const c10::cuda::CUDAGuard guard(grads[0].device());
-      Caster narrow;
+      Caster narrow(grads[0]);
       Tensor g = narrow(grads[0]);
       narrow.run(at::cuda::getCurrentCUDAStream().stream());
       return g;
@@ -1022,10 +1032,10 @@ std::vector<Tensor> latent_moe(const Tensor& x, const Tensor& wg, const Tensor& 
   const LatentOps o = latent_ops(x, wg, wdn, wup, wgus, wds, wgu, wde);
   const Sizes d = latent_sizes(o.x, o.wgu, o.wds, top_k);
   if (evaluation && !fp8 && d.T <= LMOE_FEW_TOKENS && lmoe_few_applies(&d.s)) {  // (its experts are bf16)
-    auto yz = few_forward(d, o.x, o.wg, &o.wdn, &o.wup, o.wgus, o.wds, o.wgu, o.wde, f32_bias(bias), static_cast<float>(z_coef));
+    auto yz = few_forward(d, o.x, o.wg, &o.wdn, &o.wup, o.wgus, o.wds, o.wgu, o.wde, f32_bias(bias, x), static_cast<float>(z_coef));
     return {as_param(yz[0].view(x.sizes()), x.scalar_type()), yz[1]};
   }
-  LatentOut r = latent_forward(d, o, f32_bias(bias), static_cast<float>(z_coef), fp8,
+  LatentOut r = latent_forward(d, o, f32_bias(bias, x), static_cast<float>(z_coef), fp8,
                                false, c10::nullopt, nullptr);
   return {as_param(r.y.view(x.sizes()), x.scalar_type()), r.z_loss, r.sel, r.counts};
 }
@@ -1037,20 +1047,21 @@ std::vector<Tensor> moe(const Tensor& x, const Tensor& wg, const Tensor& wgus, c
   poll_status();
   const c10::cuda::CUDAGuard guard(x.device());
   if (any_grad({&x, &wg, &wgus, &wds, &wgu, &wde})) return MoeFn::apply(x, wg, wgus, wds, wgu, wde, bias, top_k, z_coef, forced_sel);
-  Caster cast;
+  Caster cast(x);
   const MoeOps o{cast(x).view({-1, x.size(-1)}), cast(wg), cast(wgus), cast(wds), cast(wgu), cast(wde)};
   cast.run(at::cuda::getCurrentCUDAStream().stream());
   const Sizes d = moe_sizes(o.x, o.wgu, o.wds, top_k);
   if (evaluation && !forced_sel && d.T <= LMOE_FEW_TOKENS && lmoe_few_applies(&d.s)) {
-    auto yz = few_forward(d, o.x, o.wg, nullptr, nullptr, o.wgus, o.wds, o.wgu, o.wde, f32_bias(bias), static_cast<float>(z_coef));
+    auto yz = few_forward(d, o.x, o.wg, nullptr, nullptr, o.wgus, o.wds, o.wgu, o.wde, f32_bias(bias, x), static_cast<float>(z_coef));
     return {as_param(yz[0].view(x.sizes()), x.scalar_type()), yz[1]};
   }
-  LatentOut r = moe_forward(d, o, f32_bias(bias), static_cast<float>(z_coef), false, forced_sel);
+  LatentOut r = moe_forward(d, o, f32_bias(bias, x), static_cast<float>(z_coef), false, forced_sel);
   return {as_param(r.y.view(x.sizes()), x.scalar_type()), r.z_loss, r.sel, r.counts};
 }
 
 std::vector<Tensor> norm_and_pass(const Tensor& x, const Tensor& weight, double eps, bool bf16_out) {
   require_cuda(x, "fused norm");
+  check_device(weight, x.device());
   const c10::cuda::CUDAGuard guard(x.device());
   return NormFn::apply(x, weight, eps, bf16_out, any_grad({&x, &weight}));
 }
@@ -1077,7 +1088,7 @@ py::tuple latent_fwd_raw(const Tensor& x, const Tensor& wg, const Tensor& wdn, c
   const c10::cuda::CUDAGuard guard(x.device());
   const LatentOps o = latent_ops(x, wg, wdn, wup, wgus, wds, wgu, wde);
   Views views;
-  LatentOut r = latent_forward(latent_sizes(o.x, o.wgu, o.wds, top_k), o, f32_bias(bias), static_cast<float>(z_coef), fp8,
+  LatentOut r = latent_forward(latent_sizes(o.x, o.wgu, o.wds, top_k), o, f32_bias(bias, x), static_cast<float>(z_coef), fp8,
                                true, forced_sel, capture ? &views : nullptr);
   const Tensor y = as_param(r.y.view(x.sizes()), x.scalar_type());
   py::gil_scoped_acquire gil;

@@ -95,3 +95,61 @@ def test_whoever_looks_at_the_feed_forward_module_sees_the_stream_s_precision(ki
         assert ((y - plain) - add).abs().max().item() <= 2.0 ** -21   # fp32 roundings of values of a few units
     else:
         assert torch.equal(y, plain)
+
+
+@pytest.mark.parametrize("grad", [True, False])
+@pytest.mark.parametrize("kind", KINDS + ["block"])
+def test_tensors_on_another_device_are_refused(kind, grad):
+    """By the host, before anything is launched."""
+    from swamla_b200 import _cabi
+    from swamla_b200.block import NormedResidualFFN
+    layer, x = _layer("latent" if kind == "block" else kind)
+    m = NormedResidualFFN(layer, x.shape[-1]).cuda() if kind == "block" else layer
+    names = [n for n, _ in m.named_parameters()] + [n for n, _ in m.named_buffers() if n.endswith("expert_bias")]
+    lib = _cabi.load()
+    with torch.set_grad_enabled(grad):
+        for mode in (m.train(), m.eval()):
+            for n in names:
+                owner = m.get_submodule(n.rpartition(".")[0])
+                t = getattr(owner, n.rpartition(".")[2])
+                on_gpu, t.data = t.data, t.data.cpu()
+                before = lib.lmoe_launch_count()
+                try:
+                    with pytest.raises(_cabi.LmoeError, match="is on cpu"):
+                        mode(x)
+                    assert lib.lmoe_launch_count() - before <= (1 if kind == "block" else 0), n    # the block's norm
+                finally:
+                    t.data = on_gpu
+            mode(x)
+            mode.check_status() if kind != "block" else layer.check_status()
+
+
+def test_conversion_of_a_misaligned_tensor_is_refused():
+    from swamla_b200 import _cabi
+    a, b = torch.zeros(65, device="cuda:0"), torch.zeros(64, dtype=torch.bfloat16, device="cuda:0")
+    st = torch.cuda.current_stream().cuda_stream
+    rc = _cabi.load().lmoe_cast_f32_to_bf16(a[1:].data_ptr(), b.data_ptr(), 64, st)
+    assert rc == -3                                                     # LMOE_ERR_ALIGN
+
+
+@pytest.mark.parametrize("kind", KINDS)
+def test_a_call_that_fails_between_fork_and_join(kind):
+    """A weight that does not begin at 16 bytes is refused by the shared expert's GEMM, when the side stream has work already:
+    the streams are joined, and the calls after it give the bits of the ones before."""
+    from swamla_b200 import _cabi
+    layer, x = _layer(kind)
+    w = layer.shared_experts[0].gate_up_proj.weight
+    flat = torch.empty(w.numel() + 1, dtype=w.dtype, device=w.device)
+    off = flat[1:].view(w.shape)
+    off.copy_(w.detach())
+    with torch.no_grad():
+        want = layer.train()(x)
+        for _ in range(5):
+            good, w.data = w.data, off
+            try:
+                with pytest.raises(_cabi.LmoeError, match="aligned"):
+                    layer(x)
+            finally:
+                w.data = good
+            assert torch.equal(layer(x), want)
+    layer.check_status()
