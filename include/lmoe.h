@@ -201,8 +201,8 @@ int lmoe_shared_gateup_fwd(const lmoe_shape* s, const void* x, const void* w_gat
 int lmoe_combine_out_fwd(const lmoe_shape* s, const void* y_sorted, const lmoe_route* r, const float* weights,
                          void* act_cat, const void* w_down_s, const void* w_up, void* y, int32_t* status, void* stream);
 
-/* Whole forward of a few tokens (generation) in three or four launches without the padded layout: T <= LMOE_FEW_TOKENS, every other
- * dimension as lmoe_few_applies says.  With w_down = w_up = NULL and L = D: the non-latent layer (models/moe.py:344-372).
+/* Whole forward of a few tokens (generation) in three or four launches without the padded layout: T <= LMOE_FEW_TOKENS, or 24 where
+ * an expert's rows are wider than 512 (max(2F, L)), every other dimension as lmoe_few_applies says.  With w_down = w_up = NULL and L = D: the non-latent layer (models/moe.py:344-372).
  * Same stages and rounding points as the entry points above (models/moe.py:702-734), fp32 sums in another order.  bf16
  * expert weights only: a layer with e4m3 experts does not take it.  Nothing is kept for a backward. */
 #define LMOE_FEW_TOKENS 64

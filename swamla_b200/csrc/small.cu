@@ -326,9 +326,10 @@ __global__ void __launch_bounds__(kFewThreads, 2) few_expert_kernel(const FewPar
 // there are more experts than SMs, when two CTAs share one.  The weights are [k, n] with n contiguous, so the columns become
 // the rows of an m16n8k16 product through ldmatrix.trans and the tokens its eight columns; a stage row is padded by 16 bytes
 // so that the eight rows of a matrix lie in different banks.  Every thread copies with cp.async: one bulk copy per padded row
-// costs the TMA unit some 50 ns each (34 us for the launch instead of the figure below).
-// At 23 tokens of the 128-expert layer: 16 + 9 us with the two launches of the register kernel above, which needs several
-// rounds of CTAs per SM; 44 us with the products on CUDA cores (an expert with six tokens is then bound by them).
+// costs the TMA unit some 50 ns each (34 us for this launch alone).
+// At 23 tokens of the 128-expert layer the two launches of the register kernel above take 16 + 9 us (several rounds of CTAs per
+// SM), products on CUDA cores instead 44 us (an expert with six tokens is then bound by them); the whole call of three
+// launches takes 31.8 us on the device.
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
@@ -524,7 +525,7 @@ __global__ void __launch_bounds__(kFewThreads) few_out_kernel(const FewParams p)
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
   const int c_s = p.Fs / 32, chunks = c_s + (p.wup ? p.L / 32 : 0);
   const int row = blockIdx.x * 16, tok0 = blockIdx.y * 8, n_tok = min(8, p.T - tok0);
-  constexpr int U = 5;
+  constexpr int U = 5;  // steps in flight: (Fs + L) / 256 of a 1,024-wide layer; other sizes loop (3: up to 1.7 us slower)
   uint4 a[U], b[U];
   auto load = [&](int c, uint4& va, uint4& vb) {
     const __nv_bfloat16* base = c < c_s ? p.wds + static_cast<long long>(row + g) * p.Fs + c * 32 + t * 8
@@ -541,7 +542,7 @@ __global__ void __launch_bounds__(kFewThreads) few_out_kernel(const FewParams p)
     for (int i = tid; i < n_tok * vecs; i += kFewThreads) {
       const int tok = i / vecs, v = i - tok * vecs;
       float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-      for (int k0 = 0; k0 < p.K; k0 += 6) {
+      for (int k0 = 0; k0 < p.K; k0 += 6) {  // slots in flight (4 measures the same, within 0.3 us)
         uint4 yv[6];
         float wk[6];
 #pragma unroll
@@ -623,16 +624,30 @@ static int few_launch(Kernel kernel, dim3 grid, size_t smem, bool after, cudaStr
   return e == cudaSuccess ? 0 : static_cast<int>(e);
 }
 
+// Whether an expert's rows fit four tiles of 16 columns per warp: the streamed kernel then takes 16 tokens per pass over the
+// weights, else eight.
+static int few_widest(int L, int F) { return 2 * F > L ? 2 * F : L; }
+static bool few_narrow(int L, int F) { return few_widest(L, F) <= 4 * kFewWarps * 16; }
+// Up to how many tokens these kernels beat the padded path (device time of a captured call, us, these kernels / padded):
+//   rows of at most 512: L 256, F 256, 128 experts: 1 token 16 / 44, 23 32 / 57, 64 42 / 59; 256 experts: 64 70 / 74.  The masks of
+//     an expert's tokens hold kFewTokens.
+//   wider ones, where a second pass over the weights of the experts with more than eight tokens costs as much as the first:
+//     L 256, F 768, 128 experts: 24 71 / 90, 28 72 / 90, 32 96 / 91, 64 138 / 92;
+//     L 1,024, F 1,024, 32 experts (each streamed by one SM): 24 80 / 83, 28 88 / 87, 32 92 / 87, 64 158 / 89.
+static int few_tokens(int L, int F) { return few_narrow(L, F) ? kFewTokens : 24; }
+
 template <int NT>
 static int few_forward(const FewParams& p, cudaStream_t st) {
   const int units = (p.wdn ? p.L / 16 : 0) + p.Fs / 8;
-  const int cap = 512;  // two rounds of 256-thread CTAs over the SMs' slots at most; the rest loops
+  const int cap = 512;  // CTAs of 256 threads, the rest loops (256 and 1,024 measure the same, within 0.3 us)
   const int rest = ((units < cap ? units : cap) + kFewCluster - 1) / kFewCluster * kFewCluster;
   auto in = p.E <= 32 ? few_in_kernel<NT, 1> : p.E <= 64 ? few_in_kernel<NT, 2> : p.E <= 128 ? few_in_kernel<NT, 4> : few_in_kernel<NT, 8>;
   if (int rc = few_launch(in, dim3(kFewCluster + rest), 0, false, st, p)) return rc;
   // the stream kernel wherever every expert is likely to have a token and its rows fit the tiles of a warp
-  const int widest = 2 * p.F > p.L ? 2 * p.F : p.L;
-  const bool narrow = widest <= 4 * kFewWarps * 16;
+  const int widest = few_widest(p.L, p.F);
+  const bool narrow = few_narrow(p.L, p.F);
+  // Stages of the ring: many, as bytes in flight are the rate (128 experts, 23 tokens: 10 stages 31.8 us, 8 32.3, 6 32.7; wide rows:
+  // 3 71.6, 4 91.3, which leaves one CTA per SM).  More experts than SMs: two CTAs per SM share its memory.
   const int stages = !narrow ? 3 : p.E <= num_sms() ? 10 : 5;
   const StreamPlan sp = stream_plan(p.L, p.F, narrow ? 16 : 8, stages);
   constexpr size_t kMost = 220 * 1024;
@@ -667,7 +682,7 @@ static int few_forward(const FewParams& p, cudaStream_t st) {
 using namespace lmoe;
 
 static bool few_dims(const lmoe_shape* s, int L) {
-  return s && s->T > 0 && s->T <= kFewTokens && s->D > 0 && (s->D % 32) == 0 && L > 0 && (L % 64) == 0 && s->E > 0 &&
+  return s && s->T > 0 && s->T <= few_tokens(L, s->F) && s->D > 0 && (s->D % 32) == 0 && L > 0 && (L % 64) == 0 && s->E > 0 &&
          s->E <= LMOE_MAX_EXPERTS && s->K > 0 && s->K <= LMOE_MAX_TOPK && s->K <= s->E && s->F > 0 && (s->F % 64) == 0 &&
          s->Fs > 0 && (s->Fs % 32) == 0 && L <= kFewMaxLatent;
 }

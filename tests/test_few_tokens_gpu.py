@@ -13,8 +13,8 @@ from oracle import inputs
 pytestmark = pytest.mark.gpu
 
 
-# one token, the edges of every token-tile count (8, 16, 32, 64), and the first size beyond the path
-@pytest.mark.parametrize("T", [1, 2, 8, 9, 16, 17, 33, 64, 65])
+# one token, the edges of every token-tile count (8, 16, 32, 64), and the first sizes beyond the path: 65, and 25 for wide experts
+@pytest.mark.parametrize("T", [1, 2, 8, 9, 16, 17, 24, 25, 33, 64, 65])
 # widths of one and several passes, fewer slots than experts and more, 4 to 256 experts, both layer classes
 @pytest.mark.parametrize("name", ["tiny", "cfg1", "cfg5_2k", "cfg3", "tiny_moe", "moe_1b"])
 def test_few_token_forward_matches_padded_path(name, T):
@@ -31,13 +31,16 @@ def test_few_token_forward_matches_padded_path(name, T):
         x = torch.randn(T, 1, w.D).to(torch.bfloat16)
     lib = _cabi.load()
     shape = _cabi.Shape(T=T, D=w.D, L=w.L, E=w.E, K=w.K, F=w.F, Fs=w.Fs, n_shared=1)
-    assert lib.lmoe_few_applies(shape) == (1 if T <= 64 else 0)
+    few = T <= (64 if max(2 * w.F, w.L) <= 512 else 24)
+    assert lib.lmoe_few_applies(shape) == (1 if few else 0)
     with torch.no_grad():
         y_ref = layer.train()(x)
         z_ref = layer.get_aux_loss().clone()
         before = lib.lmoe_launch_count()
         y = layer.eval()(x)
-        assert (lib.lmoe_launch_count() - before <= 4) == (T <= 64)
+        assert (lib.lmoe_launch_count() - before <= 4) == few
+        if not few:
+            assert torch.equal(y, y_ref)
         y2 = layer(x)
     layer.check_status()
     assert torch.equal(y, y2)                                             # deterministic
