@@ -22,12 +22,3 @@ def capture(**tensors) -> None:
 
 def capturing() -> bool:
     return SINK is not None
-
-
-def forced_selection(logits: torch.Tensor):
-    """(sel, weights) for the forced selection, or None."""
-    if FORCE_SEL is None:
-        return None
-    forced = FORCE_SEL.to(device=logits.device, dtype=torch.int32).contiguous()
-    aff = torch.sigmoid(logits).gather(1, forced.long())
-    return forced, (aff / (aff.sum(-1, keepdim=True) + 1e-9)).contiguous()

@@ -156,7 +156,7 @@ combine_bwd_kernel(const uint4* __restrict__ d_routed, const uint4* __restrict__
 // The same adjoint token by token: one warp takes a token's row of d_routed once and walks its K expert rows (pos), four at
 // a time, so four independent y rows are in flight per lane and no index has to arrive before a row can be asked for by
 // the next one.  Pad rows (any d_y that is not some token's) are zeroed by the blocks that own the experts b, b + gridDim.x..
-// 1.57 M rows of 512 bytes beside the weight gradient GEMM: see the numbers at lmoe_combine_bwd.
+// At 16,384 tokens, 12 rows of 512 bytes each, alone: 47.1 us against 49.2 for the kernel above (4.6 TB/s of 217 MB).
 // QUANT: d_y leaves as e4m3 of the bf16-rounded product, scaled by 448 / amax (amax computed by amax_weighted_kernel).
 template <bool QUANT>
 __global__ void __launch_bounds__(kRowWarps * 32)

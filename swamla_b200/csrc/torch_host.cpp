@@ -738,7 +738,7 @@ MoeGrads moe_backward(const Sizes& d, const MoeOps& o, const Tensor& dy, const f
 
   // [adjoint of the weighted sum: d_y_sorted = w * dy[t], d_w = <dy[t], y_sorted>] beside
   // [shared expert: d_h1_s (SwiGLU adjoint in the epilogue) -> cat[:, :2Fs]; d_Wd_s = dy^T * hidden_s]
-  // (both side sections: 4,096 tokens 553 -> 537 us with both directions, 924 tokens 354 -> 323 us)
+  // (both side sections: 924 tokens 354 -> 323 us with both directions; at 4,096 tokens, 550 us, within the 3 % between runs)
   Fork fork(stream);
   void* side = fork.side();
   fork.to_side();

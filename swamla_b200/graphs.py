@@ -1,9 +1,9 @@
 """CUDA-graph replay of the LatentMoE layer's forward and backward for a fixed input shape.
 
-The layer launches ~40 kernels per step and allocates ~50 buffers from Python; captured once, a step becomes two
-graph launches (forward, backward) with static buffers, which removes the host work and the launch gaps between
-kernels.  Built on ``torch.cuda.make_graphed_callables`` (the C-ABI calls launch on the capturing stream, the side
-stream of the row kernels forks from and joins it, nothing synchronises).  Single-GPU layers only: the expert-parallel
+The layer launches 24 to 28 kernels per step through one native call per direction; captured once, a step becomes two graph
+launches (forward, backward) with static buffers, which removes the host work and the launch gaps between kernels and adds
+copies of x and the upstream gradients into those buffers.  Built on ``torch.cuda.make_graphed_callables`` (the C-ABI calls
+launch on the capturing stream, the side stream forks from and joins it, nothing synchronises).  Single-GPU layers only: the expert-parallel
 modes issue collectives and size buffers per step.
 """
 from __future__ import annotations
