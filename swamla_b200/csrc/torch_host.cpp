@@ -126,9 +126,14 @@ class Fork {
     std::lock_guard<std::mutex> lock(g_side_mutex);
     Side& s = g_sides[{main.device_index(), main_}];
     if (!s.stream) {
-      do s.stream = c10::cuda::getStreamFromPool(false, main.device_index()).stream();
-      while (s.stream == main_);
-      C10_CUDA_CHECK(cudaEventCreateWithFlags(&s.ev, cudaEventDisableTiming));
+      // A stream of its own, not one of PyTorch's pool, which hands the same 32 out to everybody: while this one is part of a
+      // capture, what another user of it queued would be recorded instead of run.
+      cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;  // the first call may be one that is being captured
+      C10_CUDA_CHECK(cudaThreadExchangeStreamCaptureMode(&mode));
+      cudaError_t e = cudaStreamCreateWithFlags(&s.stream, cudaStreamNonBlocking);
+      if (e == cudaSuccess) e = cudaEventCreateWithFlags(&s.ev, cudaEventDisableTiming);
+      cudaThreadExchangeStreamCaptureMode(&mode);
+      C10_CUDA_CHECK(e);
     }
     side_ = &s;
   }

@@ -167,3 +167,38 @@ def test_first_call_of_a_thread(kind):
     t.join()
     assert isinstance(got[0], torch.Tensor), got[0]
     assert torch.equal(got[0], want)
+
+
+@pytest.mark.parametrize("kind", ["latent", "moe"])
+def test_no_stream_that_others_use_becomes_part_of_a_capture(kind):
+    """PyTorch hands out 32 pooled streams in turn; work on any of them while a layer is being captured has to run."""
+    m, xs = _module(kind, 0)
+    x, z = xs[2], torch.zeros(1, device="cuda:0")
+    main = torch.cuda.Stream()
+    pool = [torch.cuda.Stream() for _ in range(64)]
+    with torch.no_grad():
+        with torch.cuda.stream(main):
+            want = m(x)
+        torch.cuda.synchronize()
+        others, errors = [s for s in pool if s.cuda_stream != main.cuda_stream], []
+
+        def work():
+            torch.set_grad_enabled(False)
+            try:
+                for s in others:
+                    with torch.cuda.stream(s):
+                        z.add_(1.0)
+                    s.synchronize()
+            except Exception as e:
+                errors.append(e)
+
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g, stream=main, capture_error_mode="thread_local"):
+            got = m(x)
+            t = threading.Thread(target=work)
+            t.start()
+            t.join()
+    assert not errors and z.item() == len(others)
+    g.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(got, want)
